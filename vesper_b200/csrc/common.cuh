@@ -146,16 +146,25 @@ struct WaitCtx {
     int* status;                // device status word
 };
 
+// kCluster: acquires at cluster scope, for data that other CTAs of the cluster have stored.
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, int where) {
     uint32_t addr = smem_u32(bar);
     uint32_t ok = 0;
     long long t0 = 0;
     for (uint32_t it = 0;; ++it) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
+        if (kCluster)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.b32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
+        else
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.b32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
         if (ok) return true;
         if ((it & 0xFF) == 0xFF) {
             if (*ctx.abort_flag) return false;
@@ -172,8 +181,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
 
 // Same, for code that follows the wait with warp-collective instructions
 // (tcgen05.ld/st are .sync.aligned): the outcome is made warp-uniform.
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, int where) {
-    bool ok = mbar_wait(bar, parity, ctx, where);
+    bool ok = mbar_wait<kCluster>(bar, parity, ctx, where);
     return __all_sync(0xFFFFFFFFu, ok);
 }
 

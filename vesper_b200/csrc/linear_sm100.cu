@@ -9,11 +9,12 @@
 //   linear_skinny_kernel  M <= 16 (one token per sequence).  The product is weight-bandwidth bound,
 //                         so the roles swap: 128 W rows are the UMMA M operand and the (zero padded)
 //                         16 token rows the N operand; K is split over the CTAs of a thread-block
-//                         cluster, which reduce their partial tiles through distributed shared
-//                         memory in a fixed order (deterministic) before the leader's epilogue.
+//                         cluster, which scatter their partial tiles through distributed shared
+//                         memory; each CTA sums and finishes its tokens in a fixed order (deterministic).
 // Epilogues (fused, per output element): store bf16 | store fp32 | fp32 accumulate into the residual
 // stream (optionally plus a second fp32 addend) | squared ReLU -> bf16 | SwiGLU over interleaved (gate, up) weight rows -> bf16 (src/nn/swiglu.cpp:36-48,
 // ops::silu_mul src/ops/elementwise.cpp:1297-1328) | the same with max(gate, 0).
+#include "cluster_pair.cuh"
 #include "kernels.h"
 
 #include <cuda.h>
@@ -317,37 +318,83 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
 // ------------------------------------------------------------------------------------------------
 // Skinny kernel: out[m, n] = sum_k x[m,k] W[n,k] for m < MT <= 64.  One CTA = 128 W rows x one K slice;
 // the `splits` CTAs of a cluster hold the K slices of the same 128 rows.
+//
+// What bounds it: the weights' bytes, and, in a chain of such products (a decode step), the time from the predecessor's end to
+// its own.  So the ring's first weight tiles are loaded before the predecessor has finished (two CTAs fit an SM), and the cluster's
+// sum is scattered: CTA r finishes tokens [r, r + 1) * share of the 128 rows, every other CTA stores its partials of them straight
+// into r's shared memory (st.async, counted by a barrier of r), and r adds them in rank order (bit-reproducible) while it already
+// holds the residual rows that they go onto.  Dependent products of 8 tokens, one leading CTA's sum behind two cluster
+// barriers -> now: 2048 x 2048 8.2 -> 4.4 us, 2048 x 5632 10.6 -> 7.7, 11264 x 2048 14.2 -> 10.6 (with 3 slices for 2), 160 x 4096 5.7 -> 5.2; 32000 x
+// 2048, one slice, 22.4 -> 22.6.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
+// stores of V values to another CTA's shared memory, counted by the barrier `bar` there (both shared::cluster addresses)
+template <int V>
+__device__ __forceinline__ void st_async(uint32_t addr, const float* v, uint32_t bar) {
+    if (V == 4)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                     ::"r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar) : "memory");
+    else if (V == 2)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(v[0]), "f"(v[1]), "r"(bar) : "memory");
+    else
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(v[0]), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+template <int V>
+__device__ __forceinline__ void load_v(float (&v)[V], const float* p) {
+    if (V == 4) { const float4 t = *reinterpret_cast<const float4*>(p); v[0] = t.x; v[V > 1 ? 1 : 0] = t.y; v[V > 2 ? 2 : 0] = t.z; v[V > 3 ? 3 : 0] = t.w; }
+    else if (V == 2) { const float2 t = *reinterpret_cast<const float2*>(p); v[0] = t.x; v[V > 1 ? 1 : 0] = t.y; }
+    else v[0] = *p;
 }
 
 template <int MT>
 struct SkinnyCfg {
-    static constexpr int kStages = 6;
+    static constexpr int kStages = MT == 16 ? 5 : MT == 32 ? 4 : 3;      // as many as leave room for two CTAs per SM
     static constexpr int kBBytes = MT * kBK * 2;
     static constexpr int kStageBytes = kABytes + kBBytes;
-    static constexpr int kRingBytes = kStages * kStageBytes;
-    static constexpr int kBarOffset = kRingBytes;
+    static constexpr int kMaxSplits = 8;
+    static constexpr int kRedOffset = kStages * kStageBytes;              // partials of the other CTAs [splits - 1][128][share] fp32
+    static constexpr int kRedTokens = MT == 16 ? 24 : MT == 32 ? 48 : 72; // the largest (splits - 1) * share, with 7 CTAs
+    static constexpr int kBarOffset = kRedOffset + kRedTokens * kTileA * 4;
     static constexpr int kSmemBytes = kBarOffset + 256 + 1024;
     static constexpr int kTmemCols = MT < 32 ? 32 : MT;
-    static constexpr int kPeerBytes = MT * kTileA * 4;                   // one peer's partial tile, fp32
-    static constexpr int kMaxSplits = (1 + kRingBytes / kPeerBytes) < 8 ? (1 + kRingBytes / kPeerBytes) : 8;
+    static_assert(2 * (kSmemBytes + MT * 4 + 1024) <= 228 * 1024, "two CTAs per SM");
 };
+
+// The cluster's sum: CTA r adds the partials of tokens [r * share, (r + 1) * share) in rank order.  V = 4, or share where that is smaller: tokens
+// per remote store.  (A pair of CTAs exchanges one store of a lane in about three cycles, whatever its width: single values cost 0.2 us per token.)
+template <int MT, int V>
+__device__ __forceinline__ void cluster_sum(float (&acc)[MT], float* red, float* self, uint64_t* red_full, int rank, int splits, int share, int m_count, int own,
+                                            int row, const WaitCtx& ctx) {
+    const uint32_t there = smem_u32(red) + row * share * 4, bar = smem_u32(red_full);
+#pragma unroll
+    for (int j = 0; j < MT; j += V) {
+        if (j >= m_count) break;
+        const int dst = j / share, at = j - dst * share;
+        if (dst == rank) {
+#pragma unroll
+            for (int e = 0; e < V; ++e) self[row * share + at + e] = acc[j + e];
+        } else {
+            const int slot = rank < dst ? rank : rank - 1;
+            st_async<V>(map_to_cta(there + (slot * kTileA * share + at) * 4, dst), &acc[j], map_to_cta(bar, dst));
+        }
+    }
+    if (own == 0) return;
+    mbar_wait_warp<true>(red_full, 0, ctx, 0x54);
+#pragma unroll
+    for (int j = 0; j < (MT / 2 < V ? V : MT / 2); j += V) {
+        if (j >= own) break;
+        float sum[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) sum[e] = 0.f;
+        for (int r = 0; r < splits; ++r) {               // fixed order: bit-reproducible
+            float v[V];
+            load_v<V>(v, (r == rank ? self : red + (r < rank ? r : r - 1) * kTileA * share) + row * share + j);
+#pragma unroll
+            for (int e = 0; e < V; ++e) sum[e] = r == 0 ? v[e] : sum[e] + v[e];
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[j + e] = sum[e];
+    }
+}
 
 template <int MT, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -358,16 +405,21 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::kBarOffset);
     uint64_t* empty = full + C::kStages;
     uint64_t* acc_full = empty + C::kStages;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    uint64_t* red_full = acc_full + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(red_full + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = splits > 1 ? cluster_rank() : 0;
+    const int rank = splits > 1 ? static_cast<int>(cluster_ctarank()) : 0;
     const int nt = blockIdx.x / splits;
     const int k_blocks = (p.K + kBK - 1) / kBK;
     const int kb_per = (k_blocks + splits - 1) / splits;
-    const int kb0 = static_cast<int>(rank) * kb_per;
+    const int kb0 = rank * kb_per;
     const int nkb = max(0, min(k_blocks, kb0 + kb_per) - kb0);
+    const int m_count = min(p.M, MT);
+    int share = (m_count + splits - 1) / splits;                     // tokens that a CTA of the cluster finishes: 1, 2 or a multiple of 4
+    if (splits > 1 && share > 2) share = (share + 3) & ~3;
+    const int tok0 = rank * share, own = max(0, min(m_count - tok0, share));
     const WaitCtx ctx{abort_flag, p.status};
     __shared__ float s_inv_rms[MT];
 
@@ -375,7 +427,10 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
         *abort_flag = 0;
         for (int i = 0; i < C::kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         mbar_init(acc_full, 1);
+        mbar_init(red_full, 1);
         mbar_fence_init();
+        const int wide = min(share, 4);
+        mbar_arrive_expect_tx(red_full, splits > 1 ? static_cast<uint32_t>((splits - 1) * ((own + wide - 1) / wide * wide) * kTileA * 4) : 0u);
         tma_prefetch_desc(&maps.a);
         tma_prefetch_desc(&maps.b);
     }
@@ -384,16 +439,21 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (splits > 1) cluster_arrive();             // this CTA's barriers exist; waited for before the first remote store
     // Programmatic dependent launch: the next kernel of the stream may be scheduled as soon as every CTA of
     // this grid is here, and this grid was scheduled while its predecessor was still running.  Weights do
     // not depend on the predecessor, so their first ring of TMA loads goes out BEFORE griddepcontrol.wait
     // and streams while the predecessor finishes; only the activation loads and the epilogue's global
-    // accesses wait for it.
+    // accesses wait for it.  (Fetching the rest of the slice into L2 as well made dependent products slower.)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     float acc[MT];
 #pragma unroll
     for (int j = 0; j < MT; ++j) acc[j] = 0.0f;
+    const int n = nt * kTileA + (warp & 3) * 32 + lane;              // the epilogue thread's W row
+    constexpr int kHeld = EPI == VB200_EPI_ADD_F32 ? (MT <= 16 ? MT : MT / 2) : 1;
+    float held[kHeld];                                               // residual values of the CTA's own tokens
+    float gain = 0.f;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -414,6 +474,8 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
                 tma_load_2d(st + kABytes, &maps.b, &full[s], (kb0 + i) * kBK, 0);
             }
         }
+        __syncwarp();
+        if (splits > 1) cluster_wait();
     } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, kTileA, MT);
@@ -431,15 +493,24 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
             }
             umma_commit(acc_full);       // completes once every MMA above has finished (also after a break)
         }
+        __syncwarp();
+        if (splits > 1) cluster_wait();
     } else {
         const int quarter = warp & 3;
+        if (splits > 1) cluster_wait();
         asm volatile("griddepcontrol.wait;" ::: "memory");      // before any global access of the epilogue
-        if (p.rms_rows != nullptr && rank == 0) {
-            // deferred RMSNorm: 1/rms of the token rows, computed while the weights stream (these warps are idle
+        if (EPI == VB200_EPI_ADD_F32 && n < p.N) {
+#pragma unroll
+            for (int j = 0; j < kHeld; ++j)
+                if (j < own) held[j] = __ldcg(static_cast<const float*>(p.out) + static_cast<long long>(tok0 + j) * p.ldo + n);
+            if (p.scaled_copy != nullptr) gain = __ldg(p.copy_scale + n);
+        }
+        if (p.rms_rows != nullptr) {
+            // deferred RMSNorm: 1/rms of the CTA's own token rows, computed while the weights stream (these warps are idle
             // until the accumulator is complete); one warp per row, every load of a 2048-column chunk in flight
-            const int m_count = min(p.M, MT), nv = p.rms_dim / 4;
-            for (int j = warp - 2; j < m_count; j += 4) {
-                const float4* hr = reinterpret_cast<const float4*>(p.rms_rows + static_cast<long long>(j) * p.rms_ld);
+            const int nv = p.rms_dim / 4;
+            for (int j = warp - 2; j < own; j += 4) {
+                const float4* hr = reinterpret_cast<const float4*>(p.rms_rows + static_cast<long long>(tok0 + j) * p.rms_ld);
                 float ss = 0.f;
                 for (int c0 = 0; c0 < nv; c0 += 512) {
                     float4 v[16];
@@ -469,36 +540,20 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
             }
         }
         tc_fence_before();
-    }
 
-    if (splits > 1) {
-        // (1) every CTA of the cluster has finished reading its ring, so the leader's ring can hold the partials
-        cluster_sync_all();
-        if (warp >= 2 && rank != 0) {
-            const int row = (warp & 3) * 32 + lane;
-            const uint32_t base = map_to_rank(smem_u32(smem), 0) + (rank - 1) * C::kPeerBytes + row * 4;
-#pragma unroll
-            for (int j = 0; j < MT; ++j) st_cluster_f32(base + j * (kTileA * 4), acc[j]);
+        if (splits > 1) {
+            const int row = quarter * 32 + lane;
+            float* red = reinterpret_cast<float*>(smem + C::kRedOffset);
+            float* self = reinterpret_cast<float*>(smem);       // this CTA's own partials, where its ring was: every product has read it
+            if (share >= 4) cluster_sum<MT, 4>(acc, red, self, red_full, rank, splits, share, m_count, own, row, ctx);
+            else if (share == 2) cluster_sum<MT, 2>(acc, red, self, red_full, rank, splits, share, m_count, own, row, ctx);
+            else cluster_sum<MT, 1>(acc, red, self, red_full, rank, splits, share, m_count, own, row, ctx);
         }
-        // (2) partials are visible in the leader's shared memory
-        cluster_sync_all();
-        if (warp >= 2 && rank == 0) {
-            const int row = (warp & 3) * 32 + lane;
-            const float* red = reinterpret_cast<const float*>(smem);
-            for (int r = 1; r < splits; ++r) {           // fixed order: bit-reproducible
-#pragma unroll
-                for (int j = 0; j < MT; ++j) acc[j] += red[((r - 1) * MT + j) * kTileA + row];
-            }
-        }
-    }
 
-    if (warp >= 2 && rank == 0) {
-        const int n = nt * kTileA + (warp & 3) * 32 + lane;
-        const int m_count = min(p.M, MT);
         if (p.rms_rows != nullptr) {
             asm volatile("bar.sync 2, 128;" ::: "memory");       // s_inv_rms written by the four epilogue warps
 #pragma unroll
-            for (int j = 0; j < MT; ++j) acc[j] *= (j < m_count ? s_inv_rms[j] : 0.f);
+            for (int j = 0; j < MT; ++j) acc[j] *= (j < own ? s_inv_rms[j] : 0.f);
         }
         if (p.bias != nullptr && n < p.N) {
             const float bv = __ldg(p.bias + n);
@@ -509,25 +564,27 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
             __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
 #pragma unroll
             for (int j = 0; j < MT; ++j) {
+                if (j >= own) break;
                 const float other = __shfl_xor_sync(0xFFFFFFFFu, acc[j], 1);     // odd lanes hold the `up` rows
-                if (j < m_count && !(lane & 1) && n + 1 < p.N)
-                    out[static_cast<long long>(j) * p.ldo + (n >> 1)] = __float2bfloat16_rn(gate_f<EPI>(acc[j]) * other);
+                if (!(lane & 1) && n + 1 < p.N)
+                    out[static_cast<long long>(tok0 + j) * p.ldo + (n >> 1)] = __float2bfloat16_rn(gate_f<EPI>(acc[j]) * other);
             }
         } else if (n < p.N) {
 #pragma unroll
             for (int j = 0; j < MT; ++j) {
-                if (j >= m_count) break;
-                const long long idx = static_cast<long long>(j) * p.ldo + n;
+                if (j >= own) break;
+                const long long idx = static_cast<long long>(tok0 + j) * p.ldo + n;
                 if (EPI == VB200_EPI_RELU2) {
                     const float r = fmaxf(acc[j], 0.f);
                     static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16_rn(r * r);
                 } else if (EPI == VB200_EPI_BF16) static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16_rn(acc[j]);
                 else if (EPI == VB200_EPI_F32) static_cast<float*>(p.out)[idx] = acc[j];
                 else {
-                    const float hv = static_cast<float*>(p.out)[idx] + (p.addend != nullptr ? acc[j] + p.addend[idx] : acc[j]);
+                    const float was = j < kHeld ? held[j < kHeld ? j : 0] : static_cast<float*>(p.out)[idx];
+                    const float hv = was + (p.addend != nullptr ? acc[j] + p.addend[idx] : acc[j]);
                     static_cast<float*>(p.out)[idx] = hv;
                     if (p.scaled_copy != nullptr)
-                        static_cast<__nv_bfloat16*>(p.scaled_copy)[static_cast<long long>(j) * p.N + n] = __float2bfloat16_rn(hv * __ldg(p.copy_scale + n));
+                        static_cast<__nv_bfloat16*>(p.scaled_copy)[static_cast<long long>(tok0 + j) * p.N + n] = __float2bfloat16_rn(hv * gain);
                 }
             }
         }
@@ -535,6 +592,8 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, C::kTmemCols);
+    // a CTA exits with nothing on its way to it: it has counted all that the others send, except after an expired wait
+    if (splits > 1 && *abort_flag) { __syncwarp(); cluster_arrive(); cluster_wait(); }
     abort_linger(abort_flag);
 }
 
@@ -624,14 +683,17 @@ int launch_wide(cudaStream_t s, const LinearParams& p) {
     return VB200_OK;
 }
 
+// K slices per tile of 128 rows.  The time of a grid goes with the K blocks of its busiest SM as long as all CTAs are resident at once (two per SM);
+// among equals more slices, whose sums overlap better.  8 tokens, slices: 88 tiles x 32 blocks 1: 14.8, 2: 12.9, 3: 11.2, 4: 14.0 us;
+// 66 x 32 2: 9.7, 3: 8.7, 4: 8.6, 5: 11.8 us; 16 x 88 4: 9.7, 7: 7.3, 8: 7.4 us; 250 x 32 1: 22.6, 2: 28.0 us.
 int pick_splits(int n_tiles, int k_blocks, int max_splits, int sms) {
-    int want = (sms + n_tiles - 1) / n_tiles;            // enough CTAs to touch every SM
-    if (want > max_splits) want = max_splits;
-    if (want > k_blocks) want = k_blocks;
-    if (want < 1) want = 1;
-    for (int s = want; s <= max_splits && s <= k_blocks; ++s)
-        if (k_blocks % s == 0) return s;                 // equal K slices when a nearby count allows it
-    return want;
+    int best = 1, best_cost = 1 << 30;
+    for (int s = 1; s <= max_splits && s <= k_blocks; ++s) {
+        if (s > 1 && n_tiles * s > 2 * sms) break;
+        const int cost = (n_tiles * s + sms - 1) / sms * ((k_blocks + s - 1) / s);
+        if (cost <= best_cost) { best_cost = cost; best = s; }
+    }
+    return best;
 }
 
 template <int MT, int EPI>
