@@ -2,13 +2,15 @@
 // nn::Linear::weight, src/nn/linear.cpp:19, whose forward is matmul(input, weight.transpose(0,1)),
 // src/nn/linear.cpp:41-48) on the sm_100a tensor cores, fp32 accumulation in TMEM.
 //
-// Two kernels share the TMA / tcgen05 plumbing:
-//   linear_wide_kernel    M > 16 (prompt processing).  Persistent CTAs walk 128 x 256 output tiles;
-//                         x rows are the UMMA M operand, W rows the N operand; 4-stage TMA ring,
+// Three kernels share the TMA / tcgen05 plumbing:
+//   linear_pair_kernel    M > 64 (prompt processing).  Persistent pairs of CTAs walk 256 x 256 output tiles;
+//                         x rows are the UMMA M operand, W rows the N operand; TMA ring,
 //                         two TMEM accumulators so the epilogue of one tile overlaps the next mainloop.
-//   linear_skinny_kernel  M <= 16 (one token per sequence).  The product is weight-bandwidth bound,
+//   linear_wide_kernel    the same with single CTAs and 128 x 256 tiles: grouped rows, and few rows
+//                         beyond a multiple of 256.
+//   linear_skinny_kernel  M <= 64 (one token per sequence).  The product is weight-bandwidth bound,
 //                         so the roles swap: 128 W rows are the UMMA M operand and the (zero padded)
-//                         16 token rows the N operand; K is split over the CTAs of a thread-block
+//                         16, 32 or 64 token rows the N operand; K is split over the CTAs of a thread-block
 //                         cluster, which scatter their partial tiles through distributed shared
 //                         memory; each CTA sums and finishes its tokens in a fixed order (deterministic).
 // Epilogues (fused, per output element): store bf16 | store fp32 | fp32 accumulate into the residual
@@ -75,9 +77,26 @@ template <int EPI> constexpr bool kGated = EPI == VB200_EPI_SWIGLU || EPI == VB2
 // the gate's activation of a gated epilogue
 template <int EPI> __device__ __forceinline__ float gate_f(float g) { return EPI == VB200_EPI_REGLU ? fmaxf(g, 0.f) : silu_f(g); }
 
-// One output element group of the wide kernel: 32 consecutive columns of one row.
+// The residual values that 32 consecutive columns of one row are added to; loaded ahead of the product they wait for.
+__device__ __forceinline__ void load_row32(const LinearParams& p, int row, int col0, uint32_t (&was)[32]) {
+    const float* out = static_cast<const float*>(p.out) + static_cast<long long>(row) * p.ldo + col0;
+    if (col0 + 32 <= p.N) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uint32_t w[8];
+            ld_global_v8(out + 8 * j, w);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) was[8 * j + e] = w[e];
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) was[j] = col0 + j < p.N ? __float_as_uint(out[j]) : 0u;
+    }
+}
+
+// One output element group of the tiled kernels: 32 consecutive columns of one row; `was`: their residual values (+= epilogue).
 template <int EPI>
-__device__ __forceinline__ void store_row32(const LinearParams& p, int row, int col0, uint32_t (&acc)[32]) {
+__device__ __forceinline__ void store_row32(const LinearParams& p, int row, int col0, uint32_t (&acc)[32], const uint32_t (&was)[32]) {
     if (p.row_scale != nullptr) {                // deferred RMSNorm: this row's 1/rms
         const float rs = __ldg(p.row_scale + row);
 #pragma unroll
@@ -102,7 +121,9 @@ __device__ __forceinline__ void store_row32(const LinearParams& p, int row, int 
         if (n_out == 16) {
             st_global_v8(out, packed);
         } else {
-            for (int j = 0; j < n_out; ++j) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (j >= n_out) break;
                 const uint32_t u = packed[j >> 1];
                 reinterpret_cast<uint16_t*>(out)[j] = static_cast<uint16_t>((j & 1) ? (u >> 16) : (u & 0xFFFF));
             }
@@ -131,32 +152,31 @@ __device__ __forceinline__ void store_row32(const LinearParams& p, int row, int 
                 st_global_v8(out + 16 * j, w8);
             }
         } else {
-            for (int j = 0; j < n_valid; ++j) out[j] = __float2bfloat16_rn(__uint_as_float(acc[j]));
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (j < n_valid) out[j] = __float2bfloat16_rn(__uint_as_float(acc[j]));
         }
     } else {
         float* out = static_cast<float*>(p.out) + static_cast<long long>(row) * p.ldo + col0;
         if (n_valid == 32) {
-            uint32_t hres[4][8];
-            if (EPI == VB200_EPI_ADD_F32) {                     // all four 32-byte loads of the residual in flight at once
-#pragma unroll
-                for (int j = 0; j < 4; ++j) ld_global_v8(out + 8 * j, hres[j]);
-            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint32_t w8[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     float v = __uint_as_float(acc[8 * j + e]);
-                    if (EPI == VB200_EPI_ADD_F32) v += __uint_as_float(hres[j][e]);
+                    if (EPI == VB200_EPI_ADD_F32) v += __uint_as_float(was[8 * j + e]);
                     w8[e] = __float_as_uint(v);
                     acc[8 * j + e] = w8[e];                     // the new residual value, for the scaled copy below
                 }
                 st_global_v8(out + 8 * j, w8);
             }
         } else {
-            for (int j = 0; j < n_valid; ++j) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                if (j >= n_valid) break;
                 float v = __uint_as_float(acc[j]);
-                if (EPI == VB200_EPI_ADD_F32) v += out[j];
+                if (EPI == VB200_EPI_ADD_F32) v += __uint_as_float(was[j]);
                 out[j] = v;
                 acc[j] = __float_as_uint(v);
             }
@@ -177,7 +197,9 @@ __device__ __forceinline__ void store_row32(const LinearParams& p, int row, int 
                     st_global_v8(cp + 16 * j, w8);
                 }
             } else {
-                for (int j = 0; j < n_valid; ++j) cp[j] = __float2bfloat16_rn(__uint_as_float(acc[j]) * __ldg(p.copy_scale + col0 + j));
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (j < n_valid) cp[j] = __float2bfloat16_rn(__uint_as_float(acc[j]) * __ldg(p.copy_scale + col0 + j));
             }
         }
     }
@@ -298,11 +320,11 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
             row += quarter * 32 + lane;
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
-                uint32_t acc[32];
+                uint32_t acc[32], was[32];
                 tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN + c * 32, acc);
                 tmem_ld_wait();
                 const int col0 = nt * BN + c * 32;
-                if (row < row_end && col0 < p.N) store_row32<EPI>(p, row, col0, acc);
+                if (row < row_end && col0 < p.N) store_row32<EPI>(p, row, col0, acc, was);
             }
             tc_fence_before();
             __syncwarp();
@@ -312,6 +334,164 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, C::kTmemCols);
+    abort_linger(abort_flag);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Pair kernel: out[m, n] = sum_k x[m,k] W[n,k] on tiles of 256 rows x BN columns, each by a cluster of two CTAs (cta_group::2).
+//
+// With every SM at work single CTAs wait for L2: a 128 x 256 tile reads 48 KB per 64-column K block, 148 of them 16 TB/s at
+// the rate they reached (0.45 us per block; 0.33 us with few SMs at work).  A pair reads 64 KB for twice the product: each CTA
+// loads its 128 rows of x and half of the tile's rows of W, and the tensor cores read W's halves from both.  Eight epilogue warps have
+// two chunks of the residual on their way.  4096 rows, single CTAs -> pairs: 3072 x 2048 53.4 -> 37.3 us (1380 TFLOP/s), 8448 x 2048
+// 151 -> 98 (1440), 2048 x 2048 onto the residual 52 -> 36, 2048 x 5632 95 -> 78, 11264 x 2048 gated 143 -> 131; 3003 rows, 2048 x 8448 128 -> 95.
+// ------------------------------------------------------------------------------------------------
+constexpr int kPairEpilogue = 8;                    // epilogue warps: each 32 rows x half of a tile's columns
+constexpr int kPairThreads = 64 + 32 * kPairEpilogue;
+template <int BN>
+struct PairCfg {
+    static constexpr int kBBytes = BN / 2 * kBK * 2;
+    static constexpr int kStageBytes = kABytes + kBBytes;
+    static constexpr int kStages = BN == 256 ? 6 : 8;
+    static constexpr int kBarOffset = kStages * kStageBytes;
+    static constexpr int kSmemBytes = kBarOffset + 256 + 1024;
+    static constexpr int kTmemCols = 2 * BN;                        // two accumulators
+    static_assert(kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "TMEM allocation is a power of two <= 512");
+    static_assert((2 * kStages + 5) * 8 + 8 <= 256, "barriers");
+};
+
+// TMA load whose completion bytes go to a barrier that may live in the peer CTA (shared::cluster address); no multicast
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4}], [%2];"
+        : : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
+        : "memory");
+}
+
+template <int BN, int EPI>
+__global__ void __launch_bounds__(kPairThreads, 1)
+linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
+    using C = PairCfg<BN>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::kBarOffset);       // the leader's: both CTAs' loads of a stage
+    uint64_t* empty = full + C::kStages;
+    uint64_t* acc_full = empty + C::kStages;      // [2]
+    uint64_t* acc_empty = acc_full + 2;           // [2], the leader's: both CTAs' epilogue warps
+    uint64_t* drain = acc_empty + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cta = static_cast<int>(cluster_ctarank()), pairs = gridDim.x / 2;
+    const int m_tiles = (p.M + 2 * kTileA - 1) / (2 * kTileA), n_tiles = (p.N + BN - 1) / BN, tiles = m_tiles * n_tiles;
+    const int k_blocks = (p.K + kBK - 1) / kBK;
+    const WaitCtx ctx{abort_flag, p.status};
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < C::kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 2 * kPairEpilogue); }
+        mbar_init(drain, 1);
+        mbar_fence_init();
+        tma_prefetch_desc(&maps.a);
+        tma_prefetch_desc(&maps.b);
+    }
+    if (warp == 1) { tmem_alloc2(tmem_slot, C::kTmemCols); tmem_relinquish2(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    cluster_arrive();
+    cluster_wait();                               // both CTAs' barriers exist before anything crosses the pair
+    const uint32_t tmem_base = *tmem_slot;
+    // the next kernel in the stream may be scheduled now (it waits for this grid to finish before it reads
+    // anything); the activations may come from the kernel launched just before this one
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            for (int t = blockIdx.x / 2; t < tiles && !*abort_flag; t += pairs) {
+                const int row0 = (t % m_tiles * 2 + cta) * kTileA, w0 = t / m_tiles * BN + cta * (BN / 2);      // consecutive pairs share a W tile through L2
+                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                    const int s = it % C::kStages;
+                    if (it >= C::kStages && !mbar_wait(&empty[s], ((it / C::kStages) - 1) & 1, ctx, 0x61)) break;
+                    uint8_t* st = smem + s * C::kStageBytes;
+                    if (cta == 0) mbar_arrive_expect_tx(&full[s], 2 * C::kStageBytes);
+                    const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
+                    tma_load_2d_pair(st, &maps.a, bar, kb * kBK, row0);
+                    tma_load_2d_pair(st + kABytes, &maps.b, bar, kb * kBK, w0);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            if (cta == 0) {
+                constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, 2 * kTileA, BN);
+                uint32_t it = 0, tile_no = 0;
+                bool ok = true;
+                for (int t = blockIdx.x / 2; t < tiles && ok; t += pairs, ++tile_no) {
+                    const int buf = tile_no & 1;
+                    if (tile_no >= 2) ok = mbar_wait(&acc_empty[buf], ((tile_no >> 1) - 1) & 1, ctx, 0x62);
+                    if (!ok) break;
+                    tc_fence_after();
+                    for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                        const int s = it % C::kStages;
+                        if (!mbar_wait(&full[s], (it / C::kStages) & 1, ctx, 0x63)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes);
+                        const uint64_t ad = make_smem_desc_sw128(a_addr, 16, 1024), bd = make_smem_desc_sw128(a_addr + kABytes, 16, 1024);
+#pragma unroll
+                        for (int kk = 0; kk < kBK / 16; ++kk)          // 32 bytes further, in the descriptors' units of 16
+                            umma2_ss(tmem_base + buf * BN, ad + 2 * kk, bd + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                        umma2_commit(&empty[s]);          // the stage is free in both CTAs once these MMAs have read it
+                    }
+                    if (ok) umma2_commit(&acc_full[buf]);
+                }
+                umma2_commit(drain);                      // no MMA may be in flight when TMEM is freed (also on the abort path)
+            }
+            mbar_wait(drain, 0, ctx, 0x64);
+        }
+        __syncwarp();
+    } else {
+        const int quarter = warp & 3;                 // TMEM lanes this warp may read
+        constexpr int kCols = BN / (kPairEpilogue / 4), kChunks = kCols / 32;
+        const int col_first = (warp - 2) / 4 * kCols;
+        uint32_t tile_no = 0;
+        for (int t = blockIdx.x / 2; t < tiles; t += pairs, ++tile_no) {
+            const int buf = tile_no & 1;
+            const int row = (t % m_tiles * 2 + cta) * kTileA + quarter * 32 + lane, col_tile = t / m_tiles * BN + col_first;
+            uint32_t was[2][32];                      // residual values: two chunks on their way before they are needed
+            auto ahead = [&](int c) {
+                if (EPI == VB200_EPI_ADD_F32 && c < kChunks && row < p.M && col_tile + c * 32 < p.N) load_row32(p, row, col_tile + c * 32, was[c & 1]);
+            };
+            ahead(0);
+            ahead(1);
+            if (!mbar_wait_warp(&acc_full[buf], (tile_no >> 1) & 1, ctx, 0x65)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c) {
+                uint32_t acc[32];
+                tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN + col_first + c * 32, acc);
+                tmem_ld_wait();
+                if (c + 1 == kChunks) {               // the accumulator is in registers: the next product may have its columns
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
+                }
+                const int col0 = col_tile + c * 32;
+                if (row < p.M && col0 < p.N) store_row32<EPI>(p, row, col0, acc, was[c & 1]);
+                ahead(c + 2);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();                                   // nobody signals the peer or reads its tiles any more
+    if (warp == 1) tmem_dealloc2(tmem_base, C::kTmemCols);
     abort_linger(abort_flag);
 }
 
@@ -683,6 +863,49 @@ int launch_wide(cudaStream_t s, const LinearParams& p) {
     return VB200_OK;
 }
 
+template <int BN, int EPI>
+int launch_pair(cudaStream_t s, const LinearParams& p, int sms) {
+    using C = PairCfg<BN>;
+    LinearMaps maps;
+    if (int rc = make_map_2d(&maps.a, p.x, p.M, p.K, p.ldx, kTileA)) return rc;
+    if (int rc = make_map_2d(&maps.b, p.w, p.N, p.K, p.ldw, BN / 2)) return rc;
+    auto kernel = linear_pair_kernel<BN, EPI>;
+    static thread_local bool configured[64] = {};
+    if (int rc = set_smem_once(kernel, C::kSmemBytes, configured)) return rc;
+    const int tiles = ((p.M + 2 * kTileA - 1) / (2 * kTileA)) * ((p.N + BN - 1) / BN);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * (tiles < sms / 2 ? tiles : sms / 2)));
+    cfg.blockDim = dim3(kPairThreads);
+    cfg.dynamicSmemBytes = C::kSmemBytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    VB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, p));
+    note_launch();
+    return VB200_OK;
+}
+
+// More than 64 rows.  Pairs of CTAs with tiles of 256 columns; of 128 columns while one round over the SM pairs takes them all (768 rows, 2048 x 2048:
+// 16.4 us against 21.3, 2048 x 5632 33.0 against 37.5; with more rounds the wider tile is up to 1.6 times faster); single CTAs where the rows
+// of a pair's last tile would be mostly padding and cost rounds (300 rows, 11264 x 2048: 25.1 us against 29.2).
+template <int EPI>
+int launch_many_rows(cudaStream_t s, const LinearParams& p) {
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    auto rounds = [&](int rows, int columns, int at_once) { return (((p.M + rows - 1) / rows) * ((p.N + columns - 1) / columns) + at_once - 1) / at_once; };
+    if (rounds(2 * kTileA, 128, sms / 2) == 1) return launch_pair<128, EPI>(s, p, sms);
+    const int pair = rounds(2 * kTileA, 256, sms / 2), single = rounds(kTileA, 256, sms);
+    if (single * 4 < pair * 3) return launch_wide<256, EPI>(s, p);
+    return launch_pair<256, EPI>(s, p, sms);
+}
+
 // K slices per tile of 128 rows.  The time of a grid goes with the K blocks of its busiest SM as long as all CTAs are resident at once (two per SM);
 // among equals more slices, whose sums overlap better.  8 tokens, slices: 88 tiles x 32 blocks 1: 14.8, 2: 12.9, 3: 11.2, 4: 14.0 us;
 // 66 x 32 2: 9.7, 3: 8.7, 4: 8.6, 5: 11.8 us; 16 x 88 4: 9.7, 7: 7.3, 8: 7.4 us; 250 x 32 1: 22.6, 2: 28.0 us.
@@ -738,7 +961,7 @@ int launch_epi(cudaStream_t s, const LinearParams& p) {
     if (p.M <= 16) return launch_skinny<16, EPI>(s, p);
     if (p.M <= 32) return launch_skinny<32, EPI>(s, p);
     if (p.M <= 64) return launch_skinny<64, EPI>(s, p);
-    return launch_wide<256, EPI>(s, p);
+    return launch_many_rows<EPI>(s, p);
 }
 
 }  // namespace
