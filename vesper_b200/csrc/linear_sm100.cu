@@ -321,9 +321,10 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
                 uint32_t acc[32], was[32];
+                const int col0 = nt * BN + c * 32;
+                if (EPI == VB200_EPI_ADD_F32 && row < row_end && col0 < p.N) load_row32(p, row, col0, was);
                 tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN + c * 32, acc);
                 tmem_ld_wait();
-                const int col0 = nt * BN + c * 32;
                 if (row < row_end && col0 < p.N) store_row32<EPI>(p, row, col0, acc, was);
             }
             tc_fence_before();
