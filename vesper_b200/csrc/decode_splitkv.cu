@@ -194,6 +194,12 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_splitkv_kernel(Dec
     // cluster merge: first phase of the cluster barrier, arrived at once and waited for only before the first access to
     // the leader's shared memory (every CTA of the cluster must have started by then; by that time it long has)
     if (p.cluster_merge && gridDim.x > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], CW); }
+        sm->abort_flag = 0;
+        mbar_fence_init();
+    }
+    __syncthreads();
     // launched with the programmatic-dependent-launch attribute: q / k_new / v_new and the length array
     // may come from the kernel just before this one
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -212,12 +218,6 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_splitkv_kernel(Dec
     const int k_end = min(len, k_begin + p.chunk);                  // cached keys [k_begin, k_end)
     const bool owns_new = !nothing && sl.append && (len / p.chunk == split);
     const int ntiles = (!nothing && k_end > k_begin) ? (k_end - k_begin + kTile - 1) / kTile : 0;
-    if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], CW); }
-        sm->abort_flag = 0;
-        mbar_fence_init();
-    }
-    __syncthreads();
     const WaitCtx abort_flag{&sm->abort_flag, p.status};
 
     const T* kc = static_cast<const T*>(p.k_cache.ptr) + b * p.k_cache.sb + kvh * p.k_cache.sh;
@@ -247,6 +247,16 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_splitkv_kernel(Dec
 #pragma unroll
             for (int i = 0; i < 4; ++i) st.o[h][i] = make_float2(0.f, 0.f);
 
+        // the queries, and the new token where this split owns it: on their way while the angles are computed
+        uint4 qraw[NREP], kraw = make_uint4(0, 0, 0, 0), vraw = kraw;
+#pragma unroll
+        for (int h = 0; h < NREP; ++h)
+            qraw[h] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.q.ptr) + b * p.q.sb + (kvh * NREP + h) * p.q.sh + l16 * 8);
+        const bool brings_new = owns_new && warp == 0 && lane < 16;
+        if (brings_new) {
+            kraw = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.k_new.ptr) + b * p.k_new.sb + kvh * p.k_new.sh + l16 * 8);
+            vraw = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.v_new.ptr) + b * p.v_new.sb + kvh * p.v_new.sh + l16 * 8);
+        }
         // rotation angles of the query / new token for this lane's 4 pairs
         float cs[4], sn[4];
         if (p.rope) {
@@ -257,9 +267,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_splitkv_kernel(Dec
         const float qscale = p.scale * kLog2e;
 #pragma unroll
         for (int h = 0; h < NREP; ++h) {
-            const T* qp = static_cast<const T*>(p.q.ptr) + b * p.q.sb + (kvh * NREP + h) * p.q.sh + l16 * 8;
-            uint4 raw = *reinterpret_cast<const uint4*>(qp);
-            const uint32_t* u = &raw.x;
+            const uint32_t* u = &qraw[h].x;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 float2 t = Elem<T>::unpack2(u[i]);
@@ -273,11 +281,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_splitkv_kernel(Dec
         }
 
         // new token: rotate k, stage k/v in shared memory, write the cache row
-        if (owns_new && warp == 0 && lane < 16) {
-            const T* kn = static_cast<const T*>(p.k_new.ptr) + b * p.k_new.sb + kvh * p.k_new.sh + l16 * 8;
-            const T* vn = static_cast<const T*>(p.v_new.ptr) + b * p.v_new.sb + kvh * p.v_new.sh + l16 * 8;
-            uint4 kraw = *reinterpret_cast<const uint4*>(kn);
-            uint4 vraw = *reinterpret_cast<const uint4*>(vn);
+        if (brings_new) {
             {
                 // this step scores the new key in fp32; the cache gets its 16-bit rounding
                 uint32_t* u = &kraw.x;
