@@ -412,22 +412,31 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_splitkv_kernel(Dec
             const int d = tid;
             // members without keys stored nothing: splits beyond the sequence are a suffix
             const unsigned nvalid = min(nsp, static_cast<unsigned>((total + p.chunk - 1) / p.chunk));
+            // heads inside, so that their loads and exponentials overlap: with the heads outside, this was a
+            // chain of NREP * nvalid steps (300 keys of 16/4 heads, in a chain of calls: 7.26 -> 6.36 us)
+            float M[NREP], L[NREP], acc[NREP];
 #pragma unroll
-            for (int h = 0; h < NREP; ++h) {
-                float M = -INFINITY;
-                for (unsigned r = 0; r < nvalid; ++r) M = fmaxf(M, rx[(r * NREP + h) * (D + 2) + D]);
-                float L = 0.f, acc = 0.f;
-                for (unsigned r = 0; r < nvalid; ++r) {
+            for (int h = 0; h < NREP; ++h) { M[h] = -INFINITY; L[h] = 0.f; acc[h] = 0.f; }
+            for (unsigned r = 0; r < nvalid; ++r) {
+#pragma unroll
+                for (int h = 0; h < NREP; ++h) M[h] = fmaxf(M[h], rx[(r * NREP + h) * (D + 2) + D]);
+            }
+            for (unsigned r = 0; r < nvalid; ++r) {
+#pragma unroll
+                for (int h = 0; h < NREP; ++h) {
                     const float* pr = rx + (r * NREP + h) * (D + 2);
                     const float mr = pr[D];
-                    const float w = (mr == -INFINITY) ? 0.f : fast_exp2(mr - M);
-                    L += pr[D + 1] * w;
-                    acc += pr[d] * w;
+                    const float w = (mr == -INFINITY) ? 0.f : fast_exp2(mr - M[h]);
+                    L[h] += pr[D + 1] * w;
+                    acc[h] += pr[d] * w;
                 }
+            }
+#pragma unroll
+            for (int h = 0; h < NREP; ++h) {
                 const int hq = kvh * NREP + h;
-                const float o = (total > 0) ? acc / L : 0.f;
+                const float o = (total > 0) ? acc[h] / L[h] : 0.f;
                 static_cast<T*>(p.o.ptr)[b * p.o.sb + hq * p.o.sh + d] = Elem<T>::from_f(o);
-                if (p.lse && d == 0) p.lse[static_cast<long long>(b) * p.Hq + hq] = M * kLn2 + logf(L);
+                if (p.lse && d == 0) p.lse[static_cast<long long>(b) * p.Hq + hq] = M[h] * kLn2 + logf(L[h]);
             }
         }
     }
