@@ -32,3 +32,22 @@ def test_cluster_sum(cuda, M, splits):
         gated = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
         assert ((z.double() - gated).abs() - gated.abs() / 256).max().item() < 1e-4
     capi.check_kernel_status(0)
+
+
+@pytest.mark.parametrize("N,K", [(2048, 2048), (3072, 2048), (11264, 2048), (8448, 2048), (2048, 5632), (160, 4096), (32000, 512), (8960, 2240), (304, 456)])
+@pytest.mark.parametrize("M", [1, 8, 17, 40])
+def test_default_slices(cuda, M, N, K):
+    """The slices that the library chooses fix the order of a product's sums, and with it every bit of the result: one per SM and tile of 128
+    weight rows, up to 8 (5 above 32 rows), the next larger number that divides the blocks of 64 columns where there is one."""
+    import torch
+    from vesper_b200 import capi
+    tiles, blocks, most = -(-N // 128), -(-K // 64), 5 if M > 32 else 8
+    want = max(1, min(-(-torch.cuda.get_device_properties(cuda).multi_processor_count // tiles), most, blocks))
+    want = next((s for s in range(want, min(most, blocks) + 1) if blocks % s == 0), want)
+    g = torch.Generator(device=cuda).manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g, device=cuda).bfloat16(), torch.randn(N, K, generator=g, device=cuda).bfloat16()
+    chosen, stated = torch.empty(M, N, device=cuda), torch.empty(M, N, device=cuda)
+    capi.linear_ex(x, w, chosen, epilogue=capi.EPI_F32)
+    capi.linear_ex(x, w, stated, epilogue=capi.EPI_F32, splits=want)
+    assert torch.equal(chosen, stated)
+    capi.check_kernel_status(0)

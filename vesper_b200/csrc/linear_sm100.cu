@@ -505,7 +505,7 @@ linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
 // sum is scattered: CTA r finishes tokens [r, r + 1) * share of the 128 rows, every other CTA stores its partials of them straight
 // into r's shared memory (st.async, counted by a barrier of r), and r adds them in rank order (bit-reproducible) while it already
 // holds the residual rows that they go onto.  Dependent products of 8 tokens, one leading CTA's sum behind two cluster
-// barriers -> now: 2048 x 2048 8.2 -> 4.4 us, 2048 x 5632 10.6 -> 7.7, 11264 x 2048 14.2 -> 10.6 (with 3 slices for 2), 160 x 4096 5.7 -> 5.2; 32000 x
+// barriers -> now: 2048 x 2048 8.2 -> 4.4 us, 2048 x 5632 10.6 -> 7.7, 11264 x 2048 14.2 -> 12.9, 160 x 4096 5.7 -> 5.2; 32000 x
 // 2048, one slice, 22.4 -> 22.6.
 // ------------------------------------------------------------------------------------------------
 // stores of V values to another CTA's shared memory, counted by the barrier `bar` there (both shared::cluster addresses)
@@ -531,9 +531,9 @@ struct SkinnyCfg {
     static constexpr int kStages = MT == 16 ? 5 : MT == 32 ? 4 : 3;      // as many as leave room for two CTAs per SM
     static constexpr int kBBytes = MT * kBK * 2;
     static constexpr int kStageBytes = kABytes + kBBytes;
-    static constexpr int kMaxSplits = 8;
+    static constexpr int kMaxSplits = MT == 64 ? 5 : 8;
     static constexpr int kRedOffset = kStages * kStageBytes;              // partials of the other CTAs [splits - 1][128][share] fp32
-    static constexpr int kRedTokens = MT == 16 ? 24 : MT == 32 ? 48 : 72; // the largest (splits - 1) * share, with 7 CTAs
+    static constexpr int kRedTokens = MT == 16 ? 24 : MT == 32 ? 48 : 64; // the largest (splits - 1) * share: 7 CTAs, with 64 tokens 5
     static constexpr int kBarOffset = kRedOffset + kRedTokens * kTileA * 4;
     static constexpr int kSmemBytes = kBarOffset + 256 + 1024;
     static constexpr int kTmemCols = MT < 32 ? 32 : MT;
@@ -907,17 +907,18 @@ int launch_many_rows(cudaStream_t s, const LinearParams& p) {
     return launch_pair<256, EPI>(s, p, sms);
 }
 
-// K slices per tile of 128 rows.  The time of a grid goes with the K blocks of its busiest SM as long as all CTAs are resident at once (two per SM);
-// among equals more slices, whose sums overlap better.  8 tokens, slices: 88 tiles x 32 blocks 1: 14.8, 2: 12.9, 3: 11.2, 4: 14.0 us;
-// 66 x 32 2: 9.7, 3: 8.7, 4: 8.6, 5: 11.8 us; 16 x 88 4: 9.7, 7: 7.3, 8: 7.4 us; 250 x 32 1: 22.6, 2: 28.0 us.
+// K slices per tile of 128 rows: enough CTAs to touch every SM, equal slices when a nearby count allows it.  The slices fix the order in which a
+// product's fp32 sums are added, so the count follows from N, K and the device alone and the same call keeps the same bits.  (Slices that minimise the K blocks
+// of the busiest SM instead are faster at some sizes -- 8 tokens, 88 tiles x 32 blocks 3: 11.2 us against 2: 12.9 -- but sum in another order: the
+// logits of whole models moved by 0.5 %, 2-8 % further from their 64-bit values.)
 int pick_splits(int n_tiles, int k_blocks, int max_splits, int sms) {
-    int best = 1, best_cost = 1 << 30;
-    for (int s = 1; s <= max_splits && s <= k_blocks; ++s) {
-        if (s > 1 && n_tiles * s > 2 * sms) break;
-        const int cost = (n_tiles * s + sms - 1) / sms * ((k_blocks + s - 1) / s);
-        if (cost <= best_cost) { best_cost = cost; best = s; }
-    }
-    return best;
+    int want = (sms + n_tiles - 1) / n_tiles;
+    if (want > max_splits) want = max_splits;
+    if (want > k_blocks) want = k_blocks;
+    if (want < 1) want = 1;
+    for (int s = want; s <= max_splits && s <= k_blocks; ++s)
+        if (k_blocks % s == 0) return s;
+    return want;
 }
 
 template <int MT, int EPI>
