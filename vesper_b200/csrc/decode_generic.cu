@@ -1,11 +1,11 @@
 // Split-KV decode for every shape the two tuned kernels do not take: fp32 caches (the reference's own cache
-// format, src/nn/transformer.cpp:40-41), head_dim other than 64 and 128 (any multiple of 8 up to 128), any number of
-// query heads per KV head, cache rows with a stride.  Same contract, grid (split, kv_head, batch), workspace layout
+// format, src/nn/transformer.cpp:40-41), head_dim other than 64 and 128 (any multiple of 8 up to 128), other numbers of
+// query heads per KV head than 1, 2, 4 and 8, cache rows with a stride.  Same contract, grid (split, kv_head, batch), workspace layout
 // and combine kernel as decode_splitkv.cu: RoPE of q and of the new k (src/nn/functional.cpp:424-494), append of the
 // new row (KVCache::update, src/nn/transformer.cpp:56-93), attention of the one query row of every head of the group
 // over keys [k_begin, k_end) of the split with each K / V row fetched once per KV head, partial (O/l, m, l) per head.
 // CUDA cores, fp32 math; written for coverage and correctness (parity 1e-4 in fp32), not tuned: the serving
-// formats (16-bit, head_dim 64 and 128, groups of 1, 2, 4 and 8) never come here.
+// formats (16-bit, contiguous cache rows, head_dim 64 and 128, groups of 1, 2, 4 and 8) never come here.
 #include "kernels.h"
 
 namespace vb200 {

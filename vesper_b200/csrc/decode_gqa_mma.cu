@@ -1,5 +1,4 @@
-// Split-KV decode with the products on the tensor cores: head_dim 128 for groups of 4 and 8 query heads per KV head, head_dim 64 for
-// groups of 1, 2, 4 and 8.
+// Split-KV decode for head_dim 128 and groups of 8 query heads per KV head (Hq / Hkv == 8), and of 4 over long splits.
 //
 // Same contract as decode_splitkv_kernel (grid (split, kv_head, batch), partial (O/l, m, l) per head
 // into the workspace, RoPE of q / new k and the cache append fused in), but the two products run on
@@ -67,33 +66,25 @@ struct __align__(16) MmaSmem {
 
 // Per-warp running state, in MMA fragment layout: this thread owns head h = lane / 4 and, of every
 // 8-wide column tile, columns (lane % 4) * 2 + {0, 1}.
-template <int D>
 struct FragState {
-    float o[D / 8][2];  // output accumulator: D / 8 dim tiles x 2 columns
+    float o[16][2];     // output accumulator: 16 dim tiles x 2 columns
     float m;            // running reference max of head h (log2 units)
     float l;            // this thread's share of the running sum of head h
 };
 
 // CW consumer warps (16 keys of every 64-key tile each) + 1 producer warp.
-//
-// head_dim 64 keeps the softmax weights in 32 bits as the general kernel it took these calls from does: hi + lo halves, the low
-// ones in rows 8-15 of the A tile (padding otherwise), so a product yields both partial sums and costs nothing more.  A 64-key tile is
-// 16 KB there, so the ring has twice the stages.  Measured against the general kernel, which reads a key per warp at a time:
-// see launch_decode_64.
-template <typename T, int D, int NREP, int CW, int kStages, int MINB>
+template <typename T, int NREP, int CW, int kStages, int MINB>
 __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(const __grid_constant__ KvMaps maps, DecodeParams p) {
     static_assert(CW * 16 == kTileM, "one 16-key slice per consumer warp");
-    static_assert(D == 64 || D == 128, "one or two 64-column boxes");
-    constexpr bool kSplitP = D == 64;                        // weights as hi + lo halves
-    constexpr int kSteps = D / 16, kTiles8 = D / 8;
+    constexpr int D = 128;
     static_assert(NREP >= 1 && NREP <= 8, "the heads of a group are rows 0..NREP-1 of the 16-row MMA tile");
     constexpr int kRowBytes = D * 2;
-    constexpr int kMatBytes = (D / 64) * kBoxBytes;          // one K or V tile = one box per 64 dims
+    constexpr int kMatBytes = 2 * kBoxBytes;                 // one K or V tile = two boxes (dims 0-63, 64-127)
     constexpr int kStageBytes = 2 * kMatBytes;
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem_raw = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
-    float* newk = reinterpret_cast<float*>(smem_raw + kStages * kStageBytes);           // rotated new key, fp32 [D]
-    T* newv = reinterpret_cast<T*>(smem_raw + kStages * kStageBytes + D * 4);           // new value [D]
+    float* newk = reinterpret_cast<float*>(smem_raw + kStages * kStageBytes);           // rotated new key, fp32 [128]
+    T* newv = reinterpret_cast<T*>(smem_raw + kStages * kStageBytes + D * 4);           // new value [128]
     MmaSmem<CW, kStages>* sm = reinterpret_cast<MmaSmem<CW, kStages>*>(smem_raw + kStages * kStageBytes + D * 4 + kRowBytes);
 
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
@@ -128,7 +119,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
     const T* vc = static_cast<const T*>(p.v_cache.ptr) + b * p.v_cache.sb + kvh * p.v_cache.sh;
 
     if (warp == CW) {
-        // ---------------- producer: one lane issues a TMA box per 64 dims of K and of V ----------------
+        // ---------------- producer: one lane issues four TMA boxes per tile ----------------
         if (lane == 0) {
             for (int t = 0; t < ntiles; ++t) {
                 const int s = t % kStages;
@@ -136,11 +127,10 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
                 const int row0 = k_begin + t * kTileM;
                 unsigned char* dst = smem_raw + s * kStageBytes;
                 mbar_arrive_expect_tx(&sm->full[s], kStageBytes);         // rows past the cache capacity arrive as zeros and count too
-#pragma unroll
-                for (int x = 0; x < D / 64; ++x) {
-                    tma_load_4d(dst + x * kBoxBytes, &maps.k, &sm->full[s], 64 * x, row0, kvh, b);
-                    tma_load_4d(dst + kMatBytes + x * kBoxBytes, &maps.v, &sm->full[s], 64 * x, row0, kvh, b);
-                }
+                tma_load_4d(dst, &maps.k, &sm->full[s], 0, row0, kvh, b);
+                tma_load_4d(dst + kBoxBytes, &maps.k, &sm->full[s], 64, row0, kvh, b);
+                tma_load_4d(dst + kMatBytes, &maps.v, &sm->full[s], 0, row0, kvh, b);
+                tma_load_4d(dst + kMatBytes + kBoxBytes, &maps.v, &sm->full[s], 64, row0, kvh, b);
             }
         }
         return;
@@ -152,20 +142,20 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
 
     // rotated query in A-fragment layout: step ks covers dims [16 ks, 16 ks + 16); this thread holds the
     // pairs (16 ks + 2 cq, +1) and (16 ks + 8 + 2 cq, +1) of head hh -- a register is one RoPE pair
-    uint32_t qa[kSteps][2], qlo[kSteps][2];      // q = hi + lo in the 16-bit type: the scores keep fp32-class accuracy in q
+    uint32_t qa[8][2], qlo[8][2];      // q = hi + lo in the 16-bit type: the scores keep fp32-class accuracy in q
     const float pos = __int2float_rn(p.q_positions ? p.q_positions[b] : static_cast<int>(p.pos_offset) + len);
     {
         // The 16 angles a thread needs depend on cq only: the 8 threads that share cq compute two each
         // (thread hh: step ks = hh) and pass them round with shuffles.
         float my_cs[2] = {1.f, 1.f}, my_sn[2] = {0.f, 0.f};
-        if (p.rope && hh < kSteps) {
+        if (p.rope) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) sincosf(pos * p.inv_freq.v[hh * 8 + half * 4 + cq], &my_sn[half], &my_cs[half]);
         }
         const bool live = hh < NREP;                          // rows NREP..7 of the tile are padding as well
         const T* qp = static_cast<const T*>(p.q.ptr) + b * p.q.sb + (kvh * NREP + (live ? hh : 0)) * p.q.sh;
 #pragma unroll
-        for (int ks = 0; ks < kSteps; ++ks) {
+        for (int ks = 0; ks < 8; ++ks) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 const int d0 = ks * 16 + half * 8 + cq * 2;
@@ -183,7 +173,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
     }
 
     // new token (one warp): rotate k, stage k (fp32) and v in shared memory, write the cache row
-    if (owns_new && warp == 0 && lane < kTiles8) {
+    if (owns_new && warp == 0 && lane < 16) {
         const int l16 = lane;
         const T* kn = static_cast<const T*>(p.k_new.ptr) + b * p.k_new.sb + kvh * p.k_new.sh + l16 * 8;
         const T* vn = static_cast<const T*>(p.v_new.ptr) + b * p.v_new.sb + kvh * p.v_new.sh + l16 * 8;
@@ -209,22 +199,11 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
         *reinterpret_cast<uint4*>(const_cast<T*>(vc) + static_cast<long long>(len) * D + l16 * 8) = vraw;
     }
 
-    FragState<D> st;
+    FragState st;
     st.m = -INFINITY; st.l = 0.f;
 #pragma unroll
-    for (int n = 0; n < kTiles8; ++n) { st.o[n][0] = 0.f; st.o[n][1] = 0.f; }
+    for (int n = 0; n < 16; ++n) { st.o[n][0] = 0.f; st.o[n][1] = 0.f; }
     float pad0 = 0.f, pad1 = 0.f;                 // accumulators of the zero rows 8..15 (stay zero)
-    float olo[kSplitP ? kTiles8 : 1][2];          // rows 8..15: what the low halves of the weights add
-#pragma unroll
-    for (int n = 0; n < (kSplitP ? kTiles8 : 1); ++n) { olo[n][0] = 0.f; olo[n][1] = 0.f; }
-    auto rescale = [&](float alpha) {
-#pragma unroll
-        for (int n = 0; n < kTiles8; ++n) { st.o[n][0] *= alpha; st.o[n][1] *= alpha; }
-        if constexpr (kSplitP) {
-#pragma unroll
-            for (int n = 0; n < kTiles8; ++n) { olo[n][0] *= alpha; olo[n][1] *= alpha; }
-        }
-    };
 
     const uint32_t smem_base = smem_u32(smem_raw);
     // ldmatrix lane addressing: lanes 8j..8j+7 supply the row addresses of matrix j
@@ -241,8 +220,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
                 // ragged last tile: rows past nk hold whatever the cache holds there; P is 0 for them but
                 // 0 * NaN would poison O, so their V rows are cleared (a row is 128 bytes in each box)
                 unsigned char* vrow = smem_raw + s * kStageBytes + kMatBytes;
-                for (int i = lane; i < (key0 + 16 - nk) * kTiles8; i += 32) {
-                    const int r = nk + i / kTiles8, c = i % kTiles8;
+                for (int i = lane; i < (key0 + 16 - nk) * 16; i += 32) {
+                    const int r = nk + (i >> 4), c = i & 15;
                     *reinterpret_cast<uint4*>(vrow + (c >> 3) * kBoxBytes + r * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
                 }
                 __syncwarp();
@@ -252,7 +231,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) { sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f; }
 #pragma unroll
-            for (int kp = 0; kp < D / 32; ++kp) {             // 32 dims per ldmatrix.x4
+            for (int kp = 0; kp < 4; ++kp) {                  // 32 dims per ldmatrix.x4
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt) {
                     uint32_t kb[4];
@@ -282,33 +261,26 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
                 const float alpha = (st.m == -INFINITY) ? 0.f : fast_exp2(st.m - bm);
                 st.l *= alpha;
                 st.m = bm;
-                rescale(alpha);
+#pragma unroll
+                for (int n = 0; n < 16; ++n) { st.o[n][0] *= alpha; st.o[n][1] *= alpha; }
             }
             float pv[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) { pv[i] = (sv[i] == -INFINITY) ? 0.f : fast_exp2(sv[i] - st.m); st.l += pv[i]; }
-            uint32_t pa[4] = {Elem<T>::pack2(pv[0], pv[1]), 0u, Elem<T>::pack2(pv[2], pv[3]), 0u};
-            if constexpr (kSplitP) {
-                const float2 h0 = Elem<T>::unpack2(pa[0]), h1 = Elem<T>::unpack2(pa[2]);
-                pa[1] = Elem<T>::pack2(pv[0] - h0.x, pv[1] - h0.y);
-                pa[3] = Elem<T>::pack2(pv[2] - h1.x, pv[3] - h1.y);
-            }
-            // ---- O += P V: D / 8 dim tiles, two per ldmatrix.x4.trans ----
+            const uint32_t pa[4] = {Elem<T>::pack2(pv[0], pv[1]), 0u, Elem<T>::pack2(pv[2], pv[3]), 0u};
+            // ---- O += P V: 16 dim tiles, two per ldmatrix.x4.trans ----
 #pragma unroll
-            for (int dp = 0; dp < D / 16; ++dp) {
+            for (int dp = 0; dp < 8; ++dp) {
                 uint32_t vb[4];
                 // matrices: (keys 8 (lm_mat & 1).., dims 16 dp + 8 (lm_mat >> 1) ..), transposed on load
                 ldmatrix_x4_trans(vb, vs_addr + (dp >> 2) * kBoxBytes + ((lm_mat & 1) * 8 + lm_row) * 128 +
                                           ((((dp & 3) * 2 + (lm_mat >> 1)) ^ lm_row) << 4));
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int n = 2 * dp + e;
-                    float& lo0 = kSplitP ? olo[kSplitP ? n : 0][0] : pad0;
-                    float& lo1 = kSplitP ? olo[kSplitP ? n : 0][1] : pad1;
-                    float c[4] = {st.o[n][0], st.o[n][1], lo0, lo1};
-                    MmaOp<T>::mma(c, pa, vb[2 * e], vb[2 * e + 1]);
-                    st.o[n][0] = c[0]; st.o[n][1] = c[1]; lo0 = c[2]; lo1 = c[3];
-                }
+                float c0[4] = {st.o[2 * dp][0], st.o[2 * dp][1], pad0, pad1};
+                MmaOp<T>::mma(c0, pa, vb[0], vb[1]);
+                st.o[2 * dp][0] = c0[0]; st.o[2 * dp][1] = c0[1]; pad0 = c0[2]; pad1 = c0[3];
+                float c1[4] = {st.o[2 * dp + 1][0], st.o[2 * dp + 1][1], pad0, pad1};
+                MmaOp<T>::mma(c1, pa, vb[2], vb[3]);
+                st.o[2 * dp + 1][0] = c1[0]; st.o[2 * dp + 1][1] = c1[1]; pad0 = c1[2]; pad1 = c1[3];
             }
         }
         __syncwarp();
@@ -318,13 +290,13 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
     // ---- the new token (warp 0): scored in fp32 against the staged row ----
     if (owns_new && warp == 0) {
         __syncwarp();
-        // dot of head hh: this thread covers a quarter of the dims of q (re-read, rotated again in fp32)
-        const T* qp = static_cast<const T*>(p.q.ptr) + b * p.q.sb + (kvh * NREP + (hh < NREP ? hh : 0)) * p.q.sh + cq * (D / 4);
+        // dot of head hh: this thread covers dims cq*32 .. cq*32+31 of q (re-read, rotated again in fp32)
+        const T* qp = static_cast<const T*>(p.q.ptr) + b * p.q.sb + (kvh * NREP + (hh < NREP ? hh : 0)) * p.q.sh + cq * 32;
         float dot = 0.f;
 #pragma unroll
-        for (int i = 0; i < D / 8; ++i) {
+        for (int i = 0; i < 16; ++i) {
             float2 t = Elem<T>::unpack2(*reinterpret_cast<const uint32_t*>(qp + 2 * i));
-            const int d0 = cq * (D / 4) + 2 * i;
+            const int d0 = cq * 32 + 2 * i;
             if (p.rope) {
                 float sn, cs;
                 sincosf(pos * p.inv_freq.v[d0 >> 1], &sn, &cs);
@@ -341,12 +313,13 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
             const float alpha = (st.m == -INFINITY) ? 0.f : fast_exp2(st.m - s_new);
             st.l *= alpha;
             st.m = s_new;
-            rescale(alpha);
+#pragma unroll
+            for (int n = 0; n < 16; ++n) { st.o[n][0] *= alpha; st.o[n][1] *= alpha; }
         }
         const float pn = fast_exp2(s_new - st.m);
         if (cq == 0) st.l += pn;                              // once per head
 #pragma unroll
-        for (int n = 0; n < kTiles8; ++n) {
+        for (int n = 0; n < 16; ++n) {
             const float2 v2 = Elem<T>::unpack2(*reinterpret_cast<const uint32_t*>(newv + n * 8 + cq * 2));
             st.o[n][0] = fmaf(pn, v2.x, st.o[n][0]);
             st.o[n][1] = fmaf(pn, v2.y, st.o[n][1]);
@@ -358,28 +331,21 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
     l += __shfl_xor_sync(0xFFFFFFFFu, l, 1);
     l += __shfl_xor_sync(0xFFFFFFFFu, l, 2);
     asm volatile("bar.sync 1, %0;" ::"n"(CW * 32) : "memory");
-    if constexpr (kSplitP) {
-#pragma unroll
-        for (int n = 0; n < kTiles8; ++n) { st.o[n][0] += olo[n][0]; st.o[n][1] += olo[n][1]; }
-    }
-    float* go = reinterpret_cast<float*>(smem_raw);           // [CW][NREP][D]
-    float* gm = go + CW * NREP * D;                         // [CW][NREP]
+    float* go = reinterpret_cast<float*>(smem_raw);           // [CW][NREP][128]
+    float* gm = go + CW * NREP * 128;                         // [CW][NREP]
     float* gl = gm + CW * NREP;                               // [CW][NREP]
     if (hh < NREP) {
         if (cq == 0) { gm[warp * NREP + hh] = st.m; gl[warp * NREP + hh] = l; }
 #pragma unroll
-        for (int n = 0; n < kTiles8; ++n)
-            *reinterpret_cast<float2*>(go + (warp * NREP + hh) * D + n * 8 + cq * 2) = make_float2(st.o[n][0], st.o[n][1]);
+        for (int n = 0; n < 16; ++n)
+            *reinterpret_cast<float2*>(go + (warp * NREP + hh) * 128 + n * 8 + cq * 2) = make_float2(st.o[n][0], st.o[n][1]);
     }
     asm volatile("bar.sync 1, %0;" ::"n"(CW * 32) : "memory");
-    {
-        constexpr int kRows = CW * 32 / D;                    // heads merged at a time
-        const int d = tid % D;
+    if (tid < 128) {
+        const int d = tid;
         float* wsp = p.workspace + p.ws_header;
 #pragma unroll
-        for (int h0 = 0; h0 < NREP; h0 += kRows) {
-            const int h = h0 + tid / D;
-            if (h >= NREP) break;
+        for (int h = 0; h < NREP; ++h) {
             float M = -INFINITY;
 #pragma unroll
             for (int g = 0; g < CW; ++g) M = fmaxf(M, gm[g * NREP + h]);
@@ -389,14 +355,13 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
                 const float mg = gm[g * NREP + h];
                 const float w = (mg == -INFINITY) ? 0.f : fast_exp2(mg - M);
                 L += gl[g * NREP + h] * w;
-                acc += go[(g * NREP + h) * D + d] * w;
+                acc += go[(g * NREP + h) * 128 + d] * w;
             }
             float* out = wsp + ((static_cast<long long>(b) * p.Hkv + kvh) * p.num_splits + split) * NREP * (D + 2) + h * (D + 2);
             out[d] = acc / L;
             if (d == 0) { out[D] = M * kLn2M; out[D + 1] = L; }
         }
     }
-    if constexpr (D == 128) {
     if (!p.fused_exchange) return;
 
     // ---- sequence-sharded decode in one launch: the CTA that delivers the LAST split of this (batch, kv_head) merges
@@ -514,7 +479,6 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_gqa_mma_kernel(con
     exchange_rows<T, CW * 32>(p.xchg, unit, r0, r0 + NREP, rec, tid, &s_step, &s_ok,
                               [] { asm volatile("bar.sync 1, %0;" ::"n"(CW * 32) : "memory"); },
                               reinterpret_cast<float*>(stage2), kStageCap * kBlk2 * 2, 0x80000000u);
-    }
 }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -532,14 +496,12 @@ EncodeTiledFn kv_encode_fn() {
     return fn;
 }
 
-// [B,Hkv,cap,D] cache view -> 4-D map (D, rows, Hkv, B), box [64 dims][64 rows], 128-byte swizzle.
-int make_kv_map(CUtensorMap* m, int dtype, const View4& v, int D, int rows, int H, int B) {
+// [B,Hkv,cap,128] cache view -> 4-D map (D, rows, Hkv, B), box [64 dims][64 rows], 128-byte swizzle.
+int make_kv_map(CUtensorMap* m, int dtype, const View4& v, int rows, int H, int B) {
     EncodeTiledFn enc = kv_encode_fn();
     if (!enc) return set_detail(VB200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(B)};
+    cuuint64_t dims[4] = {128, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(B)};
     cuuint64_t strides[3] = {static_cast<cuuint64_t>(v.ss) * 2, static_cast<cuuint64_t>(v.sh) * 2, static_cast<cuuint64_t>(v.sb) * 2};
-    if (H == 1) strides[1] = strides[0];             // the stride of a single element is never used and may be anything
-    if (B == 1) strides[2] = strides[0];
     for (int i = 0; i < 3; ++i) if (strides[i] == 0) strides[i] = 16;
     cuuint32_t box[4] = {64, kTileM, 1, 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
@@ -557,12 +519,11 @@ int make_kv_map(CUtensorMap* m, int dtype, const View4& v, int D, int rows, int 
 }  // namespace
 
 // Launches the split kernel; the caller follows with the common combine kernel.
-template <typename T, int D, int NREP>
+template <typename T, int NREP>
 int launch_decode_gqa_mma_split(cudaStream_t s, const DecodeParams& p) {
-    constexpr int CW = 4, kStages = D == 128 ? 3 : 6, MINB = 2;
-    constexpr int kRingBytes = kStages * 2 * (D / 64) * kBoxBytes;
-    constexpr size_t smem = static_cast<size_t>(kRingBytes) + D * 4 + D * 2 + sizeof(MmaSmem<CW, kStages>) + 1024;
-    static_assert(CW * NREP * D * 4 + 2 * CW * NREP * 4 <= kRingBytes, "merge buffers must fit in the ring");
+    constexpr int CW = 4, kStages = 3, MINB = 2;
+    constexpr size_t smem = static_cast<size_t>(kStages) * 4 * kBoxBytes + 128 * 4 + 128 * 2 + sizeof(MmaSmem<CW, kStages>) + 1024;
+    static_assert(CW * NREP * 128 * 4 + 2 * CW * NREP * 4 <= kStages * 4 * kBoxBytes, "merge buffers must fit in the ring");
     // the maps of this thread's last call, reused while the cache views are unchanged (a decode loop calls with the same
     // caches step after step)
     struct Key {
@@ -579,12 +540,12 @@ int launch_decode_gqa_mma_split(cudaStream_t s, const DecodeParams& p) {
     const Key key{p.dtype, p.cache_cap, p.Hkv, p.B, p.k_cache, p.v_cache};
     if (!cached_valid || !(cached_key == key)) {
         cached_valid = false;
-        if (int rc = make_kv_map(&maps.k, p.dtype, p.k_cache, D, p.cache_cap, p.Hkv, p.B)) return rc;
-        if (int rc = make_kv_map(&maps.v, p.dtype, p.v_cache, D, p.cache_cap, p.Hkv, p.B)) return rc;
+        if (int rc = make_kv_map(&maps.k, p.dtype, p.k_cache, p.cache_cap, p.Hkv, p.B)) return rc;
+        if (int rc = make_kv_map(&maps.v, p.dtype, p.v_cache, p.cache_cap, p.Hkv, p.B)) return rc;
         cached_key = key;
         cached_valid = true;
     }
-    auto kernel = decode_gqa_mma_kernel<T, D, NREP, CW, kStages, MINB>;
+    auto kernel = decode_gqa_mma_kernel<T, NREP, CW, kStages, MINB>;
     static thread_local bool configured[64] = {};      // per device ordinal: the attribute belongs to the device's context
     int dev = 0;
     VB200_CUDA_TRY(cudaGetDevice(&dev));
@@ -606,15 +567,10 @@ int launch_decode_gqa_mma_split(cudaStream_t s, const DecodeParams& p) {
     VB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, p));
     return VB200_OK;
 }
-#define VB200_INSTANTIATE(D, NREP)                                                                   \
-    template int launch_decode_gqa_mma_split<__nv_bfloat16, D, NREP>(cudaStream_t, const DecodeParams&); \
-    template int launch_decode_gqa_mma_split<__half, D, NREP>(cudaStream_t, const DecodeParams&);
-VB200_INSTANTIATE(128, 8)
-VB200_INSTANTIATE(128, 4)
-VB200_INSTANTIATE(64, 8)
-VB200_INSTANTIATE(64, 4)
-VB200_INSTANTIATE(64, 2)
-VB200_INSTANTIATE(64, 1)
-#undef VB200_INSTANTIATE
+template int launch_decode_gqa_mma_split<__nv_bfloat16, 8>(cudaStream_t, const DecodeParams&);
+template int launch_decode_gqa_mma_split<__half, 8>(cudaStream_t, const DecodeParams&);
+template int launch_decode_gqa_mma_split<__nv_bfloat16, 4>(cudaStream_t, const DecodeParams&);
+template int launch_decode_gqa_mma_split<__half, 4>(cudaStream_t, const DecodeParams&);
 
 }  // namespace vb200
+

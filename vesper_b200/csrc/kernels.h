@@ -129,8 +129,8 @@ __device__ __forceinline__ StepLen step_length(const DecodeParams& p, int b) {
 int decode_tile_keys();
 int launch_decode_generic_split(cudaStream_t s, const DecodeParams& p);   // decode_generic.cu
 int launch_decode(cudaStream_t s, const DecodeParams& p);
-// decode_gqa_mma.cu: split kernel with warp-MMA products (head_dim 128: Hq / Hkv of 4 and 8; 64: 1, 2, 4 and 8); same workspace layout
-template <typename T, int D, int NREP> int launch_decode_gqa_mma_split(cudaStream_t s, const DecodeParams& p);
+// decode_gqa_mma.cu: split kernel with warp-MMA products (instantiated for Hq / Hkv of 4 and 8); same workspace layout
+template <typename T, int NREP> int launch_decode_gqa_mma_split(cudaStream_t s, const DecodeParams& p);
 int launch_lse_combine(cudaStream_t s, const float* partials, int R, long long rows, int D,
                        int dtype, void* out, float* lse);
 
