@@ -79,3 +79,26 @@ def test_backward_without_16_byte_rows(cuda, D, shift):
     got = capi.attention_bwd(do, q, k, v, o.float(), lse.float(), scale=D ** -0.5, causal=True)
     for x, want in zip(got, _reference(q, k, v, 0, True, do)):
         _close(x, want)
+
+
+@pytest.mark.parametrize("D", [40, 64, 128])
+@pytest.mark.parametrize("at", [0, 70, 100])
+@pytest.mark.parametrize("which", ["d_out", "q", "k", "v"])
+def test_backward_infinite_rows_stay_where_they_are_seen(cuda, D, at, which):
+    """Causal, 130 positions: an infinite row of one operand reaches only the gradients that depend on it; a masked position adds nothing, not 0 * inf."""
+    import torch
+    from vesper_b200 import capi
+    N = 130
+    g = torch.Generator(device=cuda).manual_seed(D + at)
+    t = dict(zip(("q", "k", "v", "d_out"), (torch.randn(1, 2, N, D, generator=g, device=cuda) for _ in range(4))))
+    o, lse = _reference(t["q"], t["k"], t["v"], 0, True)
+    want = _reference(t["q"], t["k"], t["v"], 0, True, t["d_out"])
+    t[which][:, :, at, ::2] = math.inf
+    if which in ("q", "k", "v"):                     # what a forward pass gives: rows that see the position are not finite
+        first, last = at, at + 1 if which == "q" else N
+        o[:, :, first:last], lse[:, :, first:last] = math.nan, math.nan
+    got = capi.attention_bwd(t["d_out"], t["q"], t["k"], t["v"], o.float(), lse.float(), scale=D ** -0.5, causal=True)
+    row = which in ("d_out", "q")                    # a row of queries: its own dq, and dk and dv of the keys up to it
+    clean = [[i for i in range(N) if (i != at if row else i < at)]] + [[j for j in range(N) if j > at] if row else []] * 2
+    for x, y, keep in zip(got, want, clean):
+        _close(x[:, :, keep], y[:, :, keep]) if keep else None

@@ -134,12 +134,12 @@ __device__ __forceinline__ void tile_ab(Pair (&acc)[8][2 * G], const float* A, c
     }
 }
 
-// acc[i][2 g], acc[i][2 g + 1] (columns 4 tx + 64 g .. + 3) += sum over r < 64 of A[r][8 ty + i] B[r][...]; A: row pitch 64, B swizzled
+// acc[i][2 g], acc[i][2 g + 1] (columns 4 tx + 64 g .. + 3) += sum over r0 <= r < 64 of A[r][8 ty + i] B[r][...]; A: row pitch 64, B swizzled
 // with swz_a
 template <int DMAX, int G>
-__device__ __forceinline__ void tile_atb(Pair (&acc)[8][2 * G], const float* A, const float* B, int tx, int ty) {
+__device__ __forceinline__ void tile_atb(Pair (&acc)[8][2 * G], const float* A, const float* B, int tx, int ty, int r0 = 0) {
 #pragma unroll 4
-    for (int r = 0; r < kTile; ++r) {
+    for (int r = r0; r < kTile; ++r) {
         const float4 a0 = *reinterpret_cast<const float4*>(A + r * kTile + 8 * ty), a1 = *reinterpret_cast<const float4*>(A + r * kTile + 8 * ty + 4);
         const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
         Quad b[G];
@@ -152,6 +152,52 @@ __device__ __forceinline__ void tile_atb(Pair (&acc)[8][2 * G], const float* A, 
             for (int g = 0; g < G; ++g) { fma2(acc[i][2 * g], x, b[g].lo); fma2(acc[i][2 * g + 1], x, b[g].hi); }
         }
     }
+}
+
+// The two products above for the tile on the diagonal of a causal mask, where A[r][c] with c > r stands for a position that is not seen: those are
+// left out, not multiplied by zero -- a row of B that holds an infinity would reach every row of the tile as 0 * inf.
+template <int DMAX, int PA, int K0, int KN>
+__device__ __forceinline__ void tile_ab_lower(Pair (&acc)[8][2], const float* A, const float* B, int col0, int tx, int ty) {
+    const float* a0 = A + ty * PA;
+#pragma unroll
+    for (int kk = K0; kk < K0 + KN; kk += 4) {
+        const int q = kk >> 3;                            // row ty + 8 q sees kk + e up to its own place; the rows of later i see all of this octet
+        float4 a[8];
+#pragma unroll
+        for (int i = q; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(a0 + 8 * i * PA + kk);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const Quad b = *reinterpret_cast<const Quad*>(B + (kk + e) * DMAX + 4 * (((col0 >> 2) + tx) ^ swz_b(kk)));
+#pragma unroll
+            for (int i = q; i < 8; ++i) {
+                if (i == q && (kk & 7) + e > ty) continue;
+                const Pair x = dup2(e == 0 ? a[i].x : e == 1 ? a[i].y : e == 2 ? a[i].z : a[i].w);
+                fma2(acc[i][0], x, b.lo);
+                fma2(acc[i][1], x, b.hi);
+            }
+        }
+    }
+}
+
+template <int DMAX, int G>
+__device__ __forceinline__ void tile_atb_lower(Pair (&acc)[8][2 * G], const float* A, const float* B, int tx, int ty) {
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {                         // rows 8 ty + m see columns 8 ty .. 8 ty + m
+        const int r = 8 * ty + m;
+        const float4 a0 = *reinterpret_cast<const float4*>(A + r * kTile + 8 * ty), a1 = *reinterpret_cast<const float4*>(A + r * kTile + 8 * ty + 4);
+        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const Quad b = *reinterpret_cast<const Quad*>(B + r * DMAX + 4 * ((tx + 16 * g) ^ swz_a(r)));
+#pragma unroll
+            for (int i = 0; i <= m; ++i) {
+                const Pair x = dup2(a[i]);
+                fma2(acc[i][2 * g], x, b.lo);
+                fma2(acc[i][2 * g + 1], x, b.hi);
+            }
+        }
+    }
+    tile_atb<DMAX, G>(acc, A, B, tx, ty, 8 * ty + 8);
 }
 
 __device__ __forceinline__ float4 quad4(Pair lo, Pair hi) {

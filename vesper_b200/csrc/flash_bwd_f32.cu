@@ -117,7 +117,10 @@ bwd_dkdv_kernel(AttnBwdParams p) {
             }
             group_sync<1>();
         }
-        tile_atb<DMAX, G>(acc, group == 0 ? Ps : dSs, (group == 0 ? dOs : Qs) + buf * kRows, tx, ty);
+        const float* weights_of = group == 0 ? Ps : dSs;
+        const float* rows_of = (group == 0 ? dOs : Qs) + buf * kRows;
+        if (p.causal && i0 == j0) tile_atb_lower<DMAX, G>(acc, weights_of, rows_of, tx, ty);
+        else tile_atb<DMAX, G>(acc, weights_of, rows_of, tx, ty);
     }
     float* out = group == 0 ? p.dv : p.dk;
     const float scale = group == 0 ? 1.f : p.scale;
@@ -195,7 +198,11 @@ bwd_dq_kernel(AttnBwdParams p) {
             }
         }
         __syncthreads();                          // dS is complete
-        if (DMAX == 128) tile_ab<DMAX, kPitchDs, 1, true, kTile>(acc, dSs, Ks + buf * kRows, 0, 64 * group, tx, ty);
+        if (p.causal && j0 == i0) {
+            if (DMAX == 128) tile_ab_lower<DMAX, kPitchDs, 0, kTile>(acc, dSs, Ks + buf * kRows, 64 * group, tx, ty);
+            else if (group == 0) tile_ab_lower<DMAX, kPitchDs, 0, kTile / 2>(acc, dSs, Ks + buf * kRows, 0, tx, ty);
+            else tile_ab_lower<DMAX, kPitchDs, kTile / 2, kTile / 2>(acc, dSs, Ks + buf * kRows, 0, tx, ty);
+        } else if (DMAX == 128) tile_ab<DMAX, kPitchDs, 1, true, kTile>(acc, dSs, Ks + buf * kRows, 0, 64 * group, tx, ty);
         else tile_ab<DMAX, kPitchDs, 1, true, kTile / 2>(acc, dSs, Ks + buf * kRows, group * (kTile / 2), 0, tx, ty);
     }
     if (DMAX == 64) {
