@@ -505,7 +505,7 @@ linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
 // sum is scattered: CTA r finishes tokens [r, r + 1) * share of the 128 rows, every other CTA stores its partials of them straight
 // into r's shared memory (st.async, counted by a barrier of r), and r adds them in rank order (bit-reproducible) while it already
 // holds the residual rows that they go onto.  Dependent products of 8 tokens, one leading CTA's sum behind two cluster
-// barriers -> now: 2048 x 2048 8.2 -> 4.4 us, 2048 x 5632 10.6 -> 7.7, 11264 x 2048 14.2 -> 12.9, 160 x 4096 5.7 -> 5.2; 32000 x
+// barriers -> now: 2048 x 2048 8.2 -> 4.4 us, 2048 x 5632 10.6 -> 7.7, 11264 x 2048 14.2 -> 12.0, 160 x 4096 5.7 -> 5.2; 32000 x
 // 2048, one slice, 22.4 -> 22.6.
 // ------------------------------------------------------------------------------------------------
 // stores of V values to another CTA's shared memory, counted by the barrier `bar` there (both shared::cluster addresses)
@@ -528,7 +528,8 @@ __device__ __forceinline__ void load_v(float (&v)[V], const float* p) {
 
 template <int MT>
 struct SkinnyCfg {
-    static constexpr int kStages = MT == 16 ? 5 : MT == 32 ? 4 : 3;      // as many as leave room for two CTAs per SM
+    static constexpr int kResident = 2;                                   // CTAs per SM that registers and shared memory are laid out for
+    static constexpr int kStages = MT == 16 ? 5 : MT == 32 ? 4 : 3;      // as many as leave room for them
     static constexpr int kBBytes = MT * kBK * 2;
     static constexpr int kStageBytes = kABytes + kBBytes;
     static constexpr int kMaxSplits = MT == 64 ? 5 : 8;
@@ -537,7 +538,7 @@ struct SkinnyCfg {
     static constexpr int kBarOffset = kRedOffset + kRedTokens * kTileA * 4;
     static constexpr int kSmemBytes = kBarOffset + 256 + 1024;
     static constexpr int kTmemCols = MT < 32 ? 32 : MT;
-    static_assert(2 * (kSmemBytes + MT * 4 + 1024) <= 228 * 1024, "two CTAs per SM");
+    static_assert(kResident * (kSmemBytes + MT * 4 + 1024) <= 228 * 1024, "shared memory of the CTAs of an SM");
 };
 
 // The cluster's sum: CTA r adds the partials of tokens [r * share, (r + 1) * share) in rank order.  V = 4, or share where that is smaller: tokens
@@ -578,7 +579,7 @@ __device__ __forceinline__ void cluster_sum(float (&acc)[MT], float* red, float*
 }
 
 template <int MT, int EPI>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, SkinnyCfg<MT>::kResident)
 linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, int splits) {
     using C = SkinnyCfg<MT>;
     extern __shared__ uint8_t smem_raw[];
@@ -632,8 +633,15 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
 #pragma unroll
     for (int j = 0; j < MT; ++j) acc[j] = 0.0f;
     const int n = nt * kTileA + (warp & 3) * 32 + lane;              // the epilogue thread's W row
-    constexpr int kHeld = EPI == VB200_EPI_ADD_F32 ? (MT <= 16 ? MT : MT / 2) : 1;
-    float held[kHeld];                                               // residual values of the CTA's own tokens
+    constexpr int kHeld = EPI == VB200_EPI_ADD_F32 ? 16 : 1;
+    // residual values of 16 of the CTA's own tokens at a time: 32 would take 178 registers, and only one CTA would fit an SM (33 rows on 3-stage rings, one CTA -> two:
+    // 4096 x 4096 23.6 -> 11.9 us, 2048 x 5632 17.4 -> 11.7, 8192 x 8192 38.1 -> 27.0; with one CTA and 6 stages they had been 27.7, 20.5, 62.7)
+    float held[kHeld];
+    auto load_held = [&](int j0) {
+#pragma unroll
+        for (int j = 0; j < kHeld; ++j)
+            if (j0 + j < own) held[j] = __ldcg(static_cast<const float*>(p.out) + static_cast<long long>(tok0 + j0 + j) * p.ldo + n);
+    };
     float gain = 0.f;
 
     if (warp == 0) {
@@ -681,9 +689,7 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
         if (splits > 1) cluster_wait();
         asm volatile("griddepcontrol.wait;" ::: "memory");      // before any global access of the epilogue
         if (EPI == VB200_EPI_ADD_F32 && n < p.N) {
-#pragma unroll
-            for (int j = 0; j < kHeld; ++j)
-                if (j < own) held[j] = __ldcg(static_cast<const float*>(p.out) + static_cast<long long>(tok0 + j) * p.ldo + n);
+            load_held(0);
             if (p.scaled_copy != nullptr) gain = __ldg(p.copy_scale + n);
         }
         if (p.rms_rows != nullptr) {
@@ -755,14 +761,14 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
             for (int j = 0; j < MT; ++j) {
                 if (j >= own) break;
                 const long long idx = static_cast<long long>(tok0 + j) * p.ldo + n;
+                if (EPI == VB200_EPI_ADD_F32 && j > 0 && j % kHeld == 0) load_held(j);
                 if (EPI == VB200_EPI_RELU2) {
                     const float r = fmaxf(acc[j], 0.f);
                     static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16_rn(r * r);
                 } else if (EPI == VB200_EPI_BF16) static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16_rn(acc[j]);
                 else if (EPI == VB200_EPI_F32) static_cast<float*>(p.out)[idx] = acc[j];
                 else {
-                    const float was = j < kHeld ? held[j < kHeld ? j : 0] : static_cast<float*>(p.out)[idx];
-                    const float hv = was + (p.addend != nullptr ? acc[j] + p.addend[idx] : acc[j]);
+                    const float hv = held[j % kHeld] + (p.addend != nullptr ? acc[j] + p.addend[idx] : acc[j]);
                     static_cast<float*>(p.out)[idx] = hv;
                     if (p.scaled_copy != nullptr)
                         static_cast<__nv_bfloat16*>(p.scaled_copy)[static_cast<long long>(tok0 + j) * p.N + n] = __float2bfloat16_rn(hv * gain);
