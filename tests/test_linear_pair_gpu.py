@@ -36,3 +36,25 @@ def test_pairs(cuda, M, N, K):
         gated = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
         assert ((z.double() - gated).abs() - gated.abs() / 256).max().item() < 1e-4
     capi.check_kernel_status(0)
+
+
+@pytest.mark.parametrize("K", [456, 1032])
+@pytest.mark.parametrize("M,N", [(2305, 11264), (1000, 19008)])
+def test_pairs_over_several_tiles(cuda, M, N, K):
+    """Several tiles per pair with more blocks of 64 columns than the ring has stages, and not a multiple of them: stages and their parities carry over
+    from tile to tile while the accumulators alternate."""
+    import torch
+    from vesper_b200 import capi
+    g = torch.Generator(device=cuda).manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g, device=cuda).bfloat16()
+    w = (torch.randn(N, K, generator=g, device=cuda) / K ** 0.5).bfloat16()
+    want = x.double() @ w.double().T
+    h = torch.randn(M, N, generator=g, device=cuda)
+    sum64 = h.double() + want
+    capi.linear_ex(x, w, h, epilogue=capi.EPI_ADD_F32)
+    assert (h.double() - sum64).abs().max().item() < 1e-4
+    z = torch.empty(M, N // 2, dtype=torch.bfloat16, device=cuda)
+    capi.linear_ex(x, w, z, epilogue=capi.EPI_SWIGLU)
+    gated = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
+    assert ((z.double() - gated).abs() - gated.abs() / 256).max().item() < 1e-4
+    capi.check_kernel_status(0)

@@ -428,32 +428,29 @@ linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            if (cta == 0) {
-                constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, 2 * kTileA, BN);
-                uint32_t it = 0, tile_no = 0;
-                bool ok = true;
-                for (int t = blockIdx.x / 2; t < tiles && ok; t += pairs, ++tile_no) {
-                    const int buf = tile_no & 1;
-                    if (tile_no >= 2) ok = mbar_wait(&acc_empty[buf], ((tile_no >> 1) - 1) & 1, ctx, 0x62);
-                    if (!ok) break;
+        if (lane == 0 && cta == 0) {
+            constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, 2 * kTileA, BN);
+            uint32_t it = 0, tile_no = 0;
+            bool ok = true;
+            for (int t = blockIdx.x / 2; t < tiles && ok; t += pairs, ++tile_no) {
+                const int buf = tile_no & 1;
+                if (tile_no >= 2) ok = mbar_wait(&acc_empty[buf], ((tile_no >> 1) - 1) & 1, ctx, 0x62);
+                if (!ok) break;
+                tc_fence_after();
+                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                    const int s = it % C::kStages;
+                    if (!mbar_wait(&full[s], (it / C::kStages) & 1, ctx, 0x63)) { ok = false; break; }
                     tc_fence_after();
-                    for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                        const int s = it % C::kStages;
-                        if (!mbar_wait(&full[s], (it / C::kStages) & 1, ctx, 0x63)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes);
-                        const uint64_t ad = make_smem_desc_sw128(a_addr, 16, 1024), bd = make_smem_desc_sw128(a_addr + kABytes, 16, 1024);
+                    const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes);
+                    const uint64_t ad = make_smem_desc_sw128(a_addr, 16, 1024), bd = make_smem_desc_sw128(a_addr + kABytes, 16, 1024);
 #pragma unroll
-                        for (int kk = 0; kk < kBK / 16; ++kk)          // 32 bytes further, in the descriptors' units of 16
-                            umma2_ss(tmem_base + buf * BN, ad + 2 * kk, bd + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
-                        umma2_commit(&empty[s]);          // the stage is free in both CTAs once these MMAs have read it
-                    }
-                    if (ok) umma2_commit(&acc_full[buf]);
+                    for (int kk = 0; kk < kBK / 16; ++kk)          // 32 bytes further, in the descriptors' units of 16
+                        umma2_ss(tmem_base + buf * BN, ad + 2 * kk, bd + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                    umma2_commit(&empty[s]);          // the stage is free in both CTAs once these MMAs have read it
                 }
-                umma2_commit(drain);                      // no MMA may be in flight when TMEM is freed (also on the abort path)
+                if (ok) umma2_commit(&acc_full[buf]);
             }
-            mbar_wait(drain, 0, ctx, 0x64);
+            umma2_commit(drain);                          // behind every MMA above (also after a break)
         }
         __syncwarp();
     } else {
@@ -490,6 +487,10 @@ linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
     }
     tc_fence_before();
     __syncthreads();
+    // No MMA may be in flight when TMEM is freed, also on the abort path.  Waited for behind the epilogue, by both CTAs: the limit of a wait
+    // covers the last products, not the whole walk over the tiles.
+    if (threadIdx.x == 32) mbar_wait(drain, 0, ctx, 0x64);
+    __syncwarp();
     cluster_arrive();
     cluster_wait();                                   // nobody signals the peer or reads its tiles any more
     if (warp == 1) tmem_dealloc2(tmem_base, C::kTmemCols);
