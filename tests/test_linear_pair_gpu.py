@@ -58,3 +58,22 @@ def test_pairs_over_several_tiles(cuda, M, N, K):
     gated = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
     assert ((z.double() - gated).abs() - gated.abs() / 256).max().item() < 1e-4
     capi.check_kernel_status(0)
+
+
+def test_product_longer_than_a_wait(cuda):
+    """The limit of a wait inside the kernel (2e9 cycles) is for one hand-over; a product that takes longer than that as a whole is computed in full.
+    2 n^3 operations at 148 x 8192 per cycle, the most that bf16 can do, take 2.1e9 cycles."""
+    import torch
+    from vesper_b200 import capi
+    n = 108544
+    if torch.cuda.mem_get_info(cuda)[0] < 80e9:
+        pytest.skip("three matrices of 24 GB")
+    x = torch.full((n, n), 1.0, dtype=torch.bfloat16, device=cuda)
+    w = torch.full((n, n), 2.0 ** -17, dtype=torch.bfloat16, device=cuda)
+    out = torch.zeros(n, n, dtype=torch.bfloat16, device=cuda)
+    capi.linear_ex(x, w, out)
+    capi.check_kernel_status(0)
+    del x, w
+    assert all(bool((part == n * 2.0 ** -17).all()) for part in out.split(8192))       # every partial sum is a multiple of 2^-17 below 1: exact
+    del out
+    torch.cuda.empty_cache()
