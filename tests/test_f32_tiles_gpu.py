@@ -102,3 +102,18 @@ def test_backward_infinite_rows_stay_where_they_are_seen(cuda, D, at, which):
     clean = [[i for i in range(N) if (i != at if row else i < at)]] + [[j for j in range(N) if j > at] if row else []] * 2
     for x, y, keep in zip(got, want, clean):
         _close(x[:, :, keep], y[:, :, keep]) if keep else None
+
+
+@pytest.mark.parametrize("D", [8, 32, 36, 64, 128])
+@pytest.mark.parametrize("heads", [1, 160, 400])
+@pytest.mark.parametrize("N", [16, 17, 32, 33, 65, 96, 97])
+def test_backward_on_either_side_of_the_dispatch(cuda, D, heads, N):
+    """Short sequences of few and of many heads: the general kernels or the tiled ones."""
+    import torch
+    from vesper_b200 import capi
+    g = torch.Generator(device=cuda).manual_seed(N * D + heads)
+    q, k, v, do = (torch.randn(1, heads, N, D, generator=g, device=cuda) for _ in range(4))
+    o, lse = _reference(q, k, v, 0, True)
+    got = capi.attention_bwd(do, q, k, v, o.float(), lse.float(), scale=D ** -0.5, causal=True)
+    for x, want in zip(got, _reference(q, k, v, 0, True, do)):
+        _close(x, want)

@@ -12,6 +12,7 @@
 // tiles are double-buffered, which with head_dim 128 takes all of an SM's shared memory: one CTA per SM.
 #include "f32_tiles.cuh"
 #include "kernels.h"
+#include "hybrid.cuh"
 
 namespace vb200 {
 namespace {
@@ -409,10 +410,17 @@ int launch_bwd_tiled(cudaStream_t s, const AttnBwdParams& p) {
     return VB200_OK;
 }
 
-// 16-byte rows: the tiled kernels.  (A grid's second dimension ends at 65535, far above any sequence that fits the device.)
+// 16-byte rows: the tiled kernels, except where most of a 64 x 64 tile would be padding and the general kernels' 32 x 32 tiles, several CTAs of which
+// share an SM, finish first (general / tiled, causal): up to 32 positions with head_dim up to 32 (one head, 32 x 32: 16.9 / 18.9 us), or with more heads than
+// SMs (256 heads, 32 x 64: 34.6 / 44.6 us; 1024 heads, 16 x 128: 202 / 226, but 32 x 128: 241 / 232); 65 to 96 positions of many narrow heads (1024 heads,
+// 65 x 8: 233 / 272 us, 65 x 16: 271 / 289, 65 x 32: 343 / 325; not causal 64 x 8 of 200 heads 83 / 76).  (A grid's second dimension ends at 65535, far above
+// any sequence that fits the device.)
 bool tiled_ok(const AttnBwdParams& p) {
     auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-    return p.D % 4 == 0 && (p.N + kTile - 1) / kTile <= 65535 && aligned(p.d_out) && aligned(p.q) && aligned(p.k) && aligned(p.v) && aligned(p.dq) && aligned(p.dk) && aligned(p.dv);
+    if (p.D % 4 != 0 || (p.N + kTile - 1) / kTile > 65535 || !aligned(p.d_out) || !aligned(p.q) || !aligned(p.k) || !aligned(p.v) || !aligned(p.dq) || !aligned(p.dk) || !aligned(p.dv)) return false;
+    const long long heads = static_cast<long long>(p.B) * p.H, sms = device_sm_count();
+    if (p.N <= kT) return p.D > 32 && (heads <= sms || p.D > (p.N <= 16 ? 128 : 64));
+    return !(p.causal && p.N > kTile && p.N <= 3 * kT && p.D <= 16 && heads > 2 * sms);
 }
 
 }  // namespace
