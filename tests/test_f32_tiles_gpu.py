@@ -117,3 +117,18 @@ def test_backward_on_either_side_of_the_dispatch(cuda, D, heads, N):
     got = capi.attention_bwd(do, q, k, v, o.float(), lse.float(), scale=D ** -0.5, causal=True)
     for x, want in zip(got, _reference(q, k, v, 0, True, do)):
         _close(x, want)
+
+
+@pytest.mark.parametrize("D", [40, 64, 128])
+@pytest.mark.parametrize("heads,T", [(150, 128), (150, 129), (40, 700), (150, 200)])
+def test_forward_on_either_side_of_the_dispatch(cuda, D, heads, T):
+    """Grids and lengths on both sides of the rule for four or eight query rows per thread."""
+    import torch
+    from vesper_b200 import capi
+    g = torch.Generator(device=cuda).manual_seed(T * D + heads)
+    q, k, v = (torch.randn(1, heads, T, D, generator=g, device=cuda) for _ in range(3))
+    o, lse = torch.empty_like(q), torch.empty(1, heads, T, device=cuda)
+    capi.prefill(q, k, v, o, lse, scale=D ** -0.5)
+    want_o, want_lse = _reference(q, k, v, 0, True)
+    _close(o, want_o)
+    _close(lse, want_lse)

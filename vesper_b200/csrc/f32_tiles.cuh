@@ -7,6 +7,7 @@
 //   tile_abt   C[64][64] += A[64][K] B[64][K]^T    thread: rows ty + 8 i, columns 4 tx + j; even and odd k in separate
 //                                                  halves of an accumulator pair, so no operand has to be duplicated
 //   tile_ab    C[64][N]  += A[64][64] B[64][N]     thread: rows ty + 8 i, columns 4 tx + 64 g; A values duplicated
+//   (these two also with R = 4: 256 threads, rows ty + 16 i)
 //   tile_atb   C[64][N]  += A[64][64]^T B[64][N]   thread: rows 8 ty + i, columns 4 tx + 64 g; A values duplicated
 // An 8 x 4 (8 x 8) register block reads 12 (16) 16-byte words per 128 (256) FMAs: half (three eighths) of the
 // shared-memory bandwidth at the full FMA rate; the 4 x 4 block that these kernels had before needed all of it.
@@ -53,29 +54,31 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool val
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 enum class Swizzle { None, A, B };
 
 // 64 rows from row0 on (row stride ld elements, a multiple of 4; src 16-byte aligned) into a [64][DMAX] tile; rows from `rows`
-// on and columns from D on become zeros.  All `threads` threads take part.
+// on become zeros, columns from D on stay as they are (no product reads them into a column that is kept).  All `threads` threads take part.
 template <int DMAX, Swizzle SWZ>
 __device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ src, long long ld, int row0, int rows, int D, int tid, int threads) {
     constexpr int W = DMAX / 4;
     for (int i = tid; i < kTile * W; i += threads) {
         const int r = i / W, c = i % W;
-        const bool ok = row0 + r < rows && 4 * c < D;
+        if (4 * c >= D) continue;
+        const bool ok = row0 + r < rows;
         const int at = SWZ == Swizzle::None ? c : SWZ == Swizzle::A ? (c ^ swz_a(r)) : (c ^ swz_b(r));
         cp_async16(dst + r * DMAX + 4 * at, ok ? src + (row0 + r) * ld + 4 * c : src, ok);
     }
 }
 
 // s[i][j] = sum over words c < words of A[ty + 8 i] . B[4 tx + j]; A swizzled with swz_a, B with swz_b
-template <int DMAX>
-__device__ __forceinline__ void tile_abt(float (&s)[8][4], const float* A, const float* B, int words, int tx, int ty) {
-    Pair acc[8][4];
+template <int DMAX, int R = 8>
+__device__ __forceinline__ void tile_abt(float (&s)[R][4], const float* A, const float* B, int words, int tx, int ty) {
+    Pair acc[R][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0;
     const float* a0 = A + ty * DMAX;
@@ -89,8 +92,8 @@ __device__ __forceinline__ void tile_abt(float (&s)[8][4], const float* A, const
 #pragma unroll
         for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const Quad*>(bp + j * DMAX);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const Quad a = *reinterpret_cast<const Quad*>(ap + 8 * i * DMAX);
+        for (int i = 0; i < R; ++i) {
+            const Quad a = *reinterpret_cast<const Quad*>(ap + kTile / R * i * DMAX);
 #pragma unroll
             for (int j = 0; j < 4; ++j) fma2(acc[i][j], a.lo, b[j].lo);
 #pragma unroll
@@ -98,7 +101,7 @@ __device__ __forceinline__ void tile_abt(float (&s)[8][4], const float* A, const
         }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float2 h = halves(acc[i][j]);
@@ -106,16 +109,16 @@ __device__ __forceinline__ void tile_abt(float (&s)[8][4], const float* A, const
         }
 }
 
-// acc[i][2 g], acc[i][2 g + 1] (columns col0 + 4 tx + 64 g .. + 3) += sum over k0 <= kk < k0 + KN of A[ty + 8 i][kk] B[kk][...].
+// acc[i][2 g], acc[i][2 g + 1] (columns col0 + 4 tx + 64 g .. + 3) += sum over k0 <= kk < k1, in steps of 4, of A[ty + 8 i][kk] B[kk][...].
 // A: row pitch PA; B: row pitch DMAX, swizzled with swz_b when SWZ.
-template <int DMAX, int PA, int G, bool SWZ, int KN>
-__device__ __forceinline__ void tile_ab(Pair (&acc)[8][2 * G], const float* A, const float* B, int k0, int col0, int tx, int ty) {
+template <int DMAX, int PA, int G, bool SWZ, int R = 8>
+__device__ __forceinline__ void tile_ab(Pair (&acc)[R][2 * G], const float* A, const float* B, int k0, int k1, int col0, int tx, int ty) {
     const float* a0 = A + ty * PA;
 #pragma unroll 2
-    for (int kk = k0; kk < k0 + KN; kk += 4) {
-        float4 a[8];
+    for (int kk = k0; kk < k1; kk += 4) {
+        float4 a[R];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(a0 + 8 * i * PA + kk);
+        for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4*>(a0 + kTile / R * i * PA + kk);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             Quad b[G];
@@ -125,7 +128,7 @@ __device__ __forceinline__ void tile_ab(Pair (&acc)[8][2 * G], const float* A, c
                 b[g] = *reinterpret_cast<const Quad*>(B + (kk + e) * DMAX + 4 * (SWZ ? (word ^ swz_b(kk)) : word));
             }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < R; ++i) {
                 const Pair x = dup2(e == 0 ? a[i].x : e == 1 ? a[i].y : e == 2 ? a[i].z : a[i].w);
 #pragma unroll
                 for (int g = 0; g < G; ++g) { fma2(acc[i][2 * g], x, b[g].lo); fma2(acc[i][2 * g + 1], x, b[g].hi); }

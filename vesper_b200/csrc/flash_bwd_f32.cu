@@ -203,8 +203,8 @@ bwd_dq_kernel(AttnBwdParams p) {
             if (DMAX == 128) tile_ab_lower<DMAX, kPitchDs, 0, kTile>(acc, dSs, Ks + buf * kRows, 64 * group, tx, ty);
             else if (group == 0) tile_ab_lower<DMAX, kPitchDs, 0, kTile / 2>(acc, dSs, Ks + buf * kRows, 0, tx, ty);
             else tile_ab_lower<DMAX, kPitchDs, kTile / 2, kTile / 2>(acc, dSs, Ks + buf * kRows, 0, tx, ty);
-        } else if (DMAX == 128) tile_ab<DMAX, kPitchDs, 1, true, kTile>(acc, dSs, Ks + buf * kRows, 0, 64 * group, tx, ty);
-        else tile_ab<DMAX, kPitchDs, 1, true, kTile / 2>(acc, dSs, Ks + buf * kRows, group * (kTile / 2), 0, tx, ty);
+        } else if (DMAX == 128) tile_ab<DMAX, kPitchDs, 1, true>(acc, dSs, Ks + buf * kRows, 0, kTile, 64 * group, tx, ty);
+        else tile_ab<DMAX, kPitchDs, 1, true>(acc, dSs, Ks + buf * kRows, group * (kTile / 2), (group + 1) * (kTile / 2), 0, tx, ty);
     }
     if (DMAX == 64) {
         __syncthreads();                          // every tile is consumed: the second half of the keys passes its sums through Qs

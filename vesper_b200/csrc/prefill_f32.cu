@@ -7,12 +7,14 @@
 // (src/ops/flash_attention.cpp:218-364): s = scale * q.k, causal j <= i,
 // online softmax, O = acc / l, LSE = m + ln l.
 //
-// Tiling: 64 query rows x 64 keys per step, 128 threads, products as in f32_tiles.cuh (packed fp32 FMAs, 8 x 4 and 8 x 8
-// register blocks).  A CTA keeps one K and one V tile: V arrives while the scores are computed, the next K tile during the
-// softmax and the value product, so both loads hide behind arithmetic without a second buffer, and two CTAs (head_dim 128)
-// or three (64) share an SM.  A row's 64 weights are written and read by the same half warp.
+// Tiling: 64 query rows x 64 keys per step, 128 or 256 threads, products as in f32_tiles.cuh (packed fp32 FMAs, 8 x 4 and 8 x 8
+// register blocks, or half as many rows).  A CTA keeps one K and one V tile: V arrives while the scores are computed, the next K tile during the
+// softmax and the value product, so both loads hide behind arithmetic without a second buffer, and two CTAs
+// share an SM, or three (head_dim 64 with 128 threads: 16 x 2048 x 64 360 us against 364 with two, 64 x 1024 x 16 226 against 233, although
+// 84 bytes spill).  A row's 64 weights are written and read by the same half warp.
 #include "f32_tiles.cuh"
 #include "kernels.h"
+#include "hybrid.cuh"
 
 namespace vb200 {
 
@@ -20,7 +22,6 @@ namespace {
 
 using namespace f32t;
 
-constexpr int kThreads = kGroup;
 constexpr int kPitchP = kTile + 4;     // weights: rows ty and ty + 1 of one warp in distinct banks
 
 __device__ __forceinline__ float rowgroup_max(float v) {
@@ -36,10 +37,11 @@ __device__ __forceinline__ float rowgroup_sum(float v) {
 
 template <int DMAX> constexpr int smem_floats() { return 3 * kTile * DMAX + kTile * kPitchP; }
 
-template <int DMAX>
-__global__ void __launch_bounds__(kThreads, DMAX == 64 ? 3 : 2) prefill_f32_kernel(PrefillParams p) {
+// R query rows per thread
+template <int DMAX, int R>
+__global__ void __launch_bounds__(1024 / R, R == 8 && DMAX == 64 ? 3 : 2) prefill_f32_kernel(PrefillParams p) {
     extern __shared__ __align__(16) float smem[];
-    constexpr int G = DMAX / 64;
+    constexpr int G = DMAX / 64, kThreads = 1024 / R, kStep = kTile / R;
     float* Qs = smem;
     float* Ks = Qs + kTile * DMAX;
     float* Vs = Ks + kTile * DMAX;
@@ -57,44 +59,47 @@ __global__ void __launch_bounds__(kThreads, DMAX == 64 ? 3 : 2) prefill_f32_kern
 
     int kv_end = p.Skv;
     if (p.causal) kv_end = min(p.Skv, p.start_pos + min(q0 + kTile, p.T));
+    // the first tiles of Q (unless it is rotated on the way in), K and V are on their way at once
+    if (p.q_rope_table == nullptr) load_rows<DMAX, Swizzle::A>(Qs, qg, p.q.ss, q0, p.T, D, tid, kThreads);
     load_rows<DMAX, Swizzle::B>(Ks, kg, p.k.ss, 0, kv_end, D, tid, kThreads);
     cp_async_commit();
+    load_rows<DMAX, Swizzle::None>(Vs, vg, p.v.ss, 0, kv_end, D, tid, kThreads);
+    cp_async_commit();
 
-    // Q tile (rotated on the way in when a table is given)
-    for (int i = tid; i < kTile * (DMAX / 4); i += kThreads) {
+    for (int i = p.q_rope_table != nullptr ? tid : kTile * (DMAX / 4); i < kTile * (DMAX / 4); i += kThreads) {
         const int r = i / (DMAX / 4), c = i % (DMAX / 4);
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (q0 + r < p.T && c < words) {
             x = *reinterpret_cast<const float4*>(qg + static_cast<long long>(q0 + r) * p.q.ss + c * 4);
-            if (p.q_rope_table) {
-                const float2* tp = p.q_rope_table + static_cast<long long>(q0 + r) * (D / 2) + c * 2;
-                float2 cs0 = tp[0], cs1 = tp[1];
-                float t1 = __fmul_rn(x.x, cs0.x), t2 = __fmul_rn(x.y, cs0.y), t3 = __fmul_rn(x.x, cs0.y), t4 = __fmul_rn(x.y, cs0.x);
-                x.x = __fsub_rn(t1, t2); x.y = __fadd_rn(t3, t4);
-                t1 = __fmul_rn(x.z, cs1.x); t2 = __fmul_rn(x.w, cs1.y); t3 = __fmul_rn(x.z, cs1.y); t4 = __fmul_rn(x.w, cs1.x);
-                x.z = __fsub_rn(t1, t2); x.w = __fadd_rn(t3, t4);
-            }
+            const float2* tp = p.q_rope_table + static_cast<long long>(q0 + r) * (D / 2) + c * 2;
+            float2 cs0 = tp[0], cs1 = tp[1];
+            float t1 = __fmul_rn(x.x, cs0.x), t2 = __fmul_rn(x.y, cs0.y), t3 = __fmul_rn(x.x, cs0.y), t4 = __fmul_rn(x.y, cs0.x);
+            x.x = __fsub_rn(t1, t2); x.y = __fadd_rn(t3, t4);
+            t1 = __fmul_rn(x.z, cs1.x); t2 = __fmul_rn(x.w, cs1.y); t3 = __fmul_rn(x.z, cs1.y); t4 = __fmul_rn(x.w, cs1.x);
+            x.z = __fsub_rn(t1, t2); x.w = __fadd_rn(t3, t4);
         }
         *reinterpret_cast<float4*>(Qs + r * DMAX + 4 * (c ^ swz_a(r))) = x;
     }
 
-    float m_i[8], l_i[8];
-    Pair acc[8][2 * G];
+    float m_i[R], l_i[R];
+    Pair acc[R][2 * G];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < R; ++i) {
         m_i[i] = -INFINITY; l_i[i] = 0.f;
 #pragma unroll
         for (int g = 0; g < 2 * G; ++g) acc[i][g] = 0;
     }
 
     for (int k0 = 0; k0 < kv_end; k0 += kTile) {
-        cp_async_wait_all();
-        __syncthreads();   // K has arrived (and the Q stores, the first time); the previous V tile is fully consumed
-        load_rows<DMAX, Swizzle::None>(Vs, vg, p.v.ss, k0, kv_end, D, tid, kThreads);
-        cp_async_commit();
+        if (k0 == 0) cp_async_wait_but_last(); else cp_async_wait_all();
+        __syncthreads();   // K has arrived (and Q, the first time); the previous V tile is fully consumed
+        if (k0 > 0) {
+            load_rows<DMAX, Swizzle::None>(Vs, vg, p.v.ss, k0, kv_end, D, tid, kThreads);
+            cp_async_commit();
+        }
 
-        float s[8][4];
-        tile_abt<DMAX>(s, Qs, Ks, words, tx, ty);
+        float s[R][4];
+        tile_abt<DMAX, R>(s, Qs, Ks, words, tx, ty);
 
         cp_async_wait_all();
         __syncthreads();   // V has arrived; K is fully consumed
@@ -106,8 +111,8 @@ __global__ void __launch_bounds__(kThreads, DMAX == 64 ? 3 : 2) prefill_f32_kern
         // keys past the end, or past a row's own position: only the last tiles have any
         const bool edge = k0 + kTile > p.Skv || (p.causal && k0 + kTile - 1 > p.start_pos + q0);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int row = q0 + ty + 8 * i;
+        for (int i = 0; i < R; ++i) {
+            const int row = q0 + ty + kStep * i;
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[i][j] *= p.scale;
             if (edge) {
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, DMAX == 64 ? 3 : 2) prefill_f32_kern
             const float alpha = expf(m_i[i] - m_use);       // exp(-inf) = 0 on the first tile
             float4 w;
             w.x = expf(s[i][0] - m_use); w.y = expf(s[i][1] - m_use); w.z = expf(s[i][2] - m_use); w.w = expf(s[i][3] - m_use);
-            *reinterpret_cast<float4*>(Ps + (ty + 8 * i) * kPitchP + 4 * tx) = w;
+            *reinterpret_cast<float4*>(Ps + (ty + kStep * i) * kPitchP + 4 * tx) = w;
             l_i[i] = l_i[i] * alpha + ((w.x + w.y) + (w.z + w.w));      // per-thread partial; reduced at the end
             m_i[i] = m_new;
             const Pair a2 = dup2(alpha);
@@ -131,13 +136,13 @@ __global__ void __launch_bounds__(kThreads, DMAX == 64 ? 3 : 2) prefill_f32_kern
             for (int g = 0; g < 2 * G; ++g) mul2(acc[i][g], a2);
         }
         __syncwarp();
-        tile_ab<DMAX, kPitchP, G, false, kTile>(acc, Ps, Vs, 0, 0, tx, ty);
+        tile_ab<DMAX, kPitchP, G, false, R>(acc, Ps, Vs, 0, min(kTile, kv_end - k0), 0, tx, ty);      // (weights and rows past the keys are zero)
     }
 
     float* og = static_cast<float*>(p.o.ptr) + b * p.o.sb + hq * p.o.sh;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int row = q0 + ty + 8 * i;
+    for (int i = 0; i < R; ++i) {
+        const int row = q0 + ty + kStep * i;
         const float l = rowgroup_sum(l_i[i]);
         if (row >= p.T) continue;
         const float inv = 1.0f / l;
@@ -154,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, DMAX == 64 ? 3 : 2) prefill_f32_kern
     }
 }
 
-template <int DMAX>
+template <int DMAX, int R>
 int launch_t(cudaStream_t s, const PrefillParams& p) {
     constexpr int smem = smem_floats<DMAX>() * static_cast<int>(sizeof(float));
     static thread_local bool configured[64] = {};      // per device ordinal: the attribute belongs to the device's context
@@ -162,11 +167,11 @@ int launch_t(cudaStream_t s, const PrefillParams& p) {
     VB200_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return set_detail(VB200_ERR_NO_DEVICE, "device ordinal out of range");
     if (!configured[dev]) {
-        VB200_CUDA_TRY(cudaFuncSetAttribute(prefill_f32_kernel<DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        VB200_CUDA_TRY(cudaFuncSetAttribute(prefill_f32_kernel<DMAX, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured[dev] = true;
     }
     dim3 grid((p.T + kTile - 1) / kTile, p.Hq, p.B);
-    prefill_f32_kernel<DMAX><<<grid, kThreads, smem, s>>>(p);
+    prefill_f32_kernel<DMAX, R><<<grid, 1024 / R, smem, s>>>(p);
     note_launch();
     note_prefill_kernel("prefill_f32_kernel");
     VB200_CUDA_TRY(cudaPeekAtLastError());
@@ -177,7 +182,13 @@ int launch_t(cudaStream_t s, const PrefillParams& p) {
 
 int launch_prefill_f32(cudaStream_t s, const PrefillParams& p) {
     if (p.D % 4 != 0 || p.D > 128 || p.D < 4) return set_detail(VB200_ERR_UNSUPPORTED, "fp32 attention needs head_dim % 4 == 0 and <= 128");
-    return p.D <= 64 ? launch_t<64>(s, p) : launch_t<128>(s, p);
+    // Query rows per thread: 4 (256 threads) while the grid leaves SMs with few CTAs or the sequences are short, where a tile's latency counts; 8 (128 threads),
+    // which read shared memory less, for long grids.  4 / 8 rows: one head, 64 x 32 7.7 / 10.4 us; 8 heads, 512 x 64 48.8 / 52.2; 16 heads, 1400 x 64 (352 CTAs)
+    // 201 / 262; 1024 heads, 64 x 32 35.4 / 37.4; but 128 heads, 256 x 64 (512 CTAs) 63.7 / 59.3; 4 heads, 8192 x 64 1598 / 1346.
+    const long long ctas = static_cast<long long>((p.T + kTile - 1) / kTile) * p.Hq * p.B;
+    const bool few = ctas <= 3 * device_sm_count() || p.Skv <= 2 * kTile;
+    if (p.D <= 64) return few ? launch_t<64, 4>(s, p) : launch_t<64, 8>(s, p);
+    return few ? launch_t<128, 4>(s, p) : launch_t<128, 8>(s, p);
 }
 
 }  // namespace vb200
