@@ -130,13 +130,11 @@ __global__ void kv_append_kernel(int B, int H, int Tn, int D, View4 k, View4 v, 
 // memory, writes them to the table the attention kernel rotates Q with (only the CTAs of the first (batch, head) chunk
 // do), and moves those rows of K (rotated) and V (copied) for its chunk of (batch, head) pairs -- one table kernel, one
 // launch gap and one trip of the table through L2 less than table-then-append.
-// What bounds it: the latency of its loads.  A thread has kMoves words of K and of V on their way at once, the first of them while the angles are
-// computed (the whole operator with 4 x 2048 rows x 8 heads of 128 194.1 -> 190.1 us, with 8 x 512 x 4 45.5 -> 42.2; 8 words of each take 186 registers and
-// lose it again).
+// What bounds it: the latency of its loads.  A thread has MOVES words of K and of V on their way at once, the first of them while the angles are
+// computed.
 constexpr int kRopeRows = 8;
-constexpr int kMoves = 4;
 
-template <typename T>
+template <typename T, int MOVES>
 __global__ void __launch_bounds__(256) rope_append_fused_kernel(int B, int H, int Tn, int D, View4 k, View4 v, View4 kd, View4 vd, int dst_row0,
                                                                 float2* __restrict__ table, InvFreq f, int bh_per_cta) {
     __shared__ float2 cs[kRopeRows][kMaxHalfDim];
@@ -146,21 +144,18 @@ __global__ void __launch_bounds__(256) rope_append_fused_kernel(int B, int H, in
     const int bh0 = blockIdx.y * bh_per_cta;
     const int nbh = min(bh_per_cta, B * H - bh0);
     const int per_bh = rows * vecs, total = nbh * per_bh;
-    Vec8<T> x[kMoves], y[kMoves];
-    auto place = [&](int i, int& b, int& h, int& r, int& c) {
-        const int bh = bh0 + i / per_bh, rem = i % per_bh;
-        r = rem / vecs; c = rem - r * vecs;
-        b = bh / H; h = bh - b * H;
-    };
+    Vec8<T> x[MOVES], y[MOVES];
+    int at_b[MOVES], at_h[MOVES], at_r[MOVES], at_c[MOVES];
     auto fetch = [&](int i0) {
 #pragma unroll
-        for (int u = 0; u < kMoves; ++u) {
+        for (int u = 0; u < MOVES; ++u) {
             const int i = i0 + u * 256;
             if (i >= total) break;
-            int b, h, r, c;
-            place(i, b, h, r, c);
-            x[u].load(static_cast<const T*>(k.ptr) + b * k.sb + h * k.sh + static_cast<long long>(t0 + r) * k.ss + c * 8);
-            if (v.ptr != nullptr) y[u].load(static_cast<const T*>(v.ptr) + b * v.sb + h * v.sh + static_cast<long long>(t0 + r) * v.ss + c * 8);
+            const int bh = bh0 + i / per_bh, rem = i % per_bh;
+            at_r[u] = rem / vecs; at_c[u] = rem - at_r[u] * vecs;
+            at_b[u] = bh / H; at_h[u] = bh - at_b[u] * H;
+            x[u].load(static_cast<const T*>(k.ptr) + at_b[u] * k.sb + at_h[u] * k.sh + static_cast<long long>(t0 + at_r[u]) * k.ss + at_c[u] * 8);
+            if (v.ptr != nullptr) y[u].load(static_cast<const T*>(v.ptr) + at_b[u] * v.sb + at_h[u] * v.sh + static_cast<long long>(t0 + at_r[u]) * v.ss + at_c[u] * 8);
         }
     };
     fetch(threadIdx.x);                       // on their way while the angles are computed
@@ -172,21 +167,20 @@ __global__ void __launch_bounds__(256) rope_append_fused_kernel(int B, int H, in
         if (blockIdx.y == 0 && table != nullptr) table[static_cast<long long>(t0 + r) * half + pr] = make_float2(c, sn);
     }
     __syncthreads();
-    for (int i0 = threadIdx.x; i0 < total; i0 += kMoves * 256) {
-        if (i0 >= kMoves * 256) fetch(i0);
+    for (int i0 = threadIdx.x; i0 < total; i0 += MOVES * 256) {
+        if (i0 >= MOVES * 256) fetch(i0);
 #pragma unroll
-        for (int u = 0; u < kMoves; ++u) {
+        for (int u = 0; u < MOVES; ++u) {
             const int i = i0 + u * 256;
             if (i >= total) break;
-            int b, h, r, c;
-            place(i, b, h, r, c);
+            const long long to = static_cast<long long>(dst_row0 + t0 + at_r[u]);
             float e[8];
             x[u].get(e);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) rotate_pair(e[2 * j], e[2 * j + 1], cs[r][c * 4 + j]);
+            for (int j = 0; j < 4; ++j) rotate_pair(e[2 * j], e[2 * j + 1], cs[at_r[u]][at_c[u] * 4 + j]);
             x[u].set(e);
-            x[u].store(static_cast<T*>(kd.ptr) + b * kd.sb + h * kd.sh + static_cast<long long>(dst_row0 + t0 + r) * kd.ss + c * 8);
-            if (v.ptr != nullptr) y[u].store(static_cast<T*>(vd.ptr) + b * vd.sb + h * vd.sh + static_cast<long long>(dst_row0 + t0 + r) * vd.ss + c * 8);
+            x[u].store(static_cast<T*>(kd.ptr) + at_b[u] * kd.sb + at_h[u] * kd.sh + to * kd.ss + at_c[u] * 8);
+            if (v.ptr != nullptr) y[u].store(static_cast<T*>(vd.ptr) + at_b[u] * vd.sb + at_h[u] * vd.sh + to * vd.ss + at_c[u] * 8);
         }
     }
 }
@@ -202,10 +196,14 @@ int launch_rope_append_fused(cudaStream_t s, int dtype, int B, int H, int T, int
     const int bh_per_cta = (B * H + chunks - 1) / chunks;
     chunks = (B * H + bh_per_cta - 1) / bh_per_cta;
     dim3 grid(static_cast<unsigned>(row_tiles), static_cast<unsigned>(chunks));
+    // Four words of each per thread where it has more than one.  Whole operator in bf16, one word at a time behind the angles (before) / four words
+    // everywhere / this rule: 4 x 2048 rows, 8 heads of 128 124.0 / 122.3 / 121.5 us, 1 x 300 x 4 21.3 / 22.1 / 20.8, 64 x 64 x 8 33.7 / 33.9 / 32.4.
+    const bool many = bh_per_cta * kRopeRows * (D / 8) > 256;
+    auto launch = [&](auto kernel) { kernel<<<grid, 256, 0, s>>>(B, H, T, D, k, v, k_dst, v_dst, dst_row0, table, f, bh_per_cta); };
     switch (dtype) {
-        case VB200_F32: rope_append_fused_kernel<float><<<grid, 256, 0, s>>>(B, H, T, D, k, v, k_dst, v_dst, dst_row0, table, f, bh_per_cta); break;
-        case VB200_BF16: rope_append_fused_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(B, H, T, D, k, v, k_dst, v_dst, dst_row0, table, f, bh_per_cta); break;
-        case VB200_F16: rope_append_fused_kernel<__half><<<grid, 256, 0, s>>>(B, H, T, D, k, v, k_dst, v_dst, dst_row0, table, f, bh_per_cta); break;
+        case VB200_F32: many ? launch(rope_append_fused_kernel<float, 4>) : launch(rope_append_fused_kernel<float, 1>); break;
+        case VB200_BF16: many ? launch(rope_append_fused_kernel<__nv_bfloat16, 4>) : launch(rope_append_fused_kernel<__nv_bfloat16, 1>); break;
+        case VB200_F16: many ? launch(rope_append_fused_kernel<__half, 4>) : launch(rope_append_fused_kernel<__half, 1>); break;
         default: return VB200_ERR_UNSUPPORTED;
     }
     note_launch();
