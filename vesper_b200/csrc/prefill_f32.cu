@@ -160,14 +160,15 @@ __global__ void __launch_bounds__(1024 / R, R == 8 && DMAX == 64 ? 3 : 2) prefil
 }
 
 template <int DMAX, int R>
-int launch_t(cudaStream_t s, const PrefillParams& p) {
-    constexpr int smem = smem_floats<DMAX>() * static_cast<int>(sizeof(float));
+int launch_t(cudaStream_t s, const PrefillParams& p, bool alone = false) {
+    constexpr int kSmem = smem_floats<DMAX>() * static_cast<int>(sizeof(float)), kAlone = 116 * 1024;      // two of kAlone do not fit an SM
+    const int smem = alone ? kAlone : kSmem;
     static thread_local bool configured[64] = {};      // per device ordinal: the attribute belongs to the device's context
     int dev = 0;
     VB200_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return set_detail(VB200_ERR_NO_DEVICE, "device ordinal out of range");
     if (!configured[dev]) {
-        VB200_CUDA_TRY(cudaFuncSetAttribute(prefill_f32_kernel<DMAX, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        VB200_CUDA_TRY(cudaFuncSetAttribute(prefill_f32_kernel<DMAX, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem > kAlone ? kSmem : kAlone));
         configured[dev] = true;
     }
     dim3 grid((p.T + kTile - 1) / kTile, p.Hq, p.B);
@@ -188,7 +189,11 @@ int launch_prefill_f32(cudaStream_t s, const PrefillParams& p) {
     const long long ctas = static_cast<long long>((p.T + kTile - 1) / kTile) * p.Hq * p.B;
     const bool few = ctas <= 3 * device_sm_count() || p.Skv <= 2 * kTile;
     if (p.D <= 64) return few ? launch_t<64, 4>(s, p) : launch_t<64, 8>(s, p);
-    return few ? launch_t<128, 4>(s, p) : launch_t<128, 8>(s, p);
+    // head_dim above 64, long causal grids of one to two CTAs per SM: the row tiles with the most keys are the call's length, and an SM to itself each shortens them
+    // more than a second CTA hides.  Two / one per SM: 2 heads, 8192 x 128 1861 / 1155 us; 6 heads, 2048 447 / 329; 32 heads, 512 133 / 125; 16 heads, 1024 232 / 232;
+    // but 128 heads, 128 38 / 44.
+    const bool alone = p.causal && p.Skv >= 512 && ctas > device_sm_count() && ctas <= 2 * device_sm_count();
+    return few ? launch_t<128, 4>(s, p, alone) : launch_t<128, 8>(s, p);
 }
 
 }  // namespace vb200
