@@ -99,7 +99,10 @@ typedef struct vb200_prefill_args {
                                     the cache -- the T < L shape of
                                     scaled_dot_product_attention,
                                     src/nn/functional.cpp:399-421                     */
-    void* workspace;             /* vb200_prefill_workspace_bytes() bytes, 256-aligned */
+    void* workspace;             /* vb200_prefill_workspace_bytes() bytes, 256-aligned.
+                                    fp32: the part behind the RoPE table and the rotated
+                                    keys is optional; without it the call runs on the
+                                    CUDA cores, several times slower                  */
     size_t workspace_bytes;
 } vb200_prefill_args;
 
@@ -260,7 +263,7 @@ int vb200_decode_exchange_fwd(const vb200_decode_args* a, const vb200_exchange_a
  * dQ, dK, dV of O = softmax(scale Q K^T [causal]) V from the saved O and LSE of the forward, P
  * recomputed tile by tile.  All tensors contiguous [B,H,N,D] fp32 with Hq == Hkv (the reference op
  * takes q, k, v of one shape), lse [B,H,N]; dq, dk, dv are overwritten.  Deterministic (no atomics).
- * workspace: B*H*N floats (vb200_attention_bwd_workspace_bytes).  Replaces
+ * workspace: vb200_attention_bwd_workspace_bytes; B*H*N floats are enough (CUDA cores, slower).  Replaces
  * flash_attention_backward_cuda_dispatch (src/ops/flash_attention.cpp:34-39,
  * src/ops/cuda/flash_attention.cu:546-576; CPU form src/ops/flash_attention.cpp:366-482); like the
  * reference's CUDA path it has no dropout. */

@@ -94,6 +94,7 @@ bool view_aligned(const vb200_tensor4& t, int esz) {
 struct PrefillPlan {
     bool need_table, need_krot;   // krot: rotated K without a cache goes to the workspace
     size_t table_bytes, krot_bytes, total;
+    size_t split_bytes;              // fp32 on the tensor cores: behind the rest, optional
 };
 
 PrefillPlan plan_prefill(const vb200_prefill_args* a) {
@@ -103,6 +104,8 @@ PrefillPlan plan_prefill(const vb200_prefill_args* a) {
     pl.table_bytes = pl.need_table ? align_up(static_cast<size_t>(a->T) * (a->D / 2) * sizeof(float2), 256) : 0;
     pl.krot_bytes = pl.need_krot ? align_up(static_cast<size_t>(a->B) * a->Hkv * a->T * a->D * elem_size(a->dtype), 256) : 0;
     pl.total = pl.table_bytes + pl.krot_bytes;
+    if (a->dtype == VB200_F32 && prefill_f32_on_tensor_cores(a->D, a->T, a->start_pos + a->T, a->B * a->Hq))
+        pl.split_bytes = prefill_f32_split_bytes(a->D, a->B * a->Hkv, a->start_pos + a->T);
     return pl;
 }
 
@@ -310,7 +313,8 @@ int vb200_profile_read(double* total_ms, uint64_t* launches) {
 
 size_t vb200_prefill_workspace_bytes(const vb200_prefill_args* a) {
     if (!a || a->struct_size != sizeof(vb200_prefill_args)) return 0;
-    return plan_prefill(a).total;
+    const PrefillPlan pl = plan_prefill(a);
+    return pl.total + pl.split_bytes;
 }
 
 int vb200_prefill_fwd(const vb200_prefill_args* a) {
@@ -349,6 +353,8 @@ int vb200_prefill_fwd(const vb200_prefill_args* a) {
     p.inv_freq = f;
     p.status = kernel_status_word();
     if (!p.status) return set_detail(VB200_ERR_CUDA, "cannot resolve the device status word");
+    // fp32 with a smaller workspace, or none, runs on the CUDA cores
+    if (pl.split_bytes > 0 && a->workspace && a->workspace_bytes >= pl.total + pl.split_bytes && reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0) p.split = ws + pl.total;
 
     if (ro) {
         // the cache already holds every key and value this call attends to
@@ -538,9 +544,12 @@ int vb200_repeat_kv(int device, void* stream, int32_t dtype, const vb200_tensor4
     return launch_repeat_kv(static_cast<cudaStream_t>(stream), dtype, to_view(*in), out, B, Hkv, S, D, n_rep);
 }
 
+static size_t bwd_delta_bytes(const vb200_attention_bwd_args* a) { return align_up(sizeof(float) * static_cast<size_t>(a->B) * a->H * a->N, 256); }
+
 size_t vb200_attention_bwd_workspace_bytes(const vb200_attention_bwd_args* a) {
     if (!a || a->struct_size != sizeof(vb200_attention_bwd_args) || a->B <= 0 || a->H <= 0 || a->N <= 0) return 0;
-    return align_up(sizeof(float) * static_cast<size_t>(a->B) * a->H * a->N, 256);
+    const bool terms = attention_bwd_f32_on_tensor_cores(a->D, a->N);
+    return bwd_delta_bytes(a) + (terms ? attention_bwd_f32_split_bytes(a->D, a->B * a->H, a->N) : 0);
 }
 
 int vb200_attention_bwd(const vb200_attention_bwd_args* a) {
@@ -550,7 +559,8 @@ int vb200_attention_bwd(const vb200_attention_bwd_args* a) {
     if (a->D > 128) return set_detail(VB200_ERR_UNSUPPORTED, "vb200_attention_bwd: head_dim must be <= 128");
     if (!a->d_out || !a->q || !a->k || !a->v || !a->out || !a->lse || !a->dq || !a->dk || !a->dv)
         return set_detail(VB200_ERR_INVALID_ARG, "vb200_attention_bwd: null tensor");
-    if (!a->workspace || a->workspace_bytes < vb200_attention_bwd_workspace_bytes(a))
+    // enough for the row sums: the CUDA cores; enough for the terms too, and aligned: the tensor cores
+    if (!a->workspace || a->workspace_bytes < bwd_delta_bytes(a))
         return set_detail(VB200_ERR_WORKSPACE, "vb200_attention_bwd: workspace missing or too small");
     DeviceGuard g;
     if (int rc = g.init(a->device)) return rc;
@@ -560,6 +570,10 @@ int vb200_attention_bwd(const vb200_attention_bwd_args* a) {
     p.v = static_cast<const float*>(a->v); p.out = static_cast<const float*>(a->out); p.lse = a->lse;
     p.dq = static_cast<float*>(a->dq); p.dk = static_cast<float*>(a->dk); p.dv = static_cast<float*>(a->dv);
     p.delta = static_cast<float*>(a->workspace);
+    p.status = kernel_status_word();
+    if (!p.status) return set_detail(VB200_ERR_CUDA, "cannot resolve the device status word");
+    if (attention_bwd_f32_on_tensor_cores(a->D, a->N) && a->workspace_bytes >= vb200_attention_bwd_workspace_bytes(a) && reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0)
+        p.split = static_cast<unsigned char*>(a->workspace) + bwd_delta_bytes(a);
     return launch_attention_bwd_f32(static_cast<cudaStream_t>(a->stream), p);
 }
 

@@ -5,6 +5,7 @@
 //   dQ = scale dS K;  dK = scale dS^T Q.
 // Three launches, all deterministic (no atomics): the row sums; one CTA per 64-key tile walking the query
 // tiles that see it (dK, dV in registers); one CTA per 64-query tile walking its key tiles (dQ in registers).
+// Head dims of 64 and 128 above 64 positions run on the tensor cores instead (attention_f32_sm100.cu), given the workspace.
 // CUDA cores, 64 x 64 tiles, products as in f32_tiles.cuh.  A CTA is two groups of 128 threads that hold the same
 // positions of a tile: one computes S and P, the other dO V^T and dS, at the same time; then one accumulates dV while the
 // other accumulates dK (or each one half of dQ's columns).  That keeps the register blocks at 8 x 4 and 8 x 8 -- with all
@@ -415,9 +416,12 @@ int launch_bwd_tiled(cudaStream_t s, const AttnBwdParams& p) {
 // SMs (256 heads, 32 x 64: 34.6 / 44.6 us; 1024 heads, 16 x 128: 202 / 226, but 32 x 128: 241 / 232); 65 to 96 positions of many narrow heads (1024 heads,
 // 65 x 8: 233 / 272 us, 65 x 16: 271 / 289, 65 x 32: 343 / 325; not causal 64 x 8 of 200 heads 83 / 76).  (A grid's second dimension ends at 65535, far above
 // any sequence that fits the device.)
-bool tiled_ok(const AttnBwdParams& p) {
+bool rows_aligned(const AttnBwdParams& p) {
     auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-    if (p.D % 4 != 0 || (p.N + kTile - 1) / kTile > 65535 || !aligned(p.d_out) || !aligned(p.q) || !aligned(p.k) || !aligned(p.v) || !aligned(p.dq) || !aligned(p.dk) || !aligned(p.dv)) return false;
+    return p.D % 4 == 0 && aligned(p.d_out) && aligned(p.q) && aligned(p.k) && aligned(p.v) && aligned(p.dq) && aligned(p.dk) && aligned(p.dv);
+}
+bool tiled_ok(const AttnBwdParams& p) {
+    if (!rows_aligned(p) || (p.N + kTile - 1) / kTile > 65535) return false;
     const long long heads = static_cast<long long>(p.B) * p.H, sms = device_sm_count();
     if (p.N <= kT) return p.D > 32 && (heads <= sms || p.D > (p.N <= 16 ? 128 : 64));
     return !(p.causal && p.N > kTile && p.N <= 3 * kT && p.D <= 16 && heads > 2 * sms);
@@ -425,8 +429,15 @@ bool tiled_ok(const AttnBwdParams& p) {
 
 }  // namespace
 
+// The tensor cores (attention_f32_sm100.cu) from the second block of 64 positions on.  These kernels / those: 16 heads, 512 x 64 127 / 36 us; 16, 2048 x 128
+// 1595 / 439; 1024, 96 x 64 416 / 246; one head, 65 x 64 45 / 14; but 1024 heads, 64 x 64 167 / 187, 256 heads, 64 x 128 91 / 100.
+bool attention_bwd_f32_on_tensor_cores(int D, int N) {
+    return (D == 64 || D == 128) && N > 64;
+}
+
 int launch_attention_bwd_f32(cudaStream_t s, const AttnBwdParams& p) {
     if (p.D > 128) return set_detail(VB200_ERR_UNSUPPORTED, "attention backward supports head_dim <= 128");
+    if (p.split != nullptr && rows_aligned(p) && reinterpret_cast<uintptr_t>(p.out) % 16 == 0) return launch_attention_bwd_f32_sm100(s, p, p.split);
     const long long rows = static_cast<long long>(p.B) * p.H * p.N;
     bwd_delta_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, s>>>(p.d_out, p.out, p.delta, rows, p.D);
     const int rc = tiled_ok(p) ? (p.D <= 64 ? launch_bwd_tiled<64>(s, p) : launch_bwd_tiled<128>(s, p))

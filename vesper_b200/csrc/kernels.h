@@ -49,6 +49,7 @@ struct PrefillParams {
     const float2* q_rope_table;   // [T, D/2] (cos,sin) for the query rows, or null
     InvFreq inv_freq;             // rotation frequencies (valid when q_rope_table is set)
     int* status;                  // device status word (bounded waits)
+    void* split;                  // fp32: workspace of prefill_f32_split_bytes for the tensor-core kernel, or null
 };
 int launch_prefill_f32(cudaStream_t s, const PrefillParams& p);
 int launch_prefill_sm100(cudaStream_t s, const PrefillParams& p);
@@ -141,8 +142,20 @@ struct AttnBwdParams {
     const float *d_out, *q, *k, *v, *out, *lse;   // contiguous [B,H,N,D]; lse [B,H,N]
     float *dq, *dk, *dv;
     float* delta;                                 // workspace [B,H,N]
+    int* status;                                  // device status word (bounded waits)
+    void* split;                                  // workspace of attention_bwd_f32_split_bytes, or null
 };
 int launch_attention_bwd_f32(cudaStream_t s, const AttnBwdParams& p);
+
+// ---- attention_f32_sm100.cu: the fp32 operators on the tensor cores, head_dim 64 and 128 ----
+// Bytes of workspace (256-aligned) in which the bf16 terms of the streamed operands stand.
+size_t prefill_f32_split_bytes(int D, int kv_heads, int keys);
+size_t attention_bwd_f32_split_bytes(int D, int heads, int N);
+int launch_prefill_f32_sm100(cudaStream_t s, const PrefillParams& p, void* workspace);
+int launch_attention_bwd_f32_sm100(cudaStream_t s, const AttnBwdParams& p, void* workspace);      // writes delta too
+// Whether a call of this shape takes them, given that workspace.
+bool prefill_f32_on_tensor_cores(int D, int T, int keys, int heads);
+bool attention_bwd_f32_on_tensor_cores(int D, int N);
 
 // ---- decode_exchange.cu ----
 size_t exchange_buffer_bytes(int world, long long rows, int D);

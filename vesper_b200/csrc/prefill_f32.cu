@@ -1,4 +1,5 @@
-// fp32 attention forward on CUDA cores (fp32 in, fp32 math, fp32 out).
+// fp32 attention forward on CUDA cores (fp32 in, fp32 math, fp32 out): head dims other than 64 and 128, short sequences, and calls without the workspace
+// that the tensor-core kernel (attention_f32_sm100.cu) needs.
 //
 // This is the dtype the reference's flash op runs in
 // (flash_attention_cuda_dispatch, src/ops/cuda/flash_attention.cu:518-544), so
@@ -181,6 +182,14 @@ int launch_t(cudaStream_t s, const PrefillParams& p, bool alone = false) {
 
 }  // namespace
 
+// The tensor cores (attention_f32_sm100.cu) from the second block of 64 keys on, and for short portions of many heads, whose 128-row tiles are mostly
+// padding, from 512 keys on.  This kernel / those: 16 heads, 512 x 64 50 / 21 us; 16, 2048 x 128 671 / 97; 1024, 128 x 128 199 / 154; 64 heads, 65 x 64
+// 14.7 / 12.9, but 64 x 64 10.5 / 10.8 and 1024 heads, 64 x 64 45 / 65; 16 new rows of 1024 heads behind 240 keys 125 / 132, 496 238 / 223, of 128 heads
+// behind 112 16.7 / 14.7.
+bool prefill_f32_on_tensor_cores(int D, int T, int keys, int heads) {
+    return (D == 64 || D == 128) && keys > 64 && (T > 64 || heads <= 128 || keys >= 512);
+}
+
 int launch_prefill_f32(cudaStream_t s, const PrefillParams& p) {
     if (p.D % 4 != 0 || p.D > 128 || p.D < 4) return set_detail(VB200_ERR_UNSUPPORTED, "fp32 attention needs head_dim % 4 == 0 and <= 128");
     // Query rows per thread: 4 (256 threads) while the grid leaves SMs with few CTAs or the sequences are short, where a tile's latency counts; 8 (128 threads),
@@ -188,6 +197,7 @@ int launch_prefill_f32(cudaStream_t s, const PrefillParams& p) {
     // 201 / 262; 1024 heads, 64 x 32 35.4 / 37.4; but 128 heads, 256 x 64 (512 CTAs) 63.7 / 59.3; 4 heads, 8192 x 64 1598 / 1346.
     const long long ctas = static_cast<long long>((p.T + kTile - 1) / kTile) * p.Hq * p.B;
     const bool few = ctas <= 3 * device_sm_count() || p.Skv <= 2 * kTile;
+    if (p.split != nullptr) return launch_prefill_f32_sm100(s, p, p.split);
     if (p.D <= 64) return few ? launch_t<64, 4>(s, p) : launch_t<64, 8>(s, p);
     // head_dim above 64, long causal grids of one to two CTAs per SM: the row tiles with the most keys are the call's length, and an SM to itself each shortens them
     // more than a second CTA hides.  Two / one per SM: 2 heads, 8192 x 128 1861 / 1155 us; 6 heads, 2048 447 / 329; 32 heads, 512 133 / 125; 16 heads, 1024 232 / 232;

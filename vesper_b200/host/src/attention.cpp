@@ -64,6 +64,12 @@ void flash_attention_cuda_dispatch(const Tensor& q, const Tensor& k, const Tenso
     a.scale = scale;
     a.q = view4(q); a.k = view4(k); a.v = view4(v); a.o = view4(output);
     a.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
+    Tensor ws;
+    if (const size_t need = vb200_prefill_workspace_bytes(&a)) {
+        ws = workspace(need);
+        a.workspace = ws.data_ptr<char>();
+        a.workspace_bytes = ws.numel() * 4;
+    }
     check(vb200_prefill_fwd(&a), "flash_attention");
 }
 
