@@ -254,6 +254,11 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
+// a value that the lanes of a warp share, as one the compiler knows to be shared
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xFFFFFFFFu, x, 0); }
+
+// Products take their addresses and descriptors from uniform registers.  Issue them from code that a whole warp runs, under a predicate of
+// elect_one() that is taken once: in the divergent code of `if (lane == 0)` every operand is moved there first, about 100 cycles per product.
 // D[tmem] (+)= A[smem desc] * B[smem desc]
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(

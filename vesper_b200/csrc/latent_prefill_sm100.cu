@@ -110,41 +110,50 @@ latent_prefill_sm100_kernel(const __grid_constant__ LatentMaps maps, LatentTileP
             }
         }
     } else if (warp == 5) {
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();             // (the whole warp walks: see the note at umma_ss)
+            const uint32_t tmem = uniform(bar.tmem);
+            auto commit = [&](uint64_t* to) { if (leader) umma_commit(to); };
             const uint32_t idesc_qk = make_idesc_f16(1, 0, 0, kRows, kKeys);
             const uint32_t idesc_pv = make_idesc_f16(1, 0, 1, kRows, p.n_pv);
-            const uint32_t q_addr = smem_u32(q_smem), k_addr = smem_u32(k_smem), v_addr = smem_u32(v_smem);
-            bool ok = mbar_wait(&bar.q_full, 0, ctx, 0xB3);
+            const uint64_t q_desc = make_smem_desc_sw128(smem_u32(q_smem), 16, 1024), k_desc = make_smem_desc_sw128(smem_u32(k_smem), 16, 1024),
+                           v_desc = make_smem_desc_sw128(smem_u32(v_smem), kKBox, 1024);
+            bool ok = mbar_wait_warp(&bar.q_full, 0, ctx, 0xB3);
             auto issue_qk = [&](int j) {
                 const int s = j % p.k_stages;
-                ok = mbar_wait(&bar.k_full[s], (j / p.k_stages) & 1, ctx, 0xB4);
+                ok = mbar_wait_warp(&bar.k_full[s], (j / p.k_stages) & 1, ctx, 0xB4);
                 if (!ok) return;
                 tc_fence_after();
-                const uint32_t kb = k_addr + s * nb_k * kKBox, d = tmem + (j & 1) * kKeys;
+                const uint64_t kd = k_desc + s * (nb_k * kKBox >> 4);
+                const uint32_t d = tmem + (j & 1) * kKeys;
                 for (int kk = 0; kk < p.ks_n + p.ks_r; ++kk) {
-                    const int box = kk < p.ks_n ? kk >> 2 : p.nb_n + ((kk - p.ks_n) >> 2), off = (kk < p.ks_n ? kk & 3 : (kk - p.ks_n) & 3) * 32;
-                    umma_ss(d, make_smem_desc_sw128(q_addr + box * kQBox + off, 16, 1024), make_smem_desc_sw128(kb + box * kKBox + off, 16, 1024), idesc_qk, kk > 0 ? 1u : 0u);
+                    const int box = kk < p.ks_n ? kk >> 2 : p.nb_n + ((kk - p.ks_n) >> 2), off = (kk < p.ks_n ? kk & 3 : (kk - p.ks_n) & 3) * 2;
+                    if (leader) umma_ss(d, q_desc + box * (kQBox >> 4) + off, kd + box * (kKBox >> 4) + off, idesc_qk, kk > 0 ? 1u : 0u);
                 }
-                umma_commit(&bar.s_full[j & 1]);
-                umma_commit(&bar.k_empty[s]);
+                commit(&bar.s_full[j & 1]);
+                commit(&bar.k_empty[s]);
             };
             if (ok) issue_qk(0);
             for (int j = 0; j < n_blk && ok; ++j) {
                 if (j + 1 < n_blk) issue_qk(j + 1);      // its S held P of block j-1, whose product was issued before
                 if (!ok) break;
                 const int s = j % p.v_stages;
-                ok = mbar_wait(&bar.v_full[s], (j / p.v_stages) & 1, ctx, 0xB5) && mbar_wait(&bar.p_ready[j & 1], (j >> 1) & 1, ctx, 0xB6);
+                ok = mbar_wait_warp(&bar.v_full[s], (j / p.v_stages) & 1, ctx, 0xB5) && mbar_wait_warp(&bar.p_ready[j & 1], (j >> 1) & 1, ctx, 0xB6);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t vb = v_addr + s * p.nb_v * kKBox, a = tmem + (j & 1) * kKeys;
-                for (int half = 0; half < 2; ++half)
-                    for (int kk = 0; kk < kKeys / 16; ++kk)
-                        umma_ts(tmem + 2 * kKeys, a + half * 32 + kk * 8, make_smem_desc_sw128(vb + kk * 2048, kKBox, 1024), idesc_pv, (j | half | kk) ? 1u : 0u);
-                umma_commit(&bar.o_done[j & 1]);
-                umma_commit(&bar.v_empty[s]);
+                const uint64_t vd = v_desc + s * (p.nb_v * kKBox >> 4);
+                const uint32_t a = tmem + (j & 1) * kKeys;
+                if (leader)
+#pragma unroll
+                    for (int i = 0; i < 2 * (kKeys / 16); ++i) {             // hi, then lo
+                        const int half = i / (kKeys / 16), kk = i % (kKeys / 16);
+                        umma_ts(tmem + 2 * kKeys, a + half * 32 + kk * 8, vd + kk * (2048 >> 4), idesc_pv, (j | i) ? 1u : 0u);
+                    }
+                commit(&bar.o_done[j & 1]);
+                commit(&bar.v_empty[s]);
             }
-            umma_commit(&bar.drain);                     // nothing may be in flight when TMEM is freed
-            mbar_wait(&bar.drain, 0, ctx, 0xB7);
+            commit(&bar.drain);                     // nothing may be in flight when TMEM is freed
+            mbar_wait_warp(&bar.drain, 0, ctx, 0xB7);
         }
     } else {
         const int r = threadIdx.x;                       // row of the tile = TMEM lane

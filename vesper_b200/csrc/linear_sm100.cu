@@ -272,33 +272,34 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, kTileA, BN);
-            uint32_t it = 0, tile_no = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++tile_no) {
-                const int buf = tile_no & 1;
-                if (tile_no >= 2) ok = mbar_wait(&acc_empty[buf], ((tile_no >> 1) - 1) & 1, ctx, 0x42);
-                if (!ok) break;
+        constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, kTileA, BN);
+        const bool leader = elect_one();              // (the whole warp walks: see the note at umma_ss)
+        const uint32_t tmem = uniform(tmem_base);
+        uint32_t it = 0, tile_no = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++tile_no) {
+            const int buf = tile_no & 1;
+            if (tile_no >= 2) ok = mbar_wait_warp(&acc_empty[buf], ((tile_no >> 1) - 1) & 1, ctx, 0x42);
+            if (!ok) break;
+            tc_fence_after();
+            for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                const int s = it % C::kStages;
+                if (!mbar_wait_warp(&full[s], (it / C::kStages) & 1, ctx, 0x43)) { ok = false; break; }
                 tc_fence_after();
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const int s = it % C::kStages;
-                    if (!mbar_wait(&full[s], (it / C::kStages) & 1, ctx, 0x43)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes), b_addr = a_addr + kABytes;
+                const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes);
+                const uint64_t ad = make_smem_desc_sw128(a_addr, 16, 1024), bd = make_smem_desc_sw128(a_addr + kABytes, 16, 1024);
+                if (leader) {
 #pragma unroll
-                    for (int kk = 0; kk < kBK / 16; ++kk) {
-                        umma_ss(tmem_base + buf * BN, make_smem_desc_sw128(a_addr + kk * 32, 16, 1024),
-                                make_smem_desc_sw128(b_addr + kk * 32, 16, 1024), idesc, (kb | kk) ? 1u : 0u);
-                    }
+                    for (int kk = 0; kk < kBK / 16; ++kk)          // 32 bytes further, in the descriptors' units of 16
+                        umma_ss(tmem + buf * BN, ad + 2 * kk, bd + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
                     umma_commit(&empty[s]);           // the stage is free once these MMAs have read it
                 }
-                if (ok) umma_commit(&acc_full[buf]);
             }
-            // drain: no MMA may be in flight when TMEM is freed (also on the abort path)
-            umma_commit(drain);
-            mbar_wait(drain, 0, ctx, 0x44);
+            if (ok && leader) umma_commit(&acc_full[buf]);
         }
+        // drain: no MMA may be in flight when TMEM is freed (also on the abort path)
+        if (leader) umma_commit(drain);
+        mbar_wait_warp(drain, 0, ctx, 0x44);
     } else {
         const int quarter = warp & 3;                 // TMEM lanes this warp may read
         uint32_t tile_no = 0;
@@ -420,29 +421,33 @@ linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && cta == 0) {
+        if (cta == 0) {
             constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, 2 * kTileA, BN);
+            const bool leader = elect_one();
+            const uint32_t tmem = uniform(tmem_base);
             uint32_t it = 0, tile_no = 0;
             bool ok = true;
             for (int t = blockIdx.x / 2; t < tiles && ok; t += pairs, ++tile_no) {
                 const int buf = tile_no & 1;
-                if (tile_no >= 2) ok = mbar_wait(&acc_empty[buf], ((tile_no >> 1) - 1) & 1, ctx, 0x62);
+                if (tile_no >= 2) ok = mbar_wait_warp(&acc_empty[buf], ((tile_no >> 1) - 1) & 1, ctx, 0x62);
                 if (!ok) break;
                 tc_fence_after();
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % C::kStages;
-                    if (!mbar_wait(&full[s], (it / C::kStages) & 1, ctx, 0x63)) { ok = false; break; }
+                    if (!mbar_wait_warp(&full[s], (it / C::kStages) & 1, ctx, 0x63)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes);
                     const uint64_t ad = make_smem_desc_sw128(a_addr, 16, 1024), bd = make_smem_desc_sw128(a_addr + kABytes, 16, 1024);
+                    if (leader) {
 #pragma unroll
-                    for (int kk = 0; kk < kBK / 16; ++kk)          // 32 bytes further, in the descriptors' units of 16
-                        umma2_ss(tmem_base + buf * BN, ad + 2 * kk, bd + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
-                    umma2_commit(&empty[s]);          // the stage is free in both CTAs once these MMAs have read it
+                        for (int kk = 0; kk < kBK / 16; ++kk)
+                            umma2_ss(tmem + buf * BN, ad + 2 * kk, bd + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                        umma2_commit(&empty[s]);      // the stage is free in both CTAs once these MMAs have read it
+                    }
                 }
-                if (ok) umma2_commit(&acc_full[buf]);
+                if (ok && leader) umma2_commit(&acc_full[buf]);
             }
-            umma2_commit(drain);                          // behind every MMA above (also after a break)
+            if (leader) umma2_commit(drain);              // behind every MMA above (also after a break)
         }
         __syncwarp();
     } else {
@@ -659,21 +664,23 @@ linear_skinny_kernel(const __grid_constant__ LinearMaps maps, LinearParams p, in
         __syncwarp();
         if (splits > 1) cluster_wait();
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, kTileA, MT);
+            const bool leader = elect_one();
+            const uint32_t tmem = uniform(tmem_base);
             for (int i = 0; i < nkb; ++i) {
                 const int s = i % C::kStages;
-                if (!mbar_wait(&full[s], (i / C::kStages) & 1, ctx, 0x52)) break;
+                if (!mbar_wait_warp(&full[s], (i / C::kStages) & 1, ctx, 0x52)) break;
                 tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes), b_addr = a_addr + kABytes;
+                const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes);
+                const uint64_t ad = make_smem_desc_sw128(a_addr, 16, 1024), bd = make_smem_desc_sw128(a_addr + kABytes, 16, 1024);
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < kBK / 16; ++kk) {
-                    umma_ss(tmem_base, make_smem_desc_sw128(a_addr + kk * 32, 16, 1024),
-                            make_smem_desc_sw128(b_addr + kk * 32, 16, 1024), idesc, (i | kk) ? 1u : 0u);
+                    for (int kk = 0; kk < kBK / 16; ++kk) umma_ss(tmem, ad + 2 * kk, bd + 2 * kk, idesc, (i | kk) ? 1u : 0u);
+                    umma_commit(&empty[s]);
                 }
-                umma_commit(&empty[s]);
             }
-            umma_commit(acc_full);       // completes once every MMA above has finished (also after a break)
+            if (leader) umma_commit(acc_full);       // completes once every MMA above has finished (also after a break)
         }
         __syncwarp();
         if (splits > 1) cluster_wait();

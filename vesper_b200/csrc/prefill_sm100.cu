@@ -228,29 +228,35 @@ prefill_sm100_kernel(const __grid_constant__ TmaMaps maps, PrefillParams p) {
             }
         } else if (warp == kMmaWarp) {
             // =========================== MMA issuer ===========================
-            if (lane == 0) {
+            // The whole warp walks the items and one lane issues: descriptors and addresses then live in uniform registers.  Issued by `if (lane == 0)` code a
+            // product cost about 100 cycles of moves into them, more than its 64 on the tensor cores.
+            {
                 constexpr uint32_t idesc_qk = make_idesc_f16(Elem<T>::kFormat, 0, 0, kBlockM, kBlockN);
                 constexpr uint32_t idesc_pv = make_idesc_f16(Elem<T>::kFormat, 0, 1, kBlockM, D);
-                const uint32_t q_addr = smem_u32(q_smem), kv_addr = smem_u32(kv_smem);
-                auto tmem_s = [&](int t) { return tmem_base + static_cast<uint32_t>(t * 128); };
-                auto tmem_o = [&](int t) { return tmem_base + static_cast<uint32_t>(256 + t * 128); };
+                const bool leader = elect_one();
+                const uint64_t q_desc = make_smem_desc_sw128(smem_u32(q_smem), 16, 1024), k_desc = make_smem_desc_sw128(smem_u32(kv_smem), 16, 1024);
+                // V tile is MN-major for its product: 16 keys = 2048 bytes per step, second 64-column box one half-tile further (leading offset)
+                const uint64_t v_desc = make_smem_desc_sw128(smem_u32(kv_smem), C::kHalfBytes, 1024);
+                constexpr uint64_t kTileStep = C::kTileBytes >> 4;
+                // all 512 columns are this CTA's, so they start at 0
+                auto tmem_s = [&](int t) { return static_cast<uint32_t>(t * 128); };
+                auto tmem_o = [&](int t) { return static_cast<uint32_t>(256 + t * 128); };
+                auto commit = [&](uint64_t* b) { if (leader) umma_commit(b); };
                 auto issue_qk = [&](int t, int qbuf, int slot) {
+                    const uint64_t a = q_desc + qbuf * kTileStep, bd = k_desc + slot * kTileStep;
+                    if (leader)
 #pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk) {
-                        uint32_t off = (kk >> 2) * C::kHalfBytes + (kk & 3) * 32;
-                        uint64_t a = make_smem_desc_sw128(q_addr + qbuf * C::kTileBytes + off, 16, 1024);
-                        uint64_t bd = make_smem_desc_sw128(kv_addr + slot * C::kTileBytes + off, 16, 1024);
-                        umma_ss(tmem_s(t), a, bd, idesc_qk, kk > 0 ? 1u : 0u);
-                    }
+                        for (int kk = 0; kk < D / 16; ++kk) {
+                            const uint32_t off = ((kk >> 2) * C::kHalfBytes + (kk & 3) * 32) >> 4;
+                            umma_ss(tmem_s(t), a + off, bd + off, idesc_qk, kk > 0 ? 1u : 0u);
+                        }
                 };
                 auto issue_pv = [&](int t, int slot, bool accumulate) {
+                    const uint64_t bd = v_desc + slot * kTileStep;
+                    if (leader)
 #pragma unroll
-                    for (int kk = 0; kk < kBlockN / 16; ++kk) {
-                        // V tile is MN-major for this product: 16 keys = 2048 bytes per step,
-                        // second 64-column box one half-tile further (leading offset)
-                        uint64_t bd = make_smem_desc_sw128(kv_addr + slot * C::kTileBytes + kk * 2048, C::kHalfBytes, 1024);
-                        umma_ts(tmem_o(t), tmem_s(t) + kk * 8, bd, idesc_pv, (accumulate || kk > 0) ? 1u : 0u);
-                    }
+                        for (int kk = 0; kk < kBlockN / 16; ++kk)
+                            umma_ts(tmem_o(t), tmem_s(t) + kk * 8, bd + kk * (2048 >> 4), idesc_pv, (accumulate || kk > 0) ? 1u : 0u);
                 };
                 int kv_item = 0, q_seq = 0;
                 int blk0 = 0, blk1 = 0;          // running count of score tiles per query tile (barrier phases)
@@ -261,7 +267,7 @@ prefill_sm100_kernel(const __grid_constant__ TmaMaps maps, PrefillParams p) {
                     const Item w = get_item(p, idx, n_bh, n_pairs);
                     int qbuf[2] = {0, 0};
                     const int k0_slot = kv_item % kStages;
-                    ok = mbar_wait(&bar->kv_full[k0_slot], (kv_item / kStages) & 1, abort_flag, 0x200);
+                    ok = mbar_wait_warp(&bar->kv_full[k0_slot], (kv_item / kStages) & 1, abort_flag, 0x200);
 #pragma unroll
                     for (int t = 0; t < 2; ++t) {
                         if (w.nblk[t] == 0 || !ok) continue;
@@ -269,51 +275,51 @@ prefill_sm100_kernel(const __grid_constant__ TmaMaps maps, PrefillParams p) {
                         const int ph = (q_seq / kQBufs) & 1;
                         ++q_seq;
                         // S of this tile is free: every PV of the previous item was issued before this point
-                        ok = mbar_wait(rope ? &bar->q_rot[qbuf[t]] : &bar->q_full[qbuf[t]], ph, abort_flag, 0x210 + t);
+                        ok = mbar_wait_warp(rope ? &bar->q_rot[qbuf[t]] : &bar->q_full[qbuf[t]], ph, abort_flag, 0x210 + t);
                         if (!ok) continue;
                         tc_fence_after();
                         issue_qk(t, qbuf[t], k0_slot);
-                        umma_commit(&bar->s_full[t]);
-                        if (w.nblk[t] == 1) umma_commit(&bar->q_free[qbuf[t]]);
+                        commit(&bar->s_full[t]);
+                        if (w.nblk[t] == 1) commit(&bar->q_free[qbuf[t]]);
                     }
                     if (!ok) break;
-                    umma_commit(&bar->kv_empty[k0_slot]);
+                    commit(&bar->kv_empty[k0_slot]);
                     for (int j = 0; j < w.nmax && ok; ++j) {
                         const int v_item = kv_item + 2 * j + 1, k_item = kv_item + 2 * j + 2;
                         const int v_slot = v_item % kStages, k_slot = k_item % kStages;
-                        ok = mbar_wait(&bar->kv_full[v_slot], (v_item / kStages) & 1, abort_flag, 0x300);
+                        ok = mbar_wait_warp(&bar->kv_full[v_slot], (v_item / kStages) & 1, abort_flag, 0x300);
                         bool k_ready = false;
 #pragma unroll
                         for (int t = 0; t < 2; ++t) {
                             if (j >= w.nblk[t] || !ok) continue;
                             int& blk = t ? blk1 : blk0;
-                            ok = mbar_wait(&bar->p_ready[t], blk & 1, abort_flag, 0x400 + t);
+                            ok = mbar_wait_warp(&bar->p_ready[t], blk & 1, abort_flag, 0x400 + t);
                             if (!ok) continue;
                             ++blk;
                             tc_fence_after();
                             issue_pv(t, v_slot, j > 0);
-                            umma_commit(&bar->o_done[t]);
+                            commit(&bar->o_done[t]);
                             if (j + 1 < w.nblk[t]) {
                                 if (!k_ready) {
-                                    ok = mbar_wait(&bar->kv_full[k_slot], (k_item / kStages) & 1, abort_flag, 0x500);
+                                    ok = mbar_wait_warp(&bar->kv_full[k_slot], (k_item / kStages) & 1, abort_flag, 0x500);
                                     if (!ok) continue;
                                     tc_fence_after();
                                     k_ready = true;
                                 }
                                 issue_qk(t, qbuf[t], k_slot);
-                                umma_commit(&bar->s_full[t]);
-                                if (j + 2 == w.nblk[t]) umma_commit(&bar->q_free[qbuf[t]]);   // last QK of this tile
+                                commit(&bar->s_full[t]);
+                                if (j + 2 == w.nblk[t]) commit(&bar->q_free[qbuf[t]]);   // last QK of this tile
                             }
                         }
                         if (!ok) break;
-                        umma_commit(&bar->kv_empty[v_slot]);
-                        if (j + 1 < w.nmax) umma_commit(&bar->kv_empty[k_slot]);
+                        commit(&bar->kv_empty[v_slot]);
+                        if (j + 1 < w.nmax) commit(&bar->kv_empty[k_slot]);
                     }
                     kv_item += 2 * w.nmax;
                 }
                 // everything issued so far has to retire before TMEM is released
-                umma_commit(&bar->mma_done);
-                mbar_wait(&bar->mma_done, 0, abort_flag, 0x600);
+                commit(&bar->mma_done);
+                mbar_wait_warp(&bar->mma_done, 0, abort_flag, 0x600);
             }
             __syncwarp();
         } else if (rope) {

@@ -143,11 +143,13 @@ sig_prefill_sm100_kernel(const __grid_constant__ SigMaps maps, SigTileParams p) 
             }
         }
     } else if (warp == 9) {
-        if (lane == 0 && cta == 0) {
+        if (cta == 0) {
+            const bool leader = elect_one();             // (the whole warp walks: see the note at umma_ss)
+            const uint32_t tmem = uniform(bar.tmem);
             constexpr int kM = PAIR ? 2 * kRows : kRows;
             const uint32_t idesc_qk = make_idesc_f16(1, 0, 0, kM, kKeys);
             const uint32_t idesc_pv = make_idesc_f16(1, 0, 1, kM, p.n_pv);
-            // what this one thread executes between two products is what holds the tensor pipe up: descriptors are built once (only the
+            // what this warp executes between two products is what holds the tensor pipe up: descriptors are built once (only the
             // start address, in units of 16 bytes, moves), stages and parities are counted, the steps of a box are unrolled.  Columns
             // past kd are zero in both operands, so every box takes its four steps.
             const uint64_t q_desc = make_smem_desc_sw128(smem_u32(q_smem), 16, 1024), k_desc = make_smem_desc_sw128(smem_u32(k_ring), 16, 1024);
@@ -161,47 +163,49 @@ sig_prefill_sm100_kernel(const __grid_constant__ SigMaps maps, SigTileParams p) 
                 uint64_t qd = q_desc;
                 uint32_t acc = 0;
                 for (int i = 0; i < p.nb_k; i += p.kbs) {
-                    if (j == 0) ok = mbar_wait(&bar.q_full[i / p.kbs], 0, ctx, 0xD2);
-                    ok = ok && mbar_wait(&bar.k_full[ks], k_phase, ctx, 0xD3);
+                    if (j == 0) ok = mbar_wait_warp(&bar.q_full[i / p.kbs], 0, ctx, 0xD2);
+                    ok = ok && mbar_wait_warp(&bar.k_full[ks], k_phase, ctx, 0xD3);
                     if (!ok) return;
                     tc_fence_after();
                     uint64_t kd = k_desc + ks * k_stage16;
                     for (int x = 0; x < p.kbs; ++x) {
+                        if (leader)
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            if constexpr (PAIR) umma2_ss(d, qd + 2 * kk, kd + 2 * kk, idesc_qk, kk > 0 ? 1u : acc);
-                            else umma_ss(d, qd + 2 * kk, kd + 2 * kk, idesc_qk, kk > 0 ? 1u : acc);
-                        }
+                            for (int kk = 0; kk < 4; ++kk) {
+                                if constexpr (PAIR) umma2_ss(d, qd + 2 * kk, kd + 2 * kk, idesc_qk, kk > 0 ? 1u : acc);
+                                else umma_ss(d, qd + 2 * kk, kd + 2 * kk, idesc_qk, kk > 0 ? 1u : acc);
+                            }
                         acc = 1;
                         qd += kBox >> 4;
                         kd += kKBox >> 4;
                     }
-                    commit(&bar.k_empty[ks]);
+                    if (leader) commit(&bar.k_empty[ks]);
                     if (++ks == p.k_stages) { ks = 0; k_phase ^= 1; }
                 }
-                commit(&bar.s_full[j & 1]);
+                if (leader) commit(&bar.s_full[j & 1]);
             };
             if (ok) issue_qk(0);
             for (int j = 0; j < n_blk && ok; ++j) {
                 if (j + 1 < n_blk) issue_qk(j + 1);      // its S held the weights of block j-1, whose product was issued before
                 if (!ok) break;
-                ok = mbar_wait(&bar.v_full[vs], v_phase, ctx, 0xD9) && mbar_wait(&bar.p_ready[j & 1], (j >> 1) & 1, ctx, 0xD4);
+                ok = mbar_wait_warp(&bar.v_full[vs], v_phase, ctx, 0xD9) && mbar_wait_warp(&bar.p_ready[j & 1], (j >> 1) & 1, ctx, 0xD4);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t w = tmem + (j & 1) * kKeys, o = tmem + 2 * kKeys, acc = j > 0 ? 1u : 0u;
                 const uint64_t vd = v_desc + vs * v_stage16;
+                if (leader)
 #pragma unroll
-                for (int i = 0; i < 2 * (kKeys / 16); ++i) {             // hi, then lo
-                    const int half = i / (kKeys / 16), kk = i % (kKeys / 16);
-                    const uint32_t at = w + (kk >> 2) * 64 + half * 32 + (kk & 3) * 8;
-                    if constexpr (PAIR) umma2_ts(o, at, vd + kk * (2048 >> 4), idesc_pv, i > 0 ? 1u : acc);
-                    else umma_ts(o, at, vd + kk * (2048 >> 4), idesc_pv, i > 0 ? 1u : acc);
-                }
-                commit(&bar.v_empty[vs]);
+                    for (int i = 0; i < 2 * (kKeys / 16); ++i) {         // hi, then lo
+                        const int half = i / (kKeys / 16), kk = i % (kKeys / 16);
+                        const uint32_t at = w + (kk >> 2) * 64 + half * 32 + (kk & 3) * 8;
+                        if constexpr (PAIR) umma2_ts(o, at, vd + kk * (2048 >> 4), idesc_pv, i > 0 ? 1u : acc);
+                        else umma_ts(o, at, vd + kk * (2048 >> 4), idesc_pv, i > 0 ? 1u : acc);
+                    }
+                if (leader) commit(&bar.v_empty[vs]);
                 if (++vs == p.v_stages) { vs = 0; v_phase ^= 1; }
             }
-            if (ok) commit(&bar.o_done);
-            commit(&bar.drain);                          // nothing may be in flight when TMEM is freed
+            if (ok && leader) commit(&bar.o_done);
+            if (leader) commit(&bar.drain);                          // nothing may be in flight when TMEM is freed
         }
         if (lane == 0) mbar_wait(&bar.drain, 0, ctx, 0xD5);
         __syncwarp();

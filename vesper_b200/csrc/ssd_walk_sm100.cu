@@ -70,7 +70,8 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = bar.tmem, t_y = tmem + 128, t_s = tmem + 192, t_m = tmem + 256;
+    constexpr uint32_t tmem = 0;                      // all 512 columns are this CTA's
+    constexpr uint32_t t_y = tmem + 128, t_s = tmem + 192, t_m = tmem + 256;
     const bool dead = *static_cast<volatile int*>(&bar.abort_flag) != 0;
     __syncthreads();
     pdl_begin();
@@ -90,43 +91,51 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
             }
         }
     } else if (warp == 9) {
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();         // (the whole warp walks: see the note at umma_ss)
+            auto commit = [&](uint64_t* to) { if (leader) umma_commit(to); };
             constexpr uint32_t id_g = make_idesc_f16(1, 0, 0, 128, 128), id_cs = make_idesc_f16(1, 0, 1, 128, 64), id_u = make_idesc_f16(1, 1, 1, 128, 64);
-            const uint32_t xw_a = smem_u32(xw), ss_a = smem_u32(ss);
+            const uint64_t xw_mn = make_smem_desc_sw128(smem_u32(xw), kBox, 1024), s_mn = make_smem_desc_sw128(smem_u32(ss), kBox, 1024);
             for (int k = 0; k < n_chunk; ++k) {
                 const int q = k & 1, ph = k & 1;
-                if (!mbar_wait(&bar.tiles_full[q], (k / 2) & 1, ctx, 0xD2)) break;
+                if (!mbar_wait_warp(&bar.tiles_full[q], (k / 2) & 1, ctx, 0xD2)) break;
                 tc_fence_after();
+                // operands K-major (16 columns = 32 bytes) and MN-major (16 rows = 2048 bytes)
                 const uint32_t c_a = smem_u32(smem + q * kStage), b_a = c_a + 2 * kBox, x_a = c_a + 4 * kBox;
-                for (int kk = 0; kk < p.nk; ++kk) {
-                    const uint32_t off = (kk >> 2) * kBox + (kk & 3) * 32;
-                    umma_ss(tmem, make_smem_desc_sw128(c_a + off, 16, 1024), make_smem_desc_sw128(b_a + off, 16, 1024), id_g, kk > 0 ? 1u : 0u);
-                }
-                umma_commit(&bar.g_full);
-                if (!mbar_wait(&bar.s_ready, ph, ctx, 0xD3)) break;
-                if (k > 0 && !mbar_wait(&bar.y_free, (k - 1) & 1, ctx, 0xD4)) break;
+                const uint64_t c_k = make_smem_desc_sw128(c_a, 16, 1024), b_k = make_smem_desc_sw128(b_a, 16, 1024), b_mn = make_smem_desc_sw128(b_a, kBox, 1024),
+                               x_mn = make_smem_desc_sw128(x_a, kBox, 1024);
+                auto by_k = [](int kk) { return ((kk >> 2) * kBox + (kk & 3) * 32) >> 4; };
+                if (leader)
+#pragma unroll
+                    for (int kk = 0; kk < 8; ++kk)
+                        if (kk < p.nk) umma_ss(tmem, c_k + by_k(kk), b_k + by_k(kk), id_g, kk > 0 ? 1u : 0u);
+                commit(&bar.g_full);
+                if (!mbar_wait_warp(&bar.s_ready, ph, ctx, 0xD3)) break;
+                if (k > 0 && !mbar_wait_warp(&bar.y_free, (k - 1) & 1, ctx, 0xD4)) break;
                 tc_fence_after();
-                for (int half = 0; half < 2; ++half)
-                    for (int kk = 0; kk < p.nk; ++kk)
-                        umma_ss(t_y, make_smem_desc_sw128(c_a + (kk >> 2) * kBox + (kk & 3) * 32, 16, 1024), make_smem_desc_sw128(ss_a + half * kBox + kk * 2048, kBox, 1024), id_cs,
-                                (half | kk) ? 1u : 0u);
-                umma_commit(&bar.cs_full);
-                if (!mbar_wait(&bar.xw_ready, ph, ctx, 0xD5)) break;
+                if (leader)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {               // hi, then lo
+                        const int half = i >> 3, kk = i & 7;
+                        if (kk < p.nk) umma_ss(t_y, c_k + by_k(kk), s_mn + ((half * kBox + kk * 2048) >> 4), id_cs, i > 0 ? 1u : 0u);
+                    }
+                commit(&bar.cs_full);
+                if (!mbar_wait_warp(&bar.xw_ready, ph, ctx, 0xD5)) break;
                 tc_fence_after();
-                for (int half = 0; half < 2; ++half)
-                    for (int kk = 0; kk < kL / 16; ++kk)
-                        umma_ss(t_s, make_smem_desc_sw128(b_a + kk * 2048, kBox, 1024), make_smem_desc_sw128(xw_a + half * kBox + kk * 2048, kBox, 1024), id_u, 1u);
-                umma_commit(&bar.u_full);
-                if (!mbar_wait(&bar.p_ready, ph, ctx, 0xD6)) break;
+                if (leader)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) umma_ss(t_s, b_mn + (i & 7) * (2048 >> 4), xw_mn + (((i >> 3) * kBox + (i & 7) * 2048) >> 4), id_u, 1u);
+                commit(&bar.u_full);
+                if (!mbar_wait_warp(&bar.p_ready, ph, ctx, 0xD6)) break;
                 tc_fence_after();
-                for (int half = 0; half < 2; ++half)
-                    for (int kk = 0; kk < kL / 16; ++kk)
-                        umma_ts(t_y, t_m + half * 64 + kk * 8, make_smem_desc_sw128(x_a + kk * 2048, kBox, 1024), id_cs, 1u);
-                umma_commit(&bar.y_full);
-                umma_commit(&bar.tiles_empty[q]);
+                if (leader)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) umma_ts(t_y, t_m + (i >> 3) * 64 + (i & 7) * 8, x_mn + (i & 7) * (2048 >> 4), id_cs, 1u);
+                commit(&bar.y_full);
+                commit(&bar.tiles_empty[q]);
             }
-            umma_commit(&bar.drain);                 // nothing may be in flight when TMEM is freed
-            mbar_wait(&bar.drain, 0, ctx, 0xD7);
+            commit(&bar.drain);                 // nothing may be in flight when TMEM is freed
+            mbar_wait_warp(&bar.drain, 0, ctx, 0xD7);
         }
     } else {
         const int r = threadIdx.x & 127, half = threadIdx.x >> 7;           // TMEM lane, column half
@@ -335,7 +344,7 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
         tc_fence_before();
     }
     __syncthreads();
-    if (warp == 9) tmem_dealloc(tmem, 512);
+    if (warp == 9) tmem_dealloc(bar.tmem, 512);
     abort_linger(&bar.abort_flag);
 }
 
