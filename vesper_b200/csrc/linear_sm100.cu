@@ -342,6 +342,7 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
 // ------------------------------------------------------------------------------------------------
 constexpr int kPairEpilogue = 8;                    // epilogue warps: each 32 rows x half of a tile's columns
 constexpr int kPairThreads = 64 + 32 * kPairEpilogue;
+struct PairMaps { CUtensorMap a, b, b_half; };      // x; W in boxes of half a tile's columns, and of a quarter's
 template <int BN>
 struct PairCfg {
     static constexpr int kBBytes = BN / 2 * kBK * 2;
@@ -363,9 +364,18 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
         : "memory");
 }
 
+// What a pair computes at a time: a tile, or (from tile `whole` on) half of its columns.
+struct PairUnit { int row_tile, col0; bool half; };
+template <int BN>
+__device__ __forceinline__ PairUnit pair_unit(int u, int whole, int m_tiles) {
+    const bool half = u >= whole;
+    const int t = half ? whole + (u - whole) / 2 : u;
+    return PairUnit{t % m_tiles, t / m_tiles * BN + (half ? ((u - whole) & 1) * (BN / 2) : 0), half};      // consecutive pairs share a W tile through L2
+}
+
 template <int BN, int EPI>
 __global__ void __launch_bounds__(kPairThreads, 1)
-linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
+linear_pair_kernel(const __grid_constant__ PairMaps maps, LinearParams p, int whole) {
     using C = PairCfg<BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -379,7 +389,7 @@ linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cta = static_cast<int>(cluster_ctarank()), pairs = gridDim.x / 2;
-    const int m_tiles = (p.M + 2 * kTileA - 1) / (2 * kTileA), n_tiles = (p.N + BN - 1) / BN, tiles = m_tiles * n_tiles;
+    const int m_tiles = (p.M + 2 * kTileA - 1) / (2 * kTileA), units = 2 * (m_tiles * ((p.N + BN - 1) / BN)) - whole;
     const int k_blocks = (p.K + kBK - 1) / kBK;
     const WaitCtx ctx{abort_flag, p.status};
 
@@ -407,27 +417,29 @@ linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
     if (warp == 0) {
         if (lane == 0) {
             uint32_t it = 0;
-            for (int t = blockIdx.x / 2; t < tiles && !*abort_flag; t += pairs) {
-                const int row0 = (t % m_tiles * 2 + cta) * kTileA, w0 = t / m_tiles * BN + cta * (BN / 2);      // consecutive pairs share a W tile through L2
+            for (int u = blockIdx.x / 2; u < units && !*abort_flag; u += pairs) {
+                const PairUnit w = pair_unit<BN>(u, whole, m_tiles);
+                const int row0 = (w.row_tile * 2 + cta) * kTileA, cols = w.half ? BN / 4 : BN / 2, w0 = w.col0 + cta * cols;
+                const CUtensorMap* mb = w.half ? &maps.b_half : &maps.b;
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % C::kStages;
                     if (it >= C::kStages && !mbar_wait(&empty[s], ((it / C::kStages) - 1) & 1, ctx, 0x61)) break;
                     uint8_t* st = smem + s * C::kStageBytes;
-                    if (cta == 0) mbar_arrive_expect_tx(&full[s], 2 * C::kStageBytes);
+                    if (cta == 0) mbar_arrive_expect_tx(&full[s], 2 * (kABytes + cols * kBK * 2));
                     const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
                     tma_load_2d_pair(st, &maps.a, bar, kb * kBK, row0);
-                    tma_load_2d_pair(st + kABytes, &maps.b, bar, kb * kBK, w0);
+                    tma_load_2d_pair(st + kABytes, mb, bar, kb * kBK, w0);
                 }
             }
         }
     } else if (warp == 1) {
         if (cta == 0) {
-            constexpr uint32_t idesc = make_idesc_f16(1, 0, 0, 2 * kTileA, BN);
             const bool leader = elect_one();
             const uint32_t tmem = uniform(tmem_base);
             uint32_t it = 0, tile_no = 0;
             bool ok = true;
-            for (int t = blockIdx.x / 2; t < tiles && ok; t += pairs, ++tile_no) {
+            for (int u = blockIdx.x / 2; u < units && ok; u += pairs, ++tile_no) {
+                const uint32_t idesc = u < whole ? make_idesc_f16(1, 0, 0, 2 * kTileA, BN) : make_idesc_f16(1, 0, 0, 2 * kTileA, BN / 2);
                 const int buf = tile_no & 1;
                 if (tile_no >= 2) ok = mbar_wait_warp(&acc_empty[buf], ((tile_no >> 1) - 1) & 1, ctx, 0x62);
                 if (!ok) break;
@@ -452,26 +464,27 @@ linear_pair_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
         __syncwarp();
     } else {
         const int quarter = warp & 3;                 // TMEM lanes this warp may read
-        constexpr int kCols = BN / (kPairEpilogue / 4), kChunks = kCols / 32;
-        const int col_first = (warp - 2) / 4 * kCols;
         uint32_t tile_no = 0;
-        for (int t = blockIdx.x / 2; t < tiles; t += pairs, ++tile_no) {
+        for (int u = blockIdx.x / 2; u < units; u += pairs, ++tile_no) {
             const int buf = tile_no & 1;
-            const int row = (t % m_tiles * 2 + cta) * kTileA + quarter * 32 + lane, col_tile = t / m_tiles * BN + col_first;
+            const PairUnit w = pair_unit<BN>(u, whole, m_tiles);
+            const int chunks = BN / (kPairEpilogue / 4) / 32 / (w.half ? 2 : 1), col_first = (warp - 2) / 4 * chunks * 32;
+            const int row = (w.row_tile * 2 + cta) * kTileA + quarter * 32 + lane, col_tile = w.col0 + col_first;
             uint32_t was[2][32];                      // residual values: two chunks on their way before they are needed
             auto ahead = [&](int c) {
-                if (EPI == VB200_EPI_ADD_F32 && c < kChunks && row < p.M && col_tile + c * 32 < p.N) load_row32(p, row, col_tile + c * 32, was[c & 1]);
+                if (EPI == VB200_EPI_ADD_F32 && c < chunks && row < p.M && col_tile + c * 32 < p.N) load_row32(p, row, col_tile + c * 32, was[c & 1]);
             };
             ahead(0);
             ahead(1);
             if (!mbar_wait_warp(&acc_full[buf], (tile_no >> 1) & 1, ctx, 0x65)) break;
             tc_fence_after();
 #pragma unroll
-            for (int c = 0; c < kChunks; ++c) {
+            for (int c = 0; c < BN / (kPairEpilogue / 4) / 32; ++c) {
+                if (c == chunks) break;
                 uint32_t acc[32];
                 tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN + col_first + c * 32, acc);
                 tmem_ld_wait();
-                if (c + 1 == kChunks) {               // the accumulator is in registers: the next product may have its columns
+                if (c + 1 == chunks) {                // the accumulator is in registers: the next product may have its columns
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
@@ -873,15 +886,19 @@ int launch_wide(cudaStream_t s, const LinearParams& p) {
 template <int BN, int EPI>
 int launch_pair(cudaStream_t s, const LinearParams& p, int sms) {
     using C = PairCfg<BN>;
-    LinearMaps maps;
+    PairMaps maps;
     if (int rc = make_map_2d(&maps.a, p.x, p.M, p.K, p.ldx, kTileA)) return rc;
     if (int rc = make_map_2d(&maps.b, p.w, p.N, p.K, p.ldw, BN / 2)) return rc;
+    if (int rc = make_map_2d(&maps.b_half, p.w, p.N, p.K, p.ldw, BN / 4)) return rc;
     auto kernel = linear_pair_kernel<BN, EPI>;
     static thread_local bool configured[64] = {};
     if (int rc = set_smem_once(kernel, C::kSmemBytes, configured)) return rc;
-    const int tiles = ((p.M + 2 * kTileA - 1) / (2 * kTileA)) * ((p.N + BN - 1) / BN);
+    const int tiles = ((p.M + 2 * kTileA - 1) / (2 * kTileA)) * ((p.N + BN - 1) / BN), pairs = sms / 2, last = tiles % pairs;
+    // A last round that at most half of the pairs have a tile in is dealt out in halves of tiles (3003 rows, 96 tiles on 74 pairs: 2048 x 8448 94.6 -> 86.3 us,
+    // 2048 x 5632 66.3 -> 58.2, 2048 x 2048 35.1 -> 29.2; a half takes two thirds of a tile's time).
+    const int whole = BN == 256 && tiles > pairs && 2 * last <= pairs ? tiles - last : tiles;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * (tiles < sms / 2 ? tiles : sms / 2)));
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * (tiles < pairs ? tiles : pairs)));
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = C::kSmemBytes;
     cfg.stream = s;
@@ -894,13 +911,13 @@ int launch_pair(cudaStream_t s, const LinearParams& p, int sms) {
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    VB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, p));
+    VB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, p, whole));
     note_launch();
     return VB200_OK;
 }
 
 // More than 64 rows.  Pairs of CTAs with tiles of 256 columns; of 128 columns while one round over the SM pairs takes them all (768 rows, 2048 x 2048:
-// 16.4 us against 21.3, 2048 x 5632 33.0 against 37.5; with more rounds the wider tile is up to 1.6 times faster); single CTAs where the rows
+// 13.6 us, 2048 x 5632 25.3; 256 columns 21.3 and 37.5; with more rounds the wider tile is up to 1.6 times faster); single CTAs where the rows
 // of a pair's last tile would be mostly padding and cost rounds (300 rows, 11264 x 2048: 25.1 us against 29.2).
 template <int EPI>
 int launch_many_rows(cudaStream_t s, const LinearParams& p) {
