@@ -9,7 +9,7 @@
 // S stays in TMEM (fp32) over the whole walk; before a chunk's update it is scaled by the chunk's decay and published to
 // shared memory as the next C S operand.  The decays touch fp32 values only; every product operand they enter is split.
 //   warps 0-7  compute: row = TMEM lane, the two warpgroups share a row's columns
-//   warp  8    TMA: C, B and x of the next chunk into the second buffers (128-byte swizzle)
+//   warp  8    TMA: C, B and x of the next chunk into the second buffers (128-byte swizzle); step sizes and running decays
 //   warp  9    tcgen05.mma issuer, TMEM owner
 // TMEM (512 columns): G [0,128) Y [128,192) S [192,256) M [256,384): hi in its first 64 columns, lo in the others.
 // All hand-overs are mbarriers with bounded waits; there is no CTA barrier inside the walk.
@@ -40,7 +40,7 @@ struct WalkParams {
 
 struct WalkBars {
     float la[2][kL], dt[2][kL];           // running log2-decays and step sizes of a chunk
-    uint64_t tiles_full[2], tiles_empty[2], dt_ready, g_full, cs_full, xw_ready, p_ready, s_ready, u_full, y_full, y_free, drain;
+    uint64_t tiles_full[2], tiles_empty[2], dt_ready[2], g_full, cs_full, xw_ready, p_ready, s_ready, u_full, y_full, y_free, drain;
     uint32_t tmem;
     int abort_flag;
 };
@@ -58,10 +58,10 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
 
     if (threadIdx.x == 0) {
         bar.abort_flag = 0;
-        for (int i = 0; i < 2; ++i) { mbar_init(&bar.tiles_full[i], 1); mbar_init(&bar.tiles_empty[i], 1 + 256); }
-        mbar_init(&bar.dt_ready, 32);
+        for (int i = 0; i < 2; ++i) { mbar_init(&bar.tiles_full[i], 1); mbar_init(&bar.tiles_empty[i], 1 + 8); }
+        for (int i = 0; i < 2; ++i) mbar_init(&bar.dt_ready[i], 32);
         mbar_init(&bar.g_full, 1); mbar_init(&bar.cs_full, 1); mbar_init(&bar.u_full, 1); mbar_init(&bar.y_full, 1);
-        mbar_init(&bar.xw_ready, 256); mbar_init(&bar.p_ready, 256); mbar_init(&bar.s_ready, 256); mbar_init(&bar.y_free, 256);
+        mbar_init(&bar.xw_ready, 8); mbar_init(&bar.p_ready, 8); mbar_init(&bar.s_ready, 8); mbar_init(&bar.y_free, 8);
         mbar_init(&bar.drain, 1);
         mbar_fence_init();
         if ((smem_u32(smem) & 1023) != 0) { bar.abort_flag = 1; atomicCAS(p.status, 0, (3 << 24) | 0x3); }      // the swizzle needs 1024-byte tiles
@@ -78,17 +78,52 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
 
     if (dead) {
     } else if (warp == 8) {
-        if (lane == 0) {
-            const int grp = h / (p.H / p.G);
-            for (int k = 0; k < n_chunk; ++k) {
-                const int q = k & 1, t0 = (c_begin + k) * kL;
-                if (k >= 2 && !mbar_wait(&bar.tiles_empty[q], (k / 2 - 1) & 1, ctx, 0xD1)) break;
+        // ---- copies, and the step sizes and running log-decays of a chunk, four tokens per lane ----
+        const int grp = h / (p.H / p.G), inner = p.H * p.P;
+        const float nA2 = -expf(p.A_log[h]) * kLog2e, dtb = p.dt_bias[h];
+        const __nv_bfloat16* steps = p.proj + static_cast<long long>(b) * p.T * p.ldp + 2 * inner + 2 * p.G * p.N + h;
+        float raw[4] = {0.f, 0.f, 0.f, 0.f};
+        auto fetch_dt = [&](int k) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int t = (c_begin + k) * kL + lane * 4 + e;
+                raw[e] = k < n_chunk && t < p.T ? __bfloat162float(steps[static_cast<long long>(t) * p.ldp]) : 0.f;
+            }
+        };
+        fetch_dt(0);
+        for (int k = 0; k < n_chunk; ++k) {
+            const int q = k & 1, t0 = (c_begin + k) * kL;
+            if (k >= 2 && !mbar_wait_warp(&bar.tiles_empty[q], (k / 2 - 1) & 1, ctx, 0xD1)) break;
+            if (lane == 0) {
                 uint8_t* st = smem + q * kStage;
                 mbar_arrive_expect_tx(&bar.tiles_full[q], kStage);
                 for (int i = 0; i < 2; ++i) tma_load_4d(st + i * kBox, &maps.c, &bar.tiles_full[q], i * 64, grp, t0, b);
                 for (int i = 0; i < 2; ++i) tma_load_4d(st + (2 + i) * kBox, &maps.b, &bar.tiles_full[q], i * 64, grp, t0, b);
                 tma_load_4d(st + 4 * kBox, &maps.x, &bar.tiles_full[q], 0, h, t0, b);
             }
+            float d[4], a[4], s = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                d[e] = t0 + lane * 4 + e < p.T ? softplus_f(raw[e] + dtb) : 0.f;
+                s += nA2 * d[e];
+                a[e] = s;
+            }
+            fetch_dt(k + 1);
+            float inc = s;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            const float before = inc - s;
+            // every warp has the output of chunk k - 2 behind it, and with that its last look at this set
+            if (k >= 2 && !mbar_wait_warp(&bar.y_free, k & 1, ctx, 0xDF)) break;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                bar.la[q][lane * 4 + e] = before + a[e];
+                bar.dt[q][lane * 4 + e] = d[e];
+            }
+            mbar_arrive(&bar.dt_ready[q]);
         }
     } else if (warp == 9) {
         {
@@ -96,20 +131,25 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
             auto commit = [&](uint64_t* to) { if (leader) umma_commit(to); };
             constexpr uint32_t id_g = make_idesc_f16(1, 0, 0, 128, 128), id_cs = make_idesc_f16(1, 0, 1, 128, 64), id_u = make_idesc_f16(1, 1, 1, 128, 64);
             const uint64_t xw_mn = make_smem_desc_sw128(smem_u32(xw), kBox, 1024), s_mn = make_smem_desc_sw128(smem_u32(ss), kBox, 1024);
-            for (int k = 0; k < n_chunk; ++k) {
-                const int q = k & 1, ph = k & 1;
-                if (!mbar_wait_warp(&bar.tiles_full[q], (k / 2) & 1, ctx, 0xD2)) break;
+            // operands K-major (16 columns = 32 bytes) and MN-major (16 rows = 2048 bytes)
+            auto by_k = [](int kk) { return ((kk >> 2) * kBox + (kk & 3) * 32) >> 4; };
+            auto issue_g = [&](int k) {
+                if (!mbar_wait_warp(&bar.tiles_full[k & 1], (k / 2) & 1, ctx, 0xD2)) return false;
                 tc_fence_after();
-                // operands K-major (16 columns = 32 bytes) and MN-major (16 rows = 2048 bytes)
-                const uint32_t c_a = smem_u32(smem + q * kStage), b_a = c_a + 2 * kBox, x_a = c_a + 4 * kBox;
-                const uint64_t c_k = make_smem_desc_sw128(c_a, 16, 1024), b_k = make_smem_desc_sw128(b_a, 16, 1024), b_mn = make_smem_desc_sw128(b_a, kBox, 1024),
-                               x_mn = make_smem_desc_sw128(x_a, kBox, 1024);
-                auto by_k = [](int kk) { return ((kk >> 2) * kBox + (kk & 3) * 32) >> 4; };
+                const uint32_t c_a = smem_u32(smem + (k & 1) * kStage);
+                const uint64_t c_k = make_smem_desc_sw128(c_a, 16, 1024), b_k = make_smem_desc_sw128(c_a + 2 * kBox, 16, 1024);
                 if (leader)
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)
                         if (kk < p.nk) umma_ss(tmem, c_k + by_k(kk), b_k + by_k(kk), id_g, kk > 0 ? 1u : 0u);
                 commit(&bar.g_full);
+                return true;
+            };
+            bool ok = issue_g(0);
+            for (int k = 0; k < n_chunk && ok; ++k) {
+                const int q = k & 1, ph = k & 1;
+                const uint32_t c_a = smem_u32(smem + q * kStage);
+                const uint64_t c_k = make_smem_desc_sw128(c_a, 16, 1024), b_mn = make_smem_desc_sw128(c_a + 2 * kBox, kBox, 1024), x_mn = make_smem_desc_sw128(c_a + 4 * kBox, kBox, 1024);
                 if (!mbar_wait_warp(&bar.s_ready, ph, ctx, 0xD3)) break;
                 if (k > 0 && !mbar_wait_warp(&bar.y_free, (k - 1) & 1, ctx, 0xD4)) break;
                 tc_fence_after();
@@ -133,6 +173,7 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
                     for (int i = 0; i < 16; ++i) umma_ts(t_y, t_m + (i >> 3) * 64 + (i & 7) * 8, x_mn + (i & 7) * (2048 >> 4), id_cs, 1u);
                 commit(&bar.y_full);
                 commit(&bar.tiles_empty[q]);
+                if (k + 1 < n_chunk) ok = issue_g(k + 1);        // (M of this chunk has been made of its G)
             }
             commit(&bar.drain);                 // nothing may be in flight when TMEM is freed
             mbar_wait_warp(&bar.drain, 0, ctx, 0xD7);
@@ -141,39 +182,12 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
         const int r = threadIdx.x & 127, half = threadIdx.x >> 7;           // TMEM lane, column half
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const int inner = p.H * p.P, slot = p.slots ? p.slots[b] : b, col0 = half * 32;
-        const float nA2 = -expf(p.A_log[h]) * kLog2e, dtb = p.dt_bias[h], Dh = p.D[h];
-        const __nv_bfloat16* proj = p.proj + static_cast<long long>(b) * p.T * p.ldp;
+        const float Dh = p.D[h];
         const long long state_row = ((static_cast<long long>(slot) * p.H + h) * p.N + r) * p.Pp;
-        // step sizes and running log-decays of a chunk: warp 0, four tokens per lane
-        float raw[4] = {0.f, 0.f, 0.f, 0.f};
-        auto fetch_dt = [&](int k) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int t = (c_begin + k) * kL + lane * 4 + e;
-                raw[e] = t < p.T ? __bfloat162float(proj[static_cast<long long>(t) * p.ldp + 2 * inner + 2 * p.G * p.N + h]) : 0.f;
-            }
-        };
-        auto scan_dt = [&](int k) {
-            float d[4], a[4], s = 0.f;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                d[e] = (c_begin + k) * kL + lane * 4 + e < p.T ? softplus_f(raw[e] + dtb) : 0.f;
-                s += nA2 * d[e];
-                a[e] = s;
-            }
-            float inc = s;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const float v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-                if (lane >= o) inc += v;
-            }
-            const float before = inc - s;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                bar.la[k & 1][lane * 4 + e] = before + a[e];
-                bar.dt[k & 1][lane * 4 + e] = d[e];
-            }
-            mbar_arrive(&bar.dt_ready);
+        // the warp's arrival, after what its lanes have done
+        auto arrive = [&](uint64_t* to) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(to);
         };
         // the state row of this thread (32 columns) as operand of the next C S, and scaled by the next chunk's decay in TMEM
         auto publish = [&](uint32_t (&s)[32], float decay) {
@@ -194,10 +208,9 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
             tmem_st_wait();
             tc_fence_before();
             fence_proxy_async_smem();
-            mbar_arrive(&bar.s_ready);
+            arrive(&bar.s_ready);
         };
-        if (warp == 0) { fetch_dt(0); scan_dt(0); }
-        bool ok = mbar_wait_warp(&bar.dt_ready, 0, ctx, 0xDD);
+        bool ok = mbar_wait_warp(&bar.dt_ready[0], 0, ctx, 0xDD);
         if (ok) {
             uint32_t s[32];
             const float* src = p.n_seg > 1 ? p.seg_state + ((static_cast<long long>(b) * p.n_seg + seg) * p.H + h) * p.N * p.Pp + static_cast<long long>(r) * p.Pp
@@ -211,22 +224,20 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
             }
             publish(s, fast_exp2(bar.la[0][kL - 1]));
         }
-        for (int k = 0; k < n_chunk && ok; ++k) {
-            const int q = k & 1, ph = k & 1, t0 = (c_begin + k) * kL, tn = min(kL, p.T - t0);
-            const long long m = static_cast<long long>(b) * p.T + t0 + r;
+        // Every product has steps that do not need it between its issue and the wait for it.  What bounds the walk now is the instructions of the two warps of a
+        // scheduler, M's and the splits above all, and 192 CTAs in two rounds over 148 SMs.  (3 x 64 heads, 1001 tokens: 101 us with a chunk's steps in their own
+        // order, each waiting for its product; 87 in this one; 85 with the step sizes off these warps' path and one arrival per warp.)
+        //   2^la C S of chunk k | state behind it | output of k | w x of k + 1 | M of k + 1
+        uint4 xv[4];                                 // x of the chunk whose output comes next
+        float lar = 0.f;
+        auto make_xw = [&](int k) {
+            const int q = k & 1;
             const float *la = bar.la[q], *dt = bar.dt[q];
-            const bool more = k + 1 < n_chunk;
-            uint4 z[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                z[c] = r < tn && col0 + c * 8 < p.P ? *reinterpret_cast<const uint4*>(p.proj + m * p.ldp + h * p.P + col0 + c * 8) : make_uint4(0, 0, 0, 0);
-            if (warp == 0 && more) fetch_dt(k + 1);
-            ok = mbar_wait_warp(&bar.tiles_full[q], (k / 2) & 1, ctx, 0xD8);
-            if (!ok) break;
-            // ---- w x: token r, this half's columns.  (The last update has read the previous one: its completion was awaited.) ----
+            if (!mbar_wait_warp(&bar.tiles_full[q], (k / 2) & 1, ctx, 0xD8)) return false;
+            // token r, this half's columns.  (The last update has read the previous one: its completion was awaited.)
             const uint8_t* xt = smem + q * kStage + 4 * kBox;
-            uint4 xv[4];
-            const float lar = la[r], wr = dt[r] * fast_exp2(la[kL - 1] - lar);
+            lar = la[r];
+            const float wr = dt[r] * fast_exp2(la[kL - 1] - lar);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int at = r * 128 + (((half * 4 + c) ^ (r & 7)) << 4);
@@ -244,11 +255,13 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
                 *reinterpret_cast<uint4*>(xw + kBox + at) = lo;
             }
             fence_proxy_async_smem();
-            mbar_arrive(&bar.xw_ready);
-            mbar_arrive(&bar.tiles_empty[q]);        // this thread reads the tiles no more (the products' part is the commit)
-            // ---- M: row r of G, 64 columns ----
-            ok = mbar_wait_warp(&bar.g_full, ph, ctx, 0xD9);
-            if (!ok) break;
+            arrive(&bar.xw_ready);
+            if (lane == 0) mbar_arrive(&bar.tiles_empty[q]);         // this warp reads the tiles no more (the products' part is the commit)
+            return true;
+        };
+        auto make_m = [&](int k) {                   // row r of G, 64 columns
+            const float *la = bar.la[k & 1], *dt = bar.dt[k & 1];
+            if (!mbar_wait_warp(&bar.g_full, k & 1, ctx, 0xD9)) return false;
             tc_fence_after();
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {
@@ -275,6 +288,17 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
                 tmem_st16(t_m + lane_base + j0 / 2, hi);
                 tmem_st16(t_m + lane_base + 64 + j0 / 2, lo);
             }
+            return true;
+        };
+        ok = ok && make_xw(0) && make_m(0);
+        for (int k = 0; k < n_chunk && ok; ++k) {
+            const int q = k & 1, ph = k & 1, t0 = (c_begin + k) * kL, tn = min(kL, p.T - t0);
+            const long long m = static_cast<long long>(b) * p.T + t0 + r;
+            const bool more = k + 1 < n_chunk;
+            uint4 z[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                z[c] = r < tn && col0 + c * 8 < p.P ? *reinterpret_cast<const uint4*>(p.proj + m * p.ldp + h * p.P + col0 + c * 8) : make_uint4(0, 0, 0, 0);
             // ---- 2^la C S ----
             ok = mbar_wait_warp(&bar.cs_full, ph, ctx, 0xDA);
             if (!ok) break;
@@ -288,14 +312,12 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
                 for (int i = 0; i < 32; ++i) y[i] = __float_as_uint(__uint_as_float(y[i]) * e);
                 tmem_st32(t_y + lane_base + col0, y);
             }
-            tmem_st_wait();
+            tmem_st_wait();                          // (M, from the chunk before, too)
             tc_fence_before();
-            mbar_arrive(&bar.p_ready);
-            // ---- the state after this chunk.  (C S of this chunk is complete, so every thread has left the chunk before:
-            // the other set of step sizes is free.) ----
+            arrive(&bar.p_ready);
+            // ---- the state after this chunk ----
             if (more) {
-                if (warp == 0) scan_dt(k + 1);
-                ok = mbar_wait_warp(&bar.dt_ready, (k + 1) & 1, ctx, 0xDE);
+                ok = mbar_wait_warp(&bar.dt_ready[q ^ 1], ((k + 1) / 2) & 1, ctx, 0xDE);
                 if (!ok) break;
             }
             ok = mbar_wait_warp(&bar.u_full, ph, ctx, 0xDB);
@@ -316,7 +338,7 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
                     }
                 }
             }
-            // ---- outputs ----
+            // ---- output ----
             ok = mbar_wait_warp(&bar.y_full, ph, ctx, 0xDC);
             if (!ok) break;
             tc_fence_after();
@@ -324,7 +346,7 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
             tmem_ld32(t_y + lane_base + col0, y);
             tmem_ld_wait();
             tc_fence_before();
-            mbar_arrive(&bar.y_free);
+            arrive(&bar.y_free);
             if (r < tn) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -340,6 +362,8 @@ ssd_walk_sm100_kernel(const __grid_constant__ WalkMaps maps, WalkParams p) {
                     store8(p.gated + m * inner + h * p.P + col0 + c * 8, v);
                 }
             }
+            // ---- the next chunk's part that needs no state: its products run while it is made ----
+            if (more) ok = make_xw(k + 1) && make_m(k + 1);
         }
         tc_fence_before();
     }
