@@ -42,8 +42,21 @@ __device__ __forceinline__ void store2(float* p, const float (&v)[2]) { *reinter
 template <typename T, int VEC, int TAPS>
 __global__ void __launch_bounds__(128)
 ssd_conv_kernel(ConvTask p, const T* __restrict__ proj, T* __restrict__ state, T* __restrict__ out) {
-    pdl_begin();
     const int c0 = (blockIdx.x * 128 + threadIdx.x) * VEC;
+    // the weights do not depend on the launch before
+    constexpr int kTaps = TAPS > 0 ? TAPS : 1;
+    float bias[VEC], w[kTaps][VEC];
+    if (c0 < p.channels) {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            bias[j] = __ldg(p.conv_b + c0 + j);
+            if constexpr (TAPS > 0) {
+#pragma unroll
+                for (int k = 0; k < TAPS; ++k) w[k][j] = __ldg(p.conv_w + static_cast<long long>(c0 + j) * TAPS + k);
+            }
+        }
+    }
+    pdl_begin();
     if (c0 >= p.channels) return;
     const int b = blockIdx.z, t0 = blockIdx.y * kConvTile, t1 = min(p.T, t0 + kConvTile);
     const int taps = TAPS > 0 ? TAPS : p.taps;
@@ -74,15 +87,8 @@ ssd_conv_kernel(ConvTask p, const T* __restrict__ proj, T* __restrict__ state, T
             for (int j = 0; j < VEC; ++j) dst[j] = Elem<T>::from_f(a[j]);
         }
     };
-    float bias[VEC];
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) bias[j] = p.conv_b[c0 + j];
     if constexpr (TAPS > 0) {
-        float w[TAPS][VEC], x[TAPS - 1 + kAhead][VEC];           // a window of inputs: the taps before a block, then the block
-#pragma unroll
-        for (int j = 0; j < VEC; ++j)
-#pragma unroll
-            for (int k = 0; k < TAPS; ++k) w[k][j] = p.conv_w[static_cast<long long>(c0 + j) * TAPS + k];
+        float x[TAPS - 1 + kAhead][VEC];                         // a window of inputs: the taps before a block, then the block
 #pragma unroll
         for (int k = 0; k < TAPS - 1; ++k) fetch(t0 - (TAPS - 1) + k, x[k]);
         for (int tb = t0; tb < t1; tb += kAhead) {
@@ -138,9 +144,10 @@ ssd_conv_kernel(ConvTask p, const T* __restrict__ proj, T* __restrict__ state, T
 template <typename T, int NI>
 __global__ void __launch_bounds__(256, NI <= 4 ? 4 : NI <= 8 ? 3 : 2)
 ssd_scan_kernel(SsdParams p, const T* __restrict__ proj, const T* __restrict__ xbc, float* __restrict__ state, float* __restrict__ gated) {
-    pdl_begin();
     extern __shared__ float sm[];
     const int h = blockIdx.x / p.slices, sl = blockIdx.x - h * p.slices, b = blockIdx.y;
+    const float nA = -expf(__ldg(p.A_log + h)), dtb = __ldg(p.dt_bias + h), Dh = __ldg(p.D + h);      // (weights: ahead of the wait)
+    pdl_begin();
     const int g = h / (p.H / p.G), inner = p.H * p.P;
     const int pos = p.pos[b], slot = p.slots ? p.slots[b] : b;
     const int pc0 = sl * p.p4s * 4, pcn = min(p.P - pc0, p.p4s * 4);          // this slice's columns
@@ -155,7 +162,6 @@ ssd_scan_kernel(SsdParams p, const T* __restrict__ proj, const T* __restrict__ x
         const int n = r + i * p.rows;
         S[i] = active && n < p.N && pos > 0 ? *reinterpret_cast<const float4*>(sp + static_cast<long long>(n) * p.Pp) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    const float nA = -expf(p.A_log[h]), dtb = p.dt_bias[h], Dh = p.D[h];
     for (int t = 0; t < p.T; ++t) {
         const long long m = static_cast<long long>(b) * p.T + t;
         const T* prow = proj + m * p.ldp;
@@ -211,17 +217,23 @@ ssd_scan_kernel(SsdParams p, const T* __restrict__ proj, const T* __restrict__ x
 template <typename GT, typename T, bool VEC>
 __global__ void __launch_bounds__(128)
 gated_group_norm_kernel(const GT* __restrict__ gated, int inner, int part_len, const float* __restrict__ w, float eps, T* __restrict__ out, long long ldo) {
-    pdl_begin();
     const long long m = blockIdx.y;
     const int c0 = blockIdx.x * part_len;
     const GT* src = gated + m * inner + c0;
     T* dst = out + m * ldo + c0;
     __shared__ float part[4];
     float ss = 0.f;
+    if constexpr (!VEC) pdl_begin();
     if constexpr (VEC) {
-        constexpr int kMax = 8;
-        float v[kMax][8];
+        constexpr int kMax = 8, kHeld = 4;
+        float v[kMax][8], held[kHeld][8];            // the weights of the first columns are loaded ahead of the wait
         const int n8 = part_len / 8;
+#pragma unroll
+        for (int i = 0; i < kHeld; ++i) {
+            const int k = threadIdx.x + i * 128;
+            if (k < n8) load8(w + c0 + k * 8, held[i]);
+        }
+        pdl_begin();
 #pragma unroll
         for (int i = 0; i < kMax; ++i) {
             const int k = threadIdx.x + i * 128;
@@ -239,9 +251,9 @@ gated_group_norm_kernel(const GT* __restrict__ gated, int inner, int part_len, c
             const int k = threadIdx.x + i * 128;
             if (k >= n8) break;
             float wv[8];
-            load8(w + c0 + k * 8, wv);
+            if (i >= kHeld) load8(w + c0 + k * 8, wv);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) wv[e] *= v[i][e] * inv;
+            for (int e = 0; e < 8; ++e) wv[e] = (i < kHeld ? held[i < kHeld ? i : 0][e] : wv[e]) * (v[i][e] * inv);
             store8(dst + k * 8, wv);
         }
     } else {
