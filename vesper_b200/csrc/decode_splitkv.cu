@@ -217,8 +217,6 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_splitkv_kernel(Dec
         reinterpret_cast<int*>(p.workspace)[b] = sl.header();
         if (sl.overflow) atomicCAS(p.status, 0, (2 << 24) | (b & 0xFFFFFF));
     }
-    // let the combine kernel's blocks be scheduled as soon as every CTA of this grid has started
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const bool nothing = k_begin >= total;                          // no key for this split
     if (nothing && !p.cluster_merge) return;                        // (a cluster member stays for the cluster barriers)
     const int k_end = min(len, k_begin + p.chunk);                  // cached keys [k_begin, k_end)
@@ -317,10 +315,13 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) decode_splitkv_kernel(Dec
         const int group = warp * (32 / kLanes) + lane / kLanes;
         float* pbuf = pbuf_all + group * kLanes;
         bool ok = true;
+        // The next kernel's blocks may start once the last tile is here (a CTA that exits counts as one that said so): a product's, which fetch their weights at
+        // once, made the keys wait behind 20 MB of those (eight sequences of 110 keys between two products 12 -> 8 us).
         for (int t = 0; t < ntiles && ok; ++t) {
             int s = t % kStages;
             ok = mbar_wait(&sm->full[s], (t / kStages) & 1, abort_flag, 0x20);
             if (!ok) break;
+            if (t + 1 == ntiles) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             const T* ksm = ring + static_cast<size_t>(s) * (kStageBytes / sizeof(T));
             const T* vsm = ksm + kKeys * D;
             int nk = min(kKeys, k_end - (k_begin + t * kKeys));
