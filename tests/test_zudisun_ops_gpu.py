@@ -506,3 +506,28 @@ def test_experts_without_tokens(cuda):
     want = bf16_round((silu(h @ gate[-1].T) * (h @ up[-1].T)).astype(np.float32)).astype(np.float64) @ down[-1].T
     assert np.abs(got - want).max() <= TOL["bf16"] * np.abs(want).max()
     _status()
+
+
+@pytest.mark.parametrize("M,E,top", [(1, 3, 2), (33, 64, 6), (67, 40, 3), (341, 100, 3), (1365, 8, 3), (700, 1000, 7), (2050, 64, 6)])
+def test_rows_sorted_by_expert(cuda, M, E, top):
+    """Where each (token, choice) pair's row stands: by expert, pairs of one expert in their order.  Pair counts around multiples of the 4096 that
+    1024 threads take four at a time, ends that are no multiple of four, and experts whose counters do and do not fit several times."""
+    import torch
+    from vesper_b200 import hybrid_capi as hc
+    rng = np.random.default_rng(M)
+    dim = max(64, (E + 7) // 8 * 8)
+    x = np.zeros((M, dim), np.float32)                      # a token's logits are its values: whole numbers apart, so that the order is certain
+    x[:, :E] = rng.permuted(np.tile(np.arange(E), (M, 1)), axis=1) % 128 / 16 - 4
+    if E > 128:
+        x[:, :E] = -8
+        for m in range(M):
+            x[m, rng.permutation(E)[:top]] = np.arange(top)
+    router = np.eye(E, dim, dtype=np.float32)
+    w = lambda *s: _f32(bf16_round(rng.standard_normal(s) / 8), cuda)
+    core = hc.MoeCore(router=_f32(router, cuda), correction=None, gate=w(E, 8, dim), up=w(E, 8, dim), down=w(E, dim, 8), shared=None, top=top, groups=0, keep=0, scale=1.0, dtype=torch.bfloat16)
+    _, rows, gather = core.forward(_torch(x, cuda, torch.bfloat16), form=2)
+    ids = np.argsort(-x[:, :E], axis=1, kind="stable")[:, :top].ravel()
+    want = np.empty(M * top, np.int64)
+    want[np.argsort(ids, kind="stable")] = np.arange(M * top)
+    assert np.array_equal(gather.cpu().numpy().ravel(), want)
+    _status()
