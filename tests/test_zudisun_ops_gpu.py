@@ -382,6 +382,30 @@ def test_selective_scan_portions_and_slots(cuda, name, kind):
 
 
 @pytest.mark.parametrize("kind", ["f32", "bf16"])
+@pytest.mark.parametrize("cuts", [[32, 1, 32], [1, 32, 33], [2, 31, 64, 35], [3, 97]])
+def test_convolution_tiles_of_a_prompt(cuda, kind, cuts):
+    """Portions of whole tiles of 32 tokens, one more and one less, behind 0 to 3 earlier tokens; the last block of channels is not full."""
+    import torch
+    B, L = 2, sum(cuts)
+    core, w, rng = _scan_case("many channels", kind, cuda, slots=3, seed=L)
+    inner = SCAN["many channels"][0]
+    ps = [_rnd(kind)(rng.standard_normal((L, 2 * inner))) for _ in range(B)]
+    wants = [_scan_want(p, w, "many channels", kind) for p in ps]
+    core.state.fill_(1e3); core.conv_state.fill_(9.0)
+    st, at = _torch(np.array([2, 0], np.int32), cuda), 0
+    for n in cuts:
+        proj = _torch(np.concatenate([p[at:at + n] for p in ps]), cuda, core.dtype)
+        y = _np(core.forward(proj, B, torch.full((B,), at, dtype=torch.int32, device=cuda), slots=st)).reshape(B, n, inner)
+        at += n
+        for b, slot in enumerate((2, 0)):
+            assert np.abs(y[b] - wants[b][at - n:at]).max() <= (5e-5 if kind == "f32" else 2e-2) * np.abs(wants[b]).max(), (at, b)
+            for t in range(max(0, at - 3), at):            # the ring of inputs that the next portion starts from: copied, so exact
+                assert np.array_equal(_np(core.conv_state)[slot, t % 4], _np(proj)[b * n + t - at + n, :inner] if t >= at - n else _np(_torch(ps[b][t, :inner], cuda, core.dtype)))
+    assert np.all(_np(core.conv_state)[1] == 9.0)
+    _status()
+
+
+@pytest.mark.parametrize("kind", ["f32", "bf16"])
 def test_selective_steps_of_many_sequences(cuda, kind):
     """Enough rows for the step sizes to become a product of their own; sequences at unequal lengths, one of them new."""
     import torch
