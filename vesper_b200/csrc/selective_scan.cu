@@ -96,9 +96,7 @@ template <typename T, int LP, int NI>
 struct ScanTile {
     static constexpr int kCh = kThreads / LP;                  // channels per CTA
     static constexpr int kStates = LP * NI;
-    // tokens per shared-memory tile: 16 leave room for nine CTAs of the common shapes on an SM instead of six (8 x 512 tokens, 4096 channels of 16 states, 1024 CTAs:
-    // 142 -> 134 us)
-    static constexpr int kTile = kStates > 256 ? 8 : sizeof(T) == 2 ? 16 : 32;
+    static constexpr int kTile = kStates > 256 ? 8 : 32;      // tokens per shared-memory tile
     struct Stage {
         alignas(16) T x[kTile][kCh], z[kTile][kCh];
         alignas(16) float dt[kTile][kCh];
