@@ -75,6 +75,31 @@ def test_portions_of_a_prompt(cuda, D, T, start, rotate):
 
 
 @pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_masked_columns_of_huge_scores(cuda, D, causal):
+    """Scores of both signs around 1e10, where a float's neighbours are 1024 apart: masked columns and those past the end weigh nothing.
+
+    A row's weights are 1 for its largest score and 0 for the others, unless its two largest lie within the error of a score
+    (D / 16 + 8 additions of 2^-23 of the largest sum of magnitudes); such rows, about one in 10^5, are left out."""
+    import torch
+    from vesper_b200 import capi
+    N = 201
+    g = torch.Generator(device=cuda).manual_seed(D)
+    q, k, v = (torch.randn(1, 4, N, D, generator=g, device=cuda) * f for f in (3e5, 3e5, 1))
+    o, lse = torch.empty_like(q), torch.empty(1, 4, N, device=cuda)
+    capi.prefill(q, k, v, o, lse, scale=D ** -0.5, causal=causal)
+    want, want_lse = _reference(q, k, v, None, 0, causal)
+    s = q.double() @ k.double().transpose(2, 3) * D ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(N, N, dtype=torch.bool, device=cuda).triu(1), -math.inf)
+    two = s.topk(2, -1).values
+    error = (D / 16 + 8) * 2 ** -23 * (q.double().abs() @ k.double().abs().transpose(2, 3)).amax(-1) * D ** -0.5
+    sure = two[..., 0] - two[..., 1] > 2 * error + 100
+    assert sure.float().mean() > 0.99
+    assert _off(o[sure], want[sure]) <= BOUND and ((lse.double() - want_lse).abs() <= error)[sure].all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("value", [math.nan, math.inf, 3.4e38, 1e-33])
 def test_values_that_three_terms_do_not_hold(cuda, D, value):
     """Four columns of one row of V outside the range: what does not depend on them is as before, and the others hold what fp32 gives."""

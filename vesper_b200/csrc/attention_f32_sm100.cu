@@ -386,17 +386,18 @@ __device__ __forceinline__ void attend(const Job& j, unsigned char* tiles, Share
                 for (int i = 0; i < kCols; i += 2) mx[(i >> 1) & 3] = fmax3(mx[(i >> 1) & 3], s[i], s[i + 1]);
                 const float top = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
                 const float alpha = expf(m - top);                       // the first block holds a visible column: top is finite, or the rows are computed again
-                if (edge)                                                // (far below the others, and finite: the weight is zero)
-#pragma unroll
-                    for (int i = 0; i < kCols; ++i)
-                        if (i < lo - c0 || i >= hi - c0) s[i] = top - 200.f;
-                float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
                 for (int i = 0; i < kCols; i += 2) {
                     const float2 w = exp_pair_exact(__fadd2_rn(make_float2(s[i], s[i + 1]), make_float2(-top, -top)));
                     s[i] = w.x; s[i + 1] = w.y;
-                    sum[(i >> 1) & 1] = __fadd2_rn(sum[(i >> 1) & 1], w);
                 }
+                if (edge)                                                // the weight itself: a score far enough below any top is not a number of 24 bits
+#pragma unroll
+                    for (int i = 0; i < kCols; ++i)
+                        if (i < lo - c0 || i >= hi - c0) s[i] = 0.f;
+                float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+                for (int i = 0; i < kCols; i += 2) sum[(i >> 1) & 1] = __fadd2_rn(sum[(i >> 1) & 1], make_float2(s[i], s[i + 1]));
                 l = fmaf(l, alpha, (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y));
                 m = top;
                 sh.alpha[blk & 3][r] = alpha;
