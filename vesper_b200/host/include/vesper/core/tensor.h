@@ -59,16 +59,20 @@ public:
     static Stream& default_stream(Device device);
     static void set_current(const Stream& stream);
     static Stream& current(Device device);
+    // Destroys the CUDA stream with its last holder; null for the default stream.  Buffers hold the streams that they were used on.
+    const std::shared_ptr<void>& owner() const { return owner_; }
 
 private:
-    Stream(Device device, void* handle, bool own) : device_(device), handle_(handle), own_(own) {}
+    Stream(Device device, std::nullptr_t) : device_(device) {}
     Device device_;
     void* handle_ = nullptr;
-    bool own_ = true;
+    std::shared_ptr<void> owner_;
 };
 
 // Reference-counted buffer; CUDA buffers come from a small caching allocator
-// (power-of-two bins, as src/core/allocator.cpp:171-221 does).
+// (power-of-two bins, as src/core/allocator.cpp:171-221 does).  A buffer may be let go of while
+// the stream that was current when it was created, or the one current now, still has work on it: another stream
+// gets it only afterwards.  (Work on a third stream has to be waited for first.)
 class Storage {
 public:
     Storage(size_t bytes, Device device);
@@ -84,6 +88,7 @@ private:
     size_t bytes_ = 0, alloc_bytes_ = 0;
     Device device_;
     int ordinal_ = 0;
+    std::vector<std::shared_ptr<void>> streams_;    // whose work may still use data_
 };
 
 class Tensor {

@@ -19,9 +19,28 @@ void cuda_check(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+// Streams (Stream::owner) whose queued work may still use a block.  The legacy default stream needs no entry: streams of this
+// library are blocking ones, so its work and theirs are in order.
+using Streams = std::vector<std::shared_ptr<void>>;
+
+void add_stream(Streams& list, const std::shared_ptr<void>& s) {
+    for (const auto& x : list) if (x == s) return;
+    if (s) list.push_back(s);
+}
+
+bool idle(const std::shared_ptr<void>& s) {
+    cudaStream_t stream = static_cast<cudaStream_t>(s.get());
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e == cudaErrorNotReady) cudaGetLastError();          // an answer, not an error for the next check to find
+    return e == cudaSuccess;
+}
+
 // Caching allocator: freed blocks are kept per (device, rounded size) and
 // handed out again; nothing is returned to the driver before process exit
-// (src/core/allocator.cpp:205-221 has the same policy).
+// (src/core/allocator.cpp:205-221 has the same policy).  A block goes to work of the streams that it was used on, or of the
+// default stream, at once (their order is the stream's), to other streams when those are idle.
 class CachingAllocator {
 public:
     static CachingAllocator& get() { static CachingAllocator* a = new CachingAllocator(); return *a; }
@@ -30,24 +49,39 @@ public:
         while (r < n) r <<= 1;
         return r;
     }
-    void* alloc(size_t rounded, int dev) {
+    // `current`: the stream that asks; `streams`: those whose work may still use the block
+    void* alloc(size_t rounded, int dev, const std::shared_ptr<void>& current, Streams& streams) {
         {
             std::lock_guard<std::mutex> lock(mu_);
             auto& bin = free_[{dev, rounded}];
-            if (!bin.empty()) { void* p = bin.back(); bin.pop_back(); return p; }
+            for (size_t i = bin.size(); i-- > 0;) {
+                Block& b = bin[i];
+                const bool only_own = b.streams.empty() || (b.streams.size() == 1 && b.streams[0] == current);
+                if (current ? !only_own : b.streams.size() > 4) drop_idle(b.streams, current);
+                if (current && !(b.streams.empty() || (b.streams.size() == 1 && b.streams[0] == current))) continue;
+                void* p = b.p;
+                streams = std::move(b.streams);
+                bin.erase(bin.begin() + static_cast<std::ptrdiff_t>(i));
+                return p;
+            }
         }
         void* p = nullptr;
         cuda_check(cudaMalloc(&p, rounded), "cudaMalloc");
         return p;
     }
-    void release(void* p, size_t rounded, int dev) {
+    void release(void* p, size_t rounded, int dev, Streams streams) {
         std::lock_guard<std::mutex> lock(mu_);
-        free_[{dev, rounded}].push_back(p);
+        free_[{dev, rounded}].push_back(Block{p, std::move(streams)});
     }
 
 private:
+    struct Block { void* p; Streams streams; };
+    static void drop_idle(Streams& list, const std::shared_ptr<void>& except) {
+        for (size_t i = list.size(); i-- > 0;)
+            if (list[i] != except && idle(list[i])) list.erase(list.begin() + static_cast<std::ptrdiff_t>(i));
+    }
     std::mutex mu_;
-    std::map<std::pair<int, size_t>, std::vector<void*>> free_;
+    std::map<std::pair<int, size_t>, std::vector<Block>> free_;
 };
 
 thread_local Stream* t_current = nullptr;
@@ -75,18 +109,18 @@ Stream::Stream(Device device) : device_(device) {
         cudaStream_t s;
         cuda_check(cudaStreamCreate(&s), "cudaStreamCreate");
         handle_ = s;
+        owner_ = std::shared_ptr<void>(s, [](void* h) { cudaStreamDestroy(static_cast<cudaStream_t>(h)); });
     }
 }
 Stream::~Stream() {
-    if (own_ && handle_) cudaStreamDestroy(static_cast<cudaStream_t>(handle_));
     if (t_current == this) t_current = nullptr;
 }
 void Stream::synchronize() const {
     if (device_ == Device::CUDA) cuda_check(cudaStreamSynchronize(static_cast<cudaStream_t>(handle_)), "cudaStreamSynchronize");
 }
 Stream& Stream::default_stream(Device device) {
-    static Stream cuda_default(Device::CUDA, nullptr, false);   // legacy stream 0 (src/core/stream.cpp:104-111)
-    static Stream cpu_default(Device::CPU, nullptr, false);
+    static Stream& cuda_default = *new Stream(Device::CUDA, nullptr);   // legacy stream 0 (src/core/stream.cpp:104-111)
+    static Stream& cpu_default = *new Stream(Device::CPU, nullptr);
     return device == Device::CUDA ? cuda_default : cpu_default;
 }
 void Stream::set_current(const Stream& stream) { t_current = const_cast<Stream*>(&stream); }
@@ -101,14 +135,18 @@ Storage::Storage(size_t bytes, Device device) : bytes_(bytes), device_(device) {
     if (device == Device::CUDA) {
         cuda_check(cudaGetDevice(&ordinal_), "cudaGetDevice");
         alloc_bytes_ = CachingAllocator::round(bytes ? bytes : 1);
-        data_ = CachingAllocator::get().alloc(alloc_bytes_, ordinal_);
+        const std::shared_ptr<void>& current = Stream::current(Device::CUDA).owner();
+        data_ = CachingAllocator::get().alloc(alloc_bytes_, ordinal_, current, streams_);
+        add_stream(streams_, current);
     } else {
         data_ = ::operator new(bytes ? bytes : 1);
     }
 }
 Storage::~Storage() {
-    if (device_ == Device::CUDA) CachingAllocator::get().release(data_, alloc_bytes_, ordinal_);
-    else ::operator delete(data_);
+    if (device_ == Device::CUDA) {
+        add_stream(streams_, Stream::current(Device::CUDA).owner());
+        CachingAllocator::get().release(data_, alloc_bytes_, ordinal_, std::move(streams_));
+    } else ::operator delete(data_);
 }
 
 // ---- Tensor ----
