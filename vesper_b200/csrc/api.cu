@@ -262,6 +262,16 @@ void vb200_rope_inv_freq(float theta, int32_t D, float* inv_freq_host) {
     for (int i = 0; i < D / 2; ++i) inv_freq_host[i] = std::pow(theta, -2.0f * i / D);
 }
 
+int vb200_copy_kernel_status(int device, void* stream, int32_t* host_word) {
+    if (!host_word) return set_detail(VB200_ERR_INVALID_ARG, "vb200_copy_kernel_status: null word");
+    DeviceGuard g;
+    if (int rc = g.init(device)) return rc;
+    const int* word = kernel_status_word();
+    if (!word) return set_detail(VB200_ERR_CUDA, "cannot resolve the device status word");
+    VB200_CUDA_TRY(cudaMemcpyAsync(host_word, word, sizeof(int), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
+    return VB200_OK;
+}
+
 int vb200_check_kernel_status(int device, void* stream) {
     DeviceGuard g;
     if (int rc = g.init(device)) return rc;
@@ -273,6 +283,11 @@ int vb200_check_kernel_status(int device, void* stream) {
     int zero = 0;
     VB200_CUDA_TRY(cudaMemcpyToSymbolAsync(g_kernel_status, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, s));
     VB200_CUDA_TRY(cudaStreamSynchronize(s));
+    return vb200_kernel_status_of(host);
+}
+
+int vb200_kernel_status_of(int32_t host) {
+    if (host == 0) return VB200_OK;
     char buf[96];
     if ((host >> 24) == 2) {
         std::snprintf(buf, sizeof(buf), "decode: sequence %d is full (token not appended, length not advanced)", host & 0xFFFFFF);

@@ -146,6 +146,12 @@ struct WaitCtx {
     int* status;                // device status word
 };
 
+// The first code stays in the status word, except that an expired wait replaces a note about a full sequence or an id out of range: results
+// behind it are not results.
+__device__ __forceinline__ void record_expired(int* status, int word) {
+    if ((atomicCAS(status, 0, word) >> 24) == 2) atomicExch(status, word);
+}
+
 // kCluster: acquires at cluster scope, for data that other CTAs of the cluster have stored.
 template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, int where) {
@@ -172,7 +178,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
             if (t0 == 0) t0 = now;
             else if (now - t0 > kWaitCycles) {
                 *ctx.abort_flag = 1;
-                atomicCAS(ctx.status, 0, (1 << 24) | where);
+                record_expired(ctx.status, (1 << 24) | where);
                 return false;
             }
         }

@@ -81,7 +81,7 @@ __device__ __forceinline__ void exchange_rows(const ExchangeParams& p, int c, lo
             for (unsigned it = 0; ld_word(last).y != step; ++it)
                 if ((it & 63) == 63 && clock64() - t0 > p.timeout_cycles) {
                     *s_ok = 0;
-                    atomicCAS(p.status, 0, (3 << 24) | (tid << 8) | 0x71);      // which rank never arrived
+                    record_expired(p.status, (3 << 24) | (tid << 8) | 0x71);      // which rank never arrived
                     break;
                 }
         }
@@ -105,7 +105,7 @@ __device__ __forceinline__ void exchange_rows(const ExchangeParams& p, int c, lo
             if (*s_step == 0) break;
             if (late >= 0 && clock64() - t0 > p.timeout_cycles) {
                 *s_ok = 0;
-                atomicCAS(p.status, 0, (3 << 24) | (late << 8) | 0x72);
+                record_expired(p.status, (3 << 24) | (late << 8) | 0x72);
             }
             sync();
         }
@@ -124,7 +124,7 @@ __device__ __forceinline__ void exchange_rows(const ExchangeParams& p, int c, lo
                 }
                 if (!all && (it & 15) == 15 && clock64() - t0 > p.timeout_cycles) {
                     *s_ok = 0;
-                    atomicCAS(p.status, 0, (3 << 24) | (((i0 / n) & 0xFF) << 8) | 0x73);
+                    record_expired(p.status, (3 << 24) | (((i0 / n) & 0xFF) << 8) | 0x73);
                     break;
                 }
             }

@@ -53,6 +53,8 @@ public:
     ~Stream();
     Stream(const Stream&) = delete;
     Stream& operator=(const Stream&) = delete;
+    // Waits for the stream's work; throws if a wait inside one of the library's kernels has expired on the current device, since what was
+    // computed behind it is no result then.
     void synchronize() const;
     void* raw_handle() const { return handle_; }
     Device device() const { return device_; }

@@ -90,6 +90,11 @@ Tensor Generator::generate(const Tensor& prompt_ids, const SamplingParams& param
     const bool graph_ok = use_graph_ && device_decode && max_new > 2;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    struct Release {
+        cudaGraph_t& graph;
+        cudaGraphExec_t& exec;
+        ~Release() { if (exec) cudaGraphExecDestroy(exec); if (graph) cudaGraphDestroy(graph); }
+    } release{graph, exec};
     std::vector<int32_t> done_host(static_cast<size_t>(B));
     auto all_done = [&]() {
         st.done.copy_to_host(done_host.data());
@@ -132,9 +137,7 @@ Tensor Generator::generate(const Tensor& prompt_ids, const SamplingParams& param
         if (!params.stop_token_ids.empty() && (steps % poll_every_ == 0 || generated == max_new)) stopped = all_done();
     }
     cuda_check(cudaEventRecord(dec.b, stream), "cudaEventRecord");
-    cuda_check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+    own.synchronize();
     timings_.prefill_ms = pre.ms();
     timings_.decode_ms = dec.ms();
     timings_.decode_steps = steps;

@@ -84,6 +84,13 @@ private:
     std::map<std::pair<int, size_t>, std::vector<Block>> free_;
 };
 
+// A word of page-locked memory per thread, into which the device status word is copied along with a synchronisation.
+struct PageLockedWord {
+    int32_t* p = nullptr;
+    PageLockedWord() { cuda_check(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int32_t), cudaHostAllocPortable), "cudaHostAlloc"); *p = 0; }
+    ~PageLockedWord() { cudaFreeHost(p); }
+};
+
 thread_local Stream* t_current = nullptr;
 
 std::vector<int64_t> contiguous_strides(const std::vector<int64_t>& shape) {
@@ -116,7 +123,15 @@ Stream::~Stream() {
     if (t_current == this) t_current = nullptr;
 }
 void Stream::synchronize() const {
-    if (device_ == Device::CUDA) cuda_check(cudaStreamSynchronize(static_cast<cudaStream_t>(handle_)), "cudaStreamSynchronize");
+    if (device_ != Device::CUDA) return;
+    static thread_local PageLockedWord word;
+    const int queued = vb200_copy_kernel_status(-1, handle_, word.p);
+    cuda_check(cudaStreamSynchronize(static_cast<cudaStream_t>(handle_)), "cudaStreamSynchronize");
+    // (a note about a full sequence or an id out of range stays for vb200_check_kernel_status)
+    if (queued != VB200_OK || vb200_kernel_status_of(*word.p) != VB200_ERR_KERNEL_TIMEOUT) return;
+    const std::string text = vb200_last_error_detail();
+    vb200_check_kernel_status(-1, handle_);                  // clears it
+    throw std::runtime_error("a kernel gave up waiting, its results are void: " + text);
 }
 Stream& Stream::default_stream(Device device) {
     static Stream& cuda_default = *new Stream(Device::CUDA, nullptr);   // legacy stream 0 (src/core/stream.cpp:104-111)
@@ -176,7 +191,7 @@ void Tensor::copy_to_host(void* host_ptr) const {
     if (!is_contiguous()) { contiguous().copy_to_host(host_ptr); return; }
     size_t bytes = numel() * GetDTypeSize(dtype_);
     if (device() == Device::CUDA) {
-        cuda_check(cudaStreamSynchronize(static_cast<cudaStream_t>(Stream::current(Device::CUDA).raw_handle())), "sync");
+        Stream::current(Device::CUDA).synchronize();
         cuda_check(cudaMemcpy(host_ptr, data_ptr<char>(), bytes, cudaMemcpyDeviceToHost), "cudaMemcpy D2H");
     } else {
         std::memcpy(host_ptr, data_ptr<char>(), bytes);
