@@ -225,6 +225,7 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
     uint64_t* drain = acc_empty + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* row_tiles = reinterpret_cast<int*>(tmem_slot + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int m_tiles = (p.M + kTileA - 1) / kTileA;
@@ -250,7 +251,11 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
     // anything); the activations may come from the kernel launched just before this one
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (GROUPED) m_tiles = min(*p.group_tile_count, p.group_tile_max);
+    if (GROUPED) {                                // read once: copies, products and epilogue must agree on the number of tiles, or each waits for the others
+        if (threadIdx.x == 0) *row_tiles = max(0, min(__ldcg(p.group_tile_count), p.group_tile_max));
+        __syncthreads();
+        m_tiles = *row_tiles;
+    }
     const int tiles = m_tiles * n_tiles;
 
     if (warp == 0) {
@@ -260,7 +265,7 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
                 // consecutive CTAs share a W tile through L2; grouped: a row tile, and a group's W stays in L2 for its few row tiles
                 const int mt = GROUPED ? t / n_tiles : t % m_tiles, nt = GROUPED ? t % n_tiles : t / m_tiles;
                 int row0 = mt * kTileA, w0 = nt * BN;
-                if (GROUPED) { const int4 g = p.group_tiles[mt]; row0 = g.x; w0 += g.z * p.group_rows; }
+                if (GROUPED) { const int4 g = __ldcg(p.group_tiles + mt); row0 = g.x; w0 += g.z * p.group_rows; }
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % C::kStages;
                     if (it >= C::kStages && !mbar_wait(&empty[s], ((it / C::kStages) - 1) & 1, ctx, 0x41)) break;
@@ -309,7 +314,7 @@ linear_wide_kernel(const __grid_constant__ LinearMaps maps, LinearParams p) {
             if (!mbar_wait_warp(&acc_full[buf], (tile_no >> 1) & 1, ctx, 0x45)) break;
             tc_fence_after();
             int row = mt * kTileA, row_end = p.M;
-            if (GROUPED) { const int4 g = p.group_tiles[mt]; row = g.x; row_end = g.y; }
+            if (GROUPED) { const int4 g = __ldcg(p.group_tiles + mt); row = g.x; row_end = g.y; }
             row += quarter * 32 + lane;
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
