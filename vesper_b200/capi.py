@@ -206,6 +206,14 @@ def _stream_ptr(stream):
     return C.c_void_p(s.cuda_stream)
 
 
+def _workspace(nbytes, device, stream):
+    """Bytes that belong to `stream` (None: the current one): torch gives their memory to later work of that stream only."""
+    import contextlib
+    import torch
+    with torch.cuda.stream(stream) if isinstance(stream, torch.cuda.Stream) else contextlib.nullcontext():
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+
+
 def _ptr(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
@@ -240,13 +248,12 @@ def prefill_args(q, k, v, o, lse=None, *, scale, causal=True, start_pos=0, theta
 def prefill(q, k, v, o, lse=None, *, scale, causal=True, start_pos=0, theta=None,
             k_cache=None, v_cache=None, workspace=None, stream=None, cache_read_only=False):
     """vb200_prefill_fwd on torch CUDA tensors.  Allocates a workspace with torch when none is given."""
-    import torch
     L = load()
     a = prefill_args(q, k, v, o, lse, scale=scale, causal=causal, start_pos=start_pos, theta=theta,
                      k_cache=k_cache, v_cache=v_cache, workspace=workspace, stream=stream, cache_read_only=cache_read_only)
     need = L.vb200_prefill_workspace_bytes(C.byref(a))
     if need > a.workspace_bytes:
-        workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
+        workspace = _workspace(need, q.device, stream)
         a.workspace, a.workspace_bytes = _ptr(workspace), need
     check(L.vb200_prefill_fwd(C.byref(a)))
     return workspace
@@ -285,13 +292,12 @@ def decode_args(q, o, k_cache, v_cache, *, scale, k_new=None, v_new=None, lse=No
 
 def decode(q, o, k_cache, v_cache, **kw):
     """vb200_decode_fwd on torch CUDA tensors.  Allocates a workspace with torch when none is given."""
-    import torch
     L = load()
     a = decode_args(q, o, k_cache, v_cache, **kw)
     need = L.vb200_decode_workspace_bytes(C.byref(a))
     ws = kw.get("workspace")
     if need > a.workspace_bytes:
-        ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+        ws = _workspace(need, q.device, kw.get("stream"))
         a.workspace, a.workspace_bytes = _ptr(ws), need
     check(L.vb200_decode_fwd(C.byref(a)))
     return ws
@@ -330,11 +336,14 @@ def attention_bwd(d_out, q, k, v, out, lse, *, scale, causal=True, stream=None):
     a.dtype = dtype_code(q)
     a.B, a.H, a.N, a.D, a.causal, a.scale = B, H, N, D, int(causal), scale
     dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.empty_like(q)
+    if isinstance(stream, torch.cuda.Stream):
+        for t in (dq, dk, dv):
+            t.record_stream(stream)                        # let go of early, they are not the current stream's again before this call is done
     for name, t in (("d_out", d_out), ("q", q), ("k", k), ("v", v), ("out", out), ("lse", lse), ("dq", dq), ("dk", dk), ("dv", dv)):
         assert t.is_contiguous()
         setattr(a, name, _ptr(t))
     need = load().vb200_attention_bwd_workspace_bytes(C.byref(a))
-    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+    ws = _workspace(need, q.device, stream)
     a.workspace, a.workspace_bytes = _ptr(ws), need
     check(load().vb200_attention_bwd(C.byref(a)))
     return dq, dk, dv
@@ -375,14 +384,13 @@ def decode_exchange(q, k_cache, v_cache, peer_ptrs, rank, out, lse=None, *, time
     """vb200_decode_exchange_fwd: this rank's shard of a sequence-sharded decode step, split merge and exchange in one
     launch.  out [B*Hq, D] (bf16/fp16), lse [B*Hq]; kw as for decode_args (scale, theta, uniform_len, max_len, pos_offset,
     q_positions, ...)."""
-    import torch
     L = load()
     B, Hq, _, D = q.shape
     stream = kw.get("stream")
     a = decode_args(q, None, k_cache, v_cache, workspace=workspace, **kw)
     need = L.vb200_decode_workspace_bytes(C.byref(a))
     if need > a.workspace_bytes:
-        workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
+        workspace = _workspace(need, q.device, stream)
         a.workspace, a.workspace_bytes = _ptr(workspace), need
     x = exchange_args(peer_ptrs, rank, out, lse, rows=B * Hq, D=D, step=step, timeout_cycles=timeout_cycles, stream=stream)
     check(L.vb200_decode_exchange_fwd(C.byref(a), C.byref(x)))
