@@ -125,6 +125,28 @@ def test_values_that_three_terms_do_not_hold(cuda, D, value):
 
 
 @pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("tiny", ["q", "k", "v", "do"])
+def test_one_tiny_column_beside_normal_ones(cuda, D, tiny):
+    """Column 5 of one operand at 1e-37, whose second and third bf16 terms are subnormal: that column of the results it makes
+    (V: O, dO: dV, K: dQ, Q: dK) keeps what fp32 gives there, 1e-5 as for the gradient below, and the other columns are as before."""
+    import torch
+    from vesper_b200 import capi
+    N = 200
+    g = torch.Generator(device=cuda).manual_seed(D)
+    t = {n: torch.randn(1, 2, N, D, generator=g, device=cuda) for n in ("q", "k", "v", "do")}
+    t[tiny][..., 5] *= 1e-37
+    o, lse = torch.empty_like(t["q"]), torch.empty(1, 2, N, device=cuda)
+    capi.prefill(t["q"], t["k"], t["v"], o, lse, scale=D ** -0.5, causal=True)
+    got = dict(zip(("o", "dq", "dk", "dv"), (o, *capi.attention_bwd(t["do"], t["q"], t["k"], t["v"], o, lse, scale=D ** -0.5, causal=True))))
+    want = _reference(t["q"], t["k"], t["v"], t["do"], 0, True)
+    want = dict(zip(("o", "dq", "dk", "dv"), (want[0], *want[2:])))
+    made = {"v": "o", "do": "dv", "k": "dq", "q": "dk"}[tiny]
+    assert _off(got[made][..., 5], want[made][..., 5]) <= 1e-5
+    for n in got:
+        assert _off(got[n], want[n]) <= 2 * BOUND
+
+
+@pytest.mark.parametrize("D", [64, 128])
 def test_a_gradient_far_below_the_range(cuda, D):
     """dO of 1e-33: its second and third terms would be subnormal; 1e-5 as fp32 rounds numbers of 1e-36."""
     import torch

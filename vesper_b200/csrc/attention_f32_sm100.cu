@@ -30,8 +30,9 @@
 //
 // TMEM columns: A1 [3 D/2], A2 [terms in TMEM], per slot X [64] (and Y [64]) overwritten by the terms of W [96], the block sum [D].
 //
-// Numbers outside 2^-100 .. 2^126 (or inf, NaN) have terms that bf16 does not hold, and 0 * inf of a masked position would reach
-// every row of a tile: a CTA that meets one computes its rows again on the CUDA cores (plain_rows), in the order of a plain loop.
+// Numbers outside 2^-100 .. 2^126 (or inf, NaN; zeros are fine) have terms that bf16 does not hold, and 0 * inf of a masked position would
+// reach every row of a tile: a CTA that meets one element of that kind in its rows or blocks computes its rows again on the CUDA cores
+// (plain_rows), in the order of a plain loop.  Weights are not looked at: below 2^-100 they lose bits that matter only to a row without larger ones.
 #include "kernels.h"
 #include "hybrid.cuh"
 
@@ -122,8 +123,10 @@ __device__ __forceinline__ float4 load4(const float* p, bool valid) {
         : "=&f"(x.x), "=&f"(x.y), "=&f"(x.z), "=&f"(x.w) : "l"(p), "r"(static_cast<int>(valid)));
     return x;
 }
-__device__ __forceinline__ float largest(float4 x) { return fmax3(fabsf(x.x), fabsf(x.y), fmaxf(fabsf(x.z), fabsf(x.w))); }
-__device__ __forceinline__ bool too_small(float m) { return m < kLeast && m > 0.f; }
+// The least magnitude but zero that has been met, as twice its bits less one: zero, of either sign, becomes the largest.
+__device__ __forceinline__ uint32_t doubled(float x) { return 2 * __float_as_uint(x) - 1; }
+__device__ __forceinline__ uint32_t least_of(uint32_t least, float4 x) { return min(least, min(min(doubled(x.x), doubled(x.y)), min(doubled(x.z), doubled(x.w)))); }
+__device__ __forceinline__ bool too_small(uint32_t least) { return least < doubled(kLeast); }
 // e^x: the exponent x log2 e is rounded once, an error of |x| 2^-24 of the result at most, below that of the scores
 __device__ __forceinline__ float2 exp_pair(float2 x) {
     const float2 t = __fmul2_rn(x, make_float2(kLog2e, kLog2e));
@@ -257,7 +260,7 @@ __device__ __forceinline__ bool resident(const float2* rope, int row0, int rows,
     const int warp = threadIdx.x >> 5, half = warp >> 2, r = threadIdx.x & 127, row = row0 + r;
     const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
     float2 chk = make_float2(0.f, 0.f);
-    bool outside = false;
+    uint32_t least = ~0u;
 #pragma unroll 2
     for (int c = half * (D / 2); c < (half + 1) * (D / 2); c += 16) {
         const uint32_t at = lanes + col + c / 2;
@@ -267,7 +270,7 @@ __device__ __forceinline__ bool resident(const float2* rope, int row0, int rows,
             float4 v;
             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(stage + r * (D * 4) + (((c / 4 + i) ^ (r & 7)) << 4)));
             if (rope != nullptr && row < rows) v = rotated(v, rope + static_cast<long long>(row) * (D / 2) + c / 2 + 2 * i);
-            outside |= too_small(largest(v));
+            least = least_of(least, v);
             split3(v.x, v.y, t0[2 * i], t1[2 * i], t2[2 * i], chk);
             split3(v.z, v.w, t0[2 * i + 1], t1[2 * i + 1], t2[2 * i + 1], chk);
         }
@@ -285,7 +288,7 @@ __device__ __forceinline__ bool resident(const float2* rope, int row0, int rows,
             }
         }
     }
-    return outside || not_zero(chk);
+    return too_small(least) || not_zero(chk);
 }
 
 // the warp's arrival, after what its lanes have done
@@ -675,13 +678,13 @@ split_blocks_kernel(const __grid_constant__ SplitParams p) {
     const long long block = static_cast<long long>(blockIdx.y) * p.blocks + blockIdx.x;
     unsigned char* dst = t.terms + block * (3 * kCols * D * 2);
     float2 chk = make_float2(0.f, 0.f);
-    bool outside = false;
+    uint32_t least = ~0u;
     constexpr int kLanes = D / 8;              // threads of a row
 #pragma unroll
     for (int i = 0; i < kCols * kLanes / 256; ++i) {
         const int at = threadIdx.x + i * 256, r = at / kLanes, c = at % kLanes * 8, row = row0 + r;
         const float4 x = load4(src + row * t.ss + c, row < p.rows), y = load4(src + row * t.ss + c + 4, row < p.rows);
-        outside |= too_small(fmaxf(largest(x), largest(y)));
+        least = least_of(least_of(least, x), y);
         uint4 t0, t1, t2;
         split3(x.x, x.y, t0.x, t1.x, t2.x, chk);
         split3(x.z, x.w, t0.y, t1.y, t2.y, chk);
@@ -700,7 +703,7 @@ split_blocks_kernel(const __grid_constant__ SplitParams p) {
             if (c == 0 && row < p.rows) p.delta[flat] = d;
         }
     }
-    const int any = __syncthreads_or(outside || not_zero(chk));
+    const int any = __syncthreads_or(too_small(least) || not_zero(chk));
     if (threadIdx.x == 0) t.marks[block] = any;
 }
 
