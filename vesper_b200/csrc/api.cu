@@ -575,7 +575,7 @@ int vb200_attention_bwd(const vb200_attention_bwd_args* a) {
     if (!a->d_out || !a->q || !a->k || !a->v || !a->out || !a->lse || !a->dq || !a->dk || !a->dv)
         return set_detail(VB200_ERR_INVALID_ARG, "vb200_attention_bwd: null tensor");
     // enough for the row sums: the CUDA cores; enough for the terms too, and aligned: the tensor cores
-    if (!a->workspace || a->workspace_bytes < bwd_delta_bytes(a))
+    if (!a->workspace || a->workspace_bytes < sizeof(float) * static_cast<size_t>(a->B) * a->H * a->N)
         return set_detail(VB200_ERR_WORKSPACE, "vb200_attention_bwd: workspace missing or too small");
     DeviceGuard g;
     if (int rc = g.init(a->device)) return rc;
