@@ -148,18 +148,34 @@ __device__ __forceinline__ float4 rotated(float4 x, const float2* t) {
                        __fsub_rn(__fmul_rn(x.z, c1.x), __fmul_rn(x.w, c1.y)), __fadd_rn(__fmul_rn(x.z, c1.y), __fmul_rn(x.w, c1.x)));
 }
 
-// The same rows by plain loops, masked columns left out: a warp takes four rows and four columns at a time, a lane D / 32 dimensions.
+// v[i], i < 32, of every lane -> lane i has the sum over the lanes of v[i]: halves of the values are exchanged, 31 shuffles in place of 160.
+__device__ __forceinline__ float sum_across(float (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const bool upper = lane & o;
+            const float send = upper ? v[i] : v[i + o], keep = upper ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
+        }
+    return v[0];
+}
+
+// The same rows by plain loops, masked columns left out: a warp takes four rows and eight columns at a time, for the products with a lane per D / 32
+// dimensions, for the weights with a lane per (row, column).  Bound by shuffles, about 60 of them (forward) to 130 (dQ, dK) per 32 weights, on ten warps
+// of an SM.  One NaN in every head of V, forward / backward: 2 x 8 x 512 x 64 360 / 406 us, 2 x 16 x 1999 x 128 3460 / 8360 (each value summed over the
+// lanes by itself, four columns at a time: 910 / 1185, 7330 / 29250; the CUDA-core kernels, which have no such case: 87 / 160, 1150 / 3120).
 template <int D, int USE>
 __device__ __noinline__ void plain_rows(const Job j) {
-    constexpr int V = D / 32, R = 4, C = 4;
+    constexpr int V = D / 32, R = 4, C = 8;
     constexpr bool kPair = Plan<D, USE>::kPair;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, mine_q = lane / C, mine_k = lane % C;
     for (int r0 = j.row0 + warp * R; r0 < min(j.row0 + kRows, j.rows); r0 += kThreads / 32 * R) {
-        float a1[R][V], a2[R][V], acc[R][V], m[R], l[R];
+        float a1[R][V], a2[R][V], acc[R][V], m = -INFINITY, l = 0.f;     // m, l: of row mine_q
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int r = min(r0 + q, j.rows - 1);
-            m[q] = -INFINITY; l[q] = 0.f;
 #pragma unroll
             for (int i = 0; i < V; ++i) {
                 const int d = lane + 32 * i;
@@ -173,8 +189,10 @@ __device__ __noinline__ void plain_rows(const Job j) {
                 }
             }
         }
+        const int row = r0 + mine_q;
+#pragma unroll 1
         for (int c0 = j.col0; c0 < j.cols; c0 += C) {
-            float s[R][C], y[R][C], b1[C][V], b2[C][V];
+            float b1[C][V], b2[C][V];
 #pragma unroll
             for (int k = 0; k < C; ++k) {
                 const long long c = min(c0 + k, j.cols - 1);
@@ -184,58 +202,81 @@ __device__ __noinline__ void plain_rows(const Job j) {
                     b2[k][i] = j.b2[c * j.ld_b2 + lane + 32 * i];
                 }
             }
-#pragma unroll
-            for (int q = 0; q < R; ++q)
-#pragma unroll
-                for (int k = 0; k < C; ++k) {
-                    s[q][k] = y[q][k] = 0.f;
-#pragma unroll
-                    for (int i = 0; i < V; ++i) {
-                        s[q][k] = fmaf(a1[q][i], b1[k][i], s[q][k]);
-                        if (kPair) y[q][k] = fmaf(a2[q][i], b2[k][i], y[q][k]);
-                    }
-                }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
+            auto product = [&](const float (&a)[R][V], const float (&b)[C][V]) {
+                float v[R * C];
 #pragma unroll
                 for (int q = 0; q < R; ++q)
 #pragma unroll
                     for (int k = 0; k < C; ++k) {
-                        s[q][k] += __shfl_xor_sync(0xFFFFFFFFu, s[q][k], o);
-                        if (kPair) y[q][k] += __shfl_xor_sync(0xFFFFFFFFu, y[q][k], o);
+                        v[q * C + k] = 0.f;
+#pragma unroll
+                        for (int i = 0; i < V; ++i) v[q * C + k] = fmaf(a[q][i], b[k][i], v[q * C + k]);
                     }
+                return sum_across(v);
+            };
+            const float s = product(a1, b1), y = kPair ? product(a2, b2) : 0.f;
+            const int col = c0 + mine_k, at = USE == kDq ? row : col;
+            const bool seen = row < j.rows && visible<USE>(j, row, col);
+            float w = 0.f;
+            if constexpr (USE == kForward) {
+                float top = seen ? s * j.scale : -INFINITY;
+                const float x = top;
 #pragma unroll
-            for (int q = 0; q < R; ++q)
+                for (int o = C / 2; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+                top = fmaxf(top, m);
+                const float ref = top == -INFINITY ? 0.f : top, alpha = expf(m - ref);
+                if (seen) w = expf(x - ref);
+                float sum = w;
 #pragma unroll
-                for (int k = 0; k < C; ++k) {
-                    const int r = r0 + q, c = c0 + k;
-                    if (r >= j.rows || !visible<USE>(j, r, c)) continue;
-                    const int at = USE == kDq ? r : c;
-                    float w;
-                    if constexpr (USE == kForward) {
-                        const float x = s[q][k] * j.scale, top = fmaxf(m[q], x), ref = top == -INFINITY ? 0.f : top, alpha = expf(m[q] - ref);
-                        w = expf(x - ref);
-                        l[q] = l[q] * alpha + w;
-                        m[q] = top;
+                for (int o = C / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+                l = fmaf(l, alpha, sum);
+                m = top;
 #pragma unroll
-                        for (int i = 0; i < V; ++i) acc[q][i] *= alpha;
-                    } else {
-                        w = expf(s[q][k] * j.scale - j.lse[at]);
-                        if (kPair) w *= y[q][k] - __ldcg(j.delta + at);
-                    }
+                for (int q = 0; q < R; ++q) {
+                    const float f = __shfl_sync(0xFFFFFFFFu, alpha, q * C);
 #pragma unroll
-                    for (int i = 0; i < V; ++i) acc[q][i] = fmaf(w, kPair ? b1[k][i] : b2[k][i], acc[q][i]);
+                    for (int i = 0; i < V; ++i) acc[q][i] *= f;
                 }
+            } else if (seen) {
+                w = expf(s * j.scale - j.lse[at]);
+                if (kPair) w *= y - __ldcg(j.delta + at);
+            }
+            const unsigned all = __ballot_sync(0xFFFFFFFFu, seen);
+            if (all == ~0u) {
+#pragma unroll
+                for (int q = 0; q < R; ++q)
+#pragma unroll
+                    for (int k = 0; k < C; ++k) {
+                        const float f = __shfl_sync(0xFFFFFFFFu, w, q * C + k);
+#pragma unroll
+                        for (int i = 0; i < V; ++i) acc[q][i] = fmaf(f, kPair ? b1[k][i] : b2[k][i], acc[q][i]);
+                    }
+            } else {                                                     // (a weight of 0 times an infinity would be seen)
+#pragma unroll 1
+                for (int k = 0; k < min(C, j.cols - c0); ++k) {
+                    const float* from = (kPair ? j.b1 + (c0 + k) * j.ld_b1 : j.b2 + (c0 + k) * j.ld_b2) + lane;
+                    float b[V];
+#pragma unroll
+                    for (int i = 0; i < V; ++i) b[i] = from[32 * i];
+#pragma unroll
+                    for (int q = 0; q < R; ++q) {
+                        const float f = __shfl_sync(0xFFFFFFFFu, w, q * C + k);
+                        if (all >> (q * C + k) & 1)
+#pragma unroll
+                            for (int i = 0; i < V; ++i) acc[q][i] = fmaf(f, b[i], acc[q][i]);
+                    }
+                }
+            }
         }
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int r = r0 + q;
-            if (r >= j.rows) break;
-            const float f = USE == kForward ? 1.0f / l[q] : USE == kDv ? 1.f : j.scale;
+            const float f = USE == kForward ? 1.0f / __shfl_sync(0xFFFFFFFFu, l, q * C) : USE == kDv ? 1.f : j.scale;
+            if (r < j.rows)
 #pragma unroll
-            for (int i = 0; i < V; ++i) j.out[r * j.ld_out + lane + 32 * i] = acc[q][i] * f;
-            if (USE == kForward && j.lse_out != nullptr && lane == 0) j.lse_out[r] = m[q] + logf(l[q]);
+                for (int i = 0; i < V; ++i) j.out[r * j.ld_out + lane + 32 * i] = acc[q][i] * f;
         }
+        if (USE == kForward && j.lse_out != nullptr && mine_k == 0 && row < j.rows) j.lse_out[row] = m + logf(l);
     }
 }
 
