@@ -46,6 +46,64 @@ def test_edges_of_the_tiles(cuda, D, N, causal):
         assert _off(x, want) <= BOUND
 
 
+def _rows(kind, g, D, cuda):
+    """q, k, v, dO whose sums differ from those of standard normal rows, which the factors in the kernel are fitted to."""
+    import torch
+    r = [torch.randn(2, 4, 320, D, generator=g, device=cuda) for _ in range(4)]
+    if kind == "offset":
+        return [x + 1 for x in r]
+    if kind == "positive":
+        return [x.abs() for x in r]
+    if kind == "whole":                              # sums that lose nothing, scores to 40 and more
+        return [x.mul(f).round() for x, f in zip(r, (2, 2, 4, 4))]
+    if kind == "large":                              # scores to 100
+        return [x * f for x, f in zip(r, (4, 4, 1, 1))]
+    half = [x[..., :D // 2] for x in r[:2]]          # scores of two sums that cancel to a hundredth
+    return [torch.cat([half[0] * 30, half[0] * 30 + 0.1 * r[0][..., D // 2:]], -1), torch.cat([half[1], -half[1]], -1), *r[2:]]
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("kind", ["offset", "positive", "whole", "large", "cancelling"])
+def test_rows_of_other_distributions(cuda, D, kind):
+    """No further from 64 bits than the CUDA cores (which a call without the whole workspace takes): at most a quarter more, what two runs of such
+    rows differ by, and one rounding of a score, the factor that is given back where nothing was lost."""
+    import torch
+    from vesper_b200 import capi
+    q, k, v, do = _rows(kind, torch.Generator(device=cuda).manual_seed(D), D, cuda)
+    want = _reference(q, k, v, do, 0, True)
+    off = []
+    for whole in (True, False):
+        o, lse = torch.empty_like(q), torch.empty(2, 4, 320, device=cuda)
+        a = capi.prefill_args(q, k, v, o, lse, scale=D ** -0.5, causal=True)
+        ws = torch.empty(capi.load().vb200_prefill_workspace_bytes(C.byref(a)), dtype=torch.uint8, device=cuda)
+        if whole:
+            a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        capi.check(capi.load().vb200_prefill_fwd(C.byref(a)))
+        got = (o, lse) + tuple(_backward(do, q, k, v, o, lse, whole))
+        off.append([_off(x, w) for x, w in zip(got, want)])
+    for tensor, cuda_cores in zip(*off):
+        assert tensor <= 1.25 * cuda_cores + 2 ** -23
+
+
+def _backward(do, q, k, v, o, lse, whole):
+    """vb200_attention_bwd with its whole workspace, or with a float per row."""
+    import torch
+    from vesper_b200 import capi
+    B, H, N, D = q.shape
+    a = capi.AttnBwdArgs()
+    a.struct_size, a.device, a.stream, a.dtype = C.sizeof(capi.AttnBwdArgs), 0, capi._stream_ptr(None), capi.dtype_code(q)
+    a.B, a.H, a.N, a.D, a.causal, a.scale = B, H, N, D, 1, D ** -0.5
+    out = [torch.empty_like(q) for _ in range(3)]
+    need = capi.load().vb200_attention_bwd_workspace_bytes(C.byref(a)) if whole else 4 * B * H * N
+    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+    for name, t in zip(("d_out", "q", "k", "v", "out", "lse", "dq", "dk", "dv", "workspace"), (do, q, k, v, o, lse, *out, ws)):
+        setattr(a, name, t.data_ptr())
+    a.workspace_bytes = need
+    capi.check(capi.load().vb200_attention_bwd(C.byref(a)))
+    torch.cuda.synchronize()
+    return out
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("T,start,rotate", [(1, 64, False), (5, 200, True), (129, 62, False), (130, 0, True)])
 def test_portions_of_a_prompt(cuda, D, T, start, rotate):

@@ -25,7 +25,7 @@
 //
 // The tensor cores add with truncation, so no sum stays with them for long: a block's six products are added smallest first, and
 // each block's result is added to the sum in registers, rounded to nearest.  What the last eight (or four) additions of a score lose
-// on average is given back with its factor (kScoreLoss, kGradLoss).  A1 (and of A2 what fits) is read from TMEM: an
+// on average is given back by factors (Loss).  A1 (and of A2 what fits) is read from TMEM: an
 // operand of 64 columns from shared memory would make the product wait for the 128 rows of A.
 //
 // TMEM columns: A1 [3 D/2], A2 [terms in TMEM], per slot X [64] (and Y [64]) overwritten by the terms of W [96], the block sum [D].
@@ -44,9 +44,19 @@ constexpr int kLoadWarp = 8, kIssueWarp = 9;
 constexpr int kThreads = (kIssueWarp + 1) * 32;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kLeast = 0x1p-100f;
-// Mean relative loss of X per 64 columns of the head dimension, and of Y, by the truncating additions: the slopes of O, dQ and dK against 64 bits
-// (64-2048 normal rows) are -6e-8..-3e-7 without these factors and within 1e-7 with them.  (Y's is one step of a float above 1.)
-constexpr float kScoreLoss = 1.05e-7f, kGradLoss = 0x1p-23f;
+// What the truncating additions lose on average, given back by factors of the scores (X), of dO V^T and V dO^T (Y), and of the results.  Fitted to the
+// slopes of O, LSE, dQ, dK and dV against 64 bits over 64 to 2048 normal rows, -3e-7 .. -3e-8 without them and within 4e-8 with them; Y's also to rows with
+// a common offset, whose Y - Di cancels.  X's stands in the second factor of the exponent (forward) and in the exponent itself (backward), not in
+// the scale, where it would be a whole step of a float and the backward's X another one than the forward's.  Error against that of the
+// CUDA cores: normal rows 0.4-0.8, other distributions below 1.1 (test_rows_of_other_distributions in test_f32_tensor_gpu.py; with one step of a float
+// as the factor of Y and of the scale up to 2.6).  Sums that lose nothing (small whole numbers) get up to 1.5e-7 of a score too much.
+template <int D>
+struct Loss {
+    static constexpr float kLog2eUp = kLog2e + (D == 64 ? 1 : 2) * 0x1p-23f;                           // log2 e, times 1 + kScore
+    static constexpr float kScore = static_cast<float>(kLog2eUp / 1.4426950408889634 - 1.0);           // 6.9e-8, 1.5e-7
+    static constexpr float kGrad = D == 64 ? 4e-8f : 9e-8f;
+    static constexpr float kOut = 2.5e-8f, kGradOut = 7e-8f;
+};
 
 enum Use { kForward, kDv, kDq, kDk };
 
@@ -127,14 +137,10 @@ __device__ __forceinline__ float4 load4(const float* p, bool valid) {
 __device__ __forceinline__ uint32_t doubled(float x) { return 2 * __float_as_uint(x) - 1; }
 __device__ __forceinline__ uint32_t least_of(uint32_t least, float4 x) { return min(least, min(min(doubled(x.x), doubled(x.y)), min(doubled(x.z), doubled(x.w)))); }
 __device__ __forceinline__ bool too_small(uint32_t least) { return least < doubled(kLeast); }
-// e^x: the exponent x log2 e is rounded once, an error of |x| 2^-24 of the result at most, below that of the scores
+// e^(x (1 + kScore)), x finite, with the rounding of the exponent x log2 e made up for
+template <int D>
 __device__ __forceinline__ float2 exp_pair(float2 x) {
-    const float2 t = __fmul2_rn(x, make_float2(kLog2e, kLog2e));
-    return make_float2(fast_exp2(t.x), fast_exp2(t.y));
-}
-// the same with the exponent's rounding made up for; x finite
-__device__ __forceinline__ float2 exp_pair_exact(float2 x) {
-    const float2 log2e = make_float2(kLog2e, kLog2e), t = __fmul2_rn(x, log2e), lost = __ffma2_rn(x, log2e, make_float2(-t.x, -t.y));
+    const float2 t = __fmul2_rn(x, make_float2(kLog2e, kLog2e)), lost = __ffma2_rn(x, make_float2(Loss<D>::kLog2eUp, Loss<D>::kLog2eUp), make_float2(-t.x, -t.y));
     const float2 y = make_float2(fast_exp2(t.x), fast_exp2(t.y));
     return __ffma2_rn(y, __fmul2_rn(lost, make_float2(kLn2, kLn2)), y);
 }
@@ -392,7 +398,7 @@ __device__ __forceinline__ void attend(const Job& j, unsigned char* tiles, Share
             if (row >= j.rows) hi = lo;
             if (j.row0 + kRows > j.rows) all = 0;
         }
-        const float scale = fmaf(j.scale, kScoreLoss * (D / 64), j.scale);
+        const float2 scale = make_float2(j.scale, j.scale), lost = make_float2(j.scale * Loss<D>::kScore * kLog2e, j.scale * Loss<D>::kScore * kLog2e);
         float2 chk = make_float2(0.f, 0.f);
         bool ok = true;
         for (int blk = 0; blk < n; ++blk) {
@@ -419,7 +425,7 @@ __device__ __forceinline__ void attend(const Job& j, unsigned char* tiles, Share
                 float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
                 for (int i = 0; i < kCols; i += 2) {
-                    const float2 x = __fmul2_rn(make_float2(s[i], s[i + 1]), make_float2(scale, scale));
+                    const float2 x = __fmul2_rn(make_float2(s[i], s[i + 1]), scale);
                     s[i] = x.x; s[i + 1] = x.y;
                 }
                 if (edge)
@@ -429,10 +435,11 @@ __device__ __forceinline__ void attend(const Job& j, unsigned char* tiles, Share
 #pragma unroll
                 for (int i = 0; i < kCols; i += 2) mx[(i >> 1) & 3] = fmax3(mx[(i >> 1) & 3], s[i], s[i + 1]);
                 const float top = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
-                const float alpha = expf(m - top);                       // the first block holds a visible column: top is finite, or the rows are computed again
+                // (the first block holds a visible column: top is finite, or the rows are computed again)
+                const float alpha = expf(m - top) * fmaf(fmaxf(m - top, -200.f), Loss<D>::kScore, 1.f);
 #pragma unroll
                 for (int i = 0; i < kCols; i += 2) {
-                    const float2 w = exp_pair_exact(__fadd2_rn(make_float2(s[i], s[i + 1]), make_float2(-top, -top)));
+                    const float2 x = __fadd2_rn(make_float2(s[i], s[i + 1]), make_float2(-top, -top)), w = exp_pair<D>(x);
                     s[i] = w.x; s[i + 1] = w.y;
                 }
                 if (edge)                                                // the weight itself: a score far enough below any top is not a number of 24 bits
@@ -451,10 +458,11 @@ __device__ __forceinline__ void attend(const Job& j, unsigned char* tiles, Share
                 for (int i = 0; i < kCols; i += 4) {
                     float4 at = make_float4(lse, lse, lse, lse);
                     if (!by_row) at = *reinterpret_cast<const float4*>(&of_queries[0][i]);
-                    const float2 s2 = make_float2(scale, scale);
-                    const float2 w0 = exp_pair(__ffma2_rn(make_float2(s[i], s[i + 1]), s2, make_float2(-at.x, -at.y)));
-                    const float2 w1 = exp_pair(__ffma2_rn(make_float2(s[i + 2], s[i + 3]), s2, make_float2(-at.z, -at.w)));
-                    s[i] = w0.x; s[i + 1] = w0.y; s[i + 2] = w1.x; s[i + 3] = w1.y;
+                    const float2 s0 = make_float2(s[i], s[i + 1]), s1 = make_float2(s[i + 2], s[i + 3]);
+                    const float2 log2e = make_float2(kLog2e, kLog2e);
+                    const float2 t0 = __ffma2_rn(__ffma2_rn(s0, scale, make_float2(-at.x, -at.y)), log2e, __fmul2_rn(s0, lost));
+                    const float2 t1 = __ffma2_rn(__ffma2_rn(s1, scale, make_float2(-at.z, -at.w)), log2e, __fmul2_rn(s1, lost));
+                    s[i] = fast_exp2(t0.x); s[i + 1] = fast_exp2(t0.y); s[i + 2] = fast_exp2(t1.x); s[i + 3] = fast_exp2(t1.y);
                 }
                 if (edge)
 #pragma unroll
@@ -477,10 +485,11 @@ __device__ __forceinline__ void attend(const Job& j, unsigned char* tiles, Share
                     for (int i = 0; i < 16; i += 4) {
                         float4 at = make_float4(delta, delta, delta, delta);
                         if (!by_row) at = *reinterpret_cast<const float4*>(&of_queries[1][h * 16 + i]);
-                        w[i] *= fmaf(__uint_as_float(y[i]), 1.f + kGradLoss, -at.x);
-                        w[i + 1] *= fmaf(__uint_as_float(y[i + 1]), 1.f + kGradLoss, -at.y);
-                        w[i + 2] *= fmaf(__uint_as_float(y[i + 2]), 1.f + kGradLoss, -at.z);
-                        w[i + 3] *= fmaf(__uint_as_float(y[i + 3]), 1.f + kGradLoss, -at.w);
+                        const float2 y0 = make_float2(__uint_as_float(y[i]), __uint_as_float(y[i + 1])), y1 = make_float2(__uint_as_float(y[i + 2]), __uint_as_float(y[i + 3]));
+                        const float2 lost = make_float2(Loss<D>::kGrad, Loss<D>::kGrad);
+                        const float2 w0 = __fmul2_rn(make_float2(w[i], w[i + 1]), __ffma2_rn(y0, lost, __fadd2_rn(y0, make_float2(-at.x, -at.y))));
+                        const float2 w1 = __fmul2_rn(make_float2(w[i + 2], w[i + 3]), __ffma2_rn(y1, lost, __fadd2_rn(y1, make_float2(-at.z, -at.w))));
+                        w[i] = w0.x; w[i + 1] = w0.y; w[i + 2] = w1.x; w[i + 3] = w1.y;
                     }
                 }
                 uint32_t t0[8], t1[8], t2[8];
@@ -498,7 +507,10 @@ __device__ __forceinline__ void attend(const Job& j, unsigned char* tiles, Share
         if (not_zero(chk) || (USE == kForward && !(l < INFINITY))) sh.outside = 1;
         if (USE == kForward) sh.total[r] = l;
         roles_end();
-        if (USE == kForward && !sh.outside && j.lse_out != nullptr && row < j.rows) j.lse_out[row] = m + logf(l);
+        if (USE == kForward && !sh.outside && j.lse_out != nullptr && row < j.rows) {
+            const float d = m * Loss<D>::kScore;                         // within the logarithm while that is small: one rounding less
+            j.lse_out[row] = m + (fabsf(d) < 1e-4f ? logf(fmaf(l, d, l)) : d + logf(l));
+        }
     } else if (warp < kLoadWarp) {
         // ---- the sum ----
         const int r = tid & 127;
@@ -537,7 +549,9 @@ __device__ __forceinline__ void attend(const Job& j, unsigned char* tiles, Share
             const uint32_t own = smem_u32(tiles) + (warp - 4) * (32 * D * 4);
 #pragma unroll
             for (int i = 0; i < D / 4; ++i) {
-                const float v[4] = {acc[2 * i].x * f, acc[2 * i].y * f, acc[2 * i + 1].x * f, acc[2 * i + 1].y * f};
+                float v[4] = {acc[2 * i].x * f, acc[2 * i].y * f, acc[2 * i + 1].x * f, acc[2 * i + 1].y * f};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = fmaf(v[e], USE == kForward ? Loss<D>::kOut : Loss<D>::kGradOut, v[e]);
                 store_shared(own + lane * (D * 4) + ((i ^ (lane & 7)) << 4), reinterpret_cast<const uint32_t*>(v));
             }
             __syncwarp();
