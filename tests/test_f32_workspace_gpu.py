@@ -44,3 +44,29 @@ def test_backward_with_a_float_per_row(cuda, lib, D, N, causal):
     assert (rows[B * H * N:] == 7.0).all()
     for x, w in zip(got, want):
         assert _off(x, w) <= BOUND
+
+
+def test_a_caller_may_decline_the_terms(cuda, lib):
+    """A smaller workspace that a call can do with is the one it uses: nothing is allocated in its place."""
+    import torch
+    from vesper_b200 import capi
+    B, H, N, D = 2, 16, 1000, 128
+    g = torch.Generator(device=cuda).manual_seed(1)
+    q, k, v, do = (torch.randn(B, H, N, D, generator=g, device=cuda) for _ in range(4))
+    o, lse = torch.empty_like(q), torch.empty(B, H, N, device=cuda)
+    none, rows = torch.empty(0, dtype=torch.uint8, device=cuda), torch.empty(B * H * N, device=cuda)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    assert capi.prefill(q, k, v, o, lse, scale=D ** -0.5, workspace=none) is none
+    assert lib.vb200_last_prefill_kernel() == b"prefill_f32_kernel"
+    got = capi.attention_bwd(do, q, k, v, o, lse, scale=D ** -0.5, workspace=rows)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before <= 3 * q.numel() * 4 + (1 << 20)
+    whole = capi.prefill(q, k, v, o.clone(), lse.clone(), scale=D ** -0.5)
+    assert lib.vb200_last_prefill_kernel() == b"attention_f32_forward_kernel" and whole.numel() > 4 * q.numel()
+    for x, w in zip((o, lse, *got), _reference(q, k, v, do, 0, True)):
+        assert _off(x, w) <= 2 * BOUND
+    # a workspace that the call cannot do with is replaced, as it always was
+    kc, vc = (torch.zeros(B, H, N, D, device=cuda) for _ in range(2))
+    assert capi.prefill(q, k, v, o, lse, scale=D ** -0.5, theta=1e4, k_cache=kc, v_cache=vc, workspace=none) is not none

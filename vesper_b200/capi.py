@@ -106,6 +106,9 @@ EPI_BF16, EPI_F32, EPI_ADD_F32, EPI_SWIGLU, EPI_RELU2, EPI_REGLU = 0, 1, 2, 3, 4
 _lib = None
 
 
+ERR_WORKSPACE = -4               # VB200_ERR_WORKSPACE
+
+
 class Vb200Error(RuntimeError):
     def __init__(self, status, text):
         super().__init__(text)
@@ -247,15 +250,18 @@ def prefill_args(q, k, v, o, lse=None, *, scale, causal=True, start_pos=0, theta
 
 def prefill(q, k, v, o, lse=None, *, scale, causal=True, start_pos=0, theta=None,
             k_cache=None, v_cache=None, workspace=None, stream=None, cache_read_only=False):
-    """vb200_prefill_fwd on torch CUDA tensors.  Allocates a workspace with torch when none is given."""
+    """vb200_prefill_fwd on torch CUDA tensors.  Allocates a workspace with torch when none is given, or one that the call refuses: fp32 takes less
+    than vb200_prefill_workspace_bytes (without rotation an empty tensor) and then runs on the CUDA cores."""
     L = load()
     a = prefill_args(q, k, v, o, lse, scale=scale, causal=causal, start_pos=start_pos, theta=theta,
                      k_cache=k_cache, v_cache=v_cache, workspace=workspace, stream=stream, cache_read_only=cache_read_only)
     need = L.vb200_prefill_workspace_bytes(C.byref(a))
-    if need > a.workspace_bytes:
+    rc = ERR_WORKSPACE if need > a.workspace_bytes and workspace is None else L.vb200_prefill_fwd(C.byref(a))
+    if rc == ERR_WORKSPACE:
         workspace = _workspace(need, q.device, stream)
         a.workspace, a.workspace_bytes = _ptr(workspace), need
-    check(L.vb200_prefill_fwd(C.byref(a)))
+        rc = L.vb200_prefill_fwd(C.byref(a))
+    check(rc)
     return workspace
 
 
@@ -325,8 +331,9 @@ def profile_read():
     return ms.value, n.value
 
 
-def attention_bwd(d_out, q, k, v, out, lse, *, scale, causal=True, stream=None):
-    """fp32 contiguous [B,H,N,D] tensors; returns (dq, dk, dv)."""
+def attention_bwd(d_out, q, k, v, out, lse, *, scale, causal=True, stream=None, workspace=None):
+    """fp32 contiguous [B,H,N,D] tensors; returns (dq, dk, dv).  A workspace smaller than vb200_attention_bwd_workspace_bytes, B*H*N floats at least,
+    runs on the CUDA cores."""
     import torch
     B, H, N, D = q.shape
     a = AttnBwdArgs()
@@ -342,9 +349,9 @@ def attention_bwd(d_out, q, k, v, out, lse, *, scale, causal=True, stream=None):
     for name, t in (("d_out", d_out), ("q", q), ("k", k), ("v", v), ("out", out), ("lse", lse), ("dq", dq), ("dk", dk), ("dv", dv)):
         assert t.is_contiguous()
         setattr(a, name, _ptr(t))
-    need = load().vb200_attention_bwd_workspace_bytes(C.byref(a))
-    ws = _workspace(need, q.device, stream)
-    a.workspace, a.workspace_bytes = _ptr(ws), need
+    if workspace is None:
+        workspace = _workspace(load().vb200_attention_bwd_workspace_bytes(C.byref(a)), q.device, stream)
+    a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel() * workspace.element_size()
     check(load().vb200_attention_bwd(C.byref(a)))
     return dq, dk, dv
 
