@@ -15,7 +15,9 @@
 namespace fake {
 enum State { kIdle, kBusy, kCapturing };
 std::map<cudaStream_t, State> streams;
-std::map<void*, size_t> blocks;
+std::map<void*, size_t> blocks;         // what the driver has given out, at most `memory` bytes
+size_t memory = size_t{180} << 30;
+size_t given() { size_t n = 0; for (auto& b : blocks) n += b.second; return n; }
 cudaError_t last = cudaSuccess;
 int32_t status = 0;             // the device status word
 char detail[64];
@@ -27,6 +29,7 @@ cudaError_t cudaGetLastError() { cudaError_t e = fake::last; fake::last = cudaSu
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
     static uintptr_t next = 1 << 20;
+    if (fake::given() + n > fake::memory) return fake::last = cudaErrorMemoryAllocation;
     *p = reinterpret_cast<void*>(next);
     next += 1 << 20;
     fake::blocks[*p] = n;

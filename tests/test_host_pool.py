@@ -8,7 +8,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-@pytest.mark.parametrize("program", ["test_block_pool", "test_expired_wait"])
+@pytest.mark.parametrize("program", ["test_block_pool", "test_pool_bounds", "test_expired_wait"])
 def test_against_a_fake_runtime(program):
     from vesper_b200.build import _nvcc
     exe = os.path.join(ROOT, "tests", "cpp", "_build", program)

@@ -772,11 +772,11 @@ struct SplitLayout {
         marks_bytes = (static_cast<size_t>(heads) * blocks * sizeof(int) + 255) / 256 * 256;
     }
 };
-// Heads whose terms are in the workspace at a time: as many as one gigabyte holds, and at least one.
+// Heads whose terms and marks are in the workspace at a time: as many as one gigabyte holds, and at least one.
 constexpr size_t kWorkspaceGoal = size_t{1} << 30;
 int heads_at_a_time(int rows, int D, int heads, int tensors) {
     const SplitLayout one(rows, D, 1);
-    size_t most = kWorkspaceGoal / (tensors * one.terms_bytes);
+    size_t most = (kWorkspaceGoal - tensors * 256) / (tensors * (one.terms_bytes + one.blocks * sizeof(int)));      // (marks are rounded up to 256 bytes)
     if (most > 65535) most = 65535;            // the second dimension of a grid
     return most < 1 ? 1 : most < static_cast<size_t>(heads) ? static_cast<int>(most) : heads;
 }

@@ -72,7 +72,7 @@ private:
 };
 
 // Reference-counted buffer; CUDA buffers come from a small caching allocator
-// (power-of-two bins, as src/core/allocator.cpp:171-221 does).  A buffer may be let go of while
+// (bins by size, as src/core/allocator.cpp:171-221 has), which gives back what is free beyond 8 GiB.  A buffer may be let go of while
 // the stream that was current when it was created, or the one current now, still has work on it: another stream
 // gets it only afterwards.  (Work on a third stream has to be waited for first.)
 class Storage {

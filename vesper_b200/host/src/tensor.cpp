@@ -38,16 +38,18 @@ bool idle(const std::shared_ptr<void>& s) {
 }
 
 // Caching allocator: freed blocks are kept per (device, rounded size) and
-// handed out again; nothing is returned to the driver before process exit
-// (src/core/allocator.cpp:205-221 has the same policy).  A block goes to work of the streams that it was used on, or of the
+// handed out again (src/core/allocator.cpp:205-221 keeps them all; here what is free stays below kMostFree per device, and goes back
+// to the driver when that has no more).  A block goes to work of the streams that it was used on, or of the
 // default stream, at once (their order is the stream's), to other streams when those are idle.
 class CachingAllocator {
 public:
     static CachingAllocator& get() { static CachingAllocator* a = new CachingAllocator(); return *a; }
+    // powers of two; large blocks in steps of an eighth of one, so that a workspace of a gigabyte and a little does not hold two
     static size_t round(size_t n) {
         size_t r = 512;
         while (r < n) r <<= 1;
-        return r;
+        const size_t step = r / 16;
+        return r <= kLarge ? r : (n + step - 1) / step * step;
     }
     // `current`: the stream that asks; `streams`: those whose work may still use the block
     void* alloc(size_t rounded, int dev, const std::shared_ptr<void>& current, Streams& streams) {
@@ -62,26 +64,54 @@ public:
                 void* p = b.p;
                 streams = std::move(b.streams);
                 bin.erase(bin.begin() + static_cast<std::ptrdiff_t>(i));
+                free_bytes_[dev] -= rounded;
                 return p;
             }
         }
         void* p = nullptr;
-        cuda_check(cudaMalloc(&p, rounded), "cudaMalloc");
+        cudaError_t e = cudaMalloc(&p, rounded);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            std::lock_guard<std::mutex> lock(mu_);
+            give_back(dev, 0);
+            e = cudaMalloc(&p, rounded);
+        }
+        cuda_check(e, "cudaMalloc");
         return p;
     }
     void release(void* p, size_t rounded, int dev, Streams streams) {
         std::lock_guard<std::mutex> lock(mu_);
         free_[{dev, rounded}].push_back(Block{p, std::move(streams)});
+        free_bytes_[dev] += rounded;
+        if (free_bytes_[dev] > kMostFree) give_back(dev, kMostFree);
     }
 
 private:
+    static constexpr size_t kLarge = size_t{64} << 20, kMostFree = size_t{8} << 30;
     struct Block { void* p; Streams streams; };
+    // Idle blocks, the largest first, until at most `keep` bytes are free.  Not while this thread captures a graph (cudaFree would end that).
+    void give_back(int dev, size_t keep) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        const auto current = Stream::current(Device::CUDA).owner();
+        if (current && (cudaStreamIsCapturing(static_cast<cudaStream_t>(current.get()), &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)) return;
+        for (auto it = free_.rbegin(); it != free_.rend() && free_bytes_[dev] > keep; ++it) {
+            if (it->first.first != dev) continue;
+            auto& bin = it->second;
+            for (size_t i = bin.size(); i-- > 0 && free_bytes_[dev] > keep;) {
+                drop_idle(bin[i].streams, nullptr);
+                if (!bin[i].streams.empty() || cudaFree(bin[i].p) != cudaSuccess) continue;
+                bin.erase(bin.begin() + static_cast<std::ptrdiff_t>(i));
+                free_bytes_[dev] -= it->first.second;
+            }
+        }
+    }
     static void drop_idle(Streams& list, const std::shared_ptr<void>& except) {
         for (size_t i = list.size(); i-- > 0;)
             if (list[i] != except && idle(list[i])) list.erase(list.begin() + static_cast<std::ptrdiff_t>(i));
     }
     std::mutex mu_;
     std::map<std::pair<int, size_t>, std::vector<Block>> free_;
+    std::map<int, size_t> free_bytes_;          // per device
 };
 
 // A word of page-locked memory per thread, into which the device status word is copied along with a synchronisation.
