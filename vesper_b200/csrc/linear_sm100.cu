@@ -894,14 +894,17 @@ int launch_pair(cudaStream_t s, const LinearParams& p, int sms) {
     PairMaps maps;
     if (int rc = make_map_2d(&maps.a, p.x, p.M, p.K, p.ldx, kTileA)) return rc;
     if (int rc = make_map_2d(&maps.b, p.w, p.N, p.K, p.ldw, BN / 2)) return rc;
-    if (int rc = make_map_2d(&maps.b_half, p.w, p.N, p.K, p.ldw, BN / 4)) return rc;
     auto kernel = linear_pair_kernel<BN, EPI>;
     static thread_local bool configured[64] = {};
     if (int rc = set_smem_once(kernel, C::kSmemBytes, configured)) return rc;
     const int tiles = ((p.M + 2 * kTileA - 1) / (2 * kTileA)) * ((p.N + BN - 1) / BN), pairs = sms / 2, last = tiles % pairs;
-    // A last round that at most half of the pairs have a tile in is dealt out in halves of tiles (3003 rows, 96 tiles on 74 pairs: 2048 x 8448 94.6 -> 86.3 us,
-    // 2048 x 5632 66.3 -> 58.2, 2048 x 2048 35.1 -> 29.2; a half takes two thirds of a tile's time).
+    // A last round that at most half of the pairs have a tile in is dealt out in halves of tiles; a half takes two thirds of a tile's time.  Whole tiles / halves,
+    // weights from HBM: 3003 rows 2048 x 5632 60.2-62.1 / 53.3-58.4 us, 2048 x 2048 24-27 / 20.8-24.9, 11264 x 2048 94.4 / 91.6; 2100 rows 3072 x 2048
+    // 24.2 / 21.9, 11264 x 2048 72.8 / 71.3; 1001 rows 11264 x 2048 36.8 / 35.7; 3500 rows 3072 x 2048 42.4-44.9 / 40.0-43.7, 11264 x 2048 107-116 / 105-114.
     const int whole = BN == 256 && tiles > pairs && 2 * last <= pairs ? tiles - last : tiles;
+    maps.b_half = maps.b;                             // (the kernel reads it for halves only)
+    if (whole < tiles)
+        if (int rc = make_map_2d(&maps.b_half, p.w, p.N, p.K, p.ldw, BN / 4)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(2 * (tiles < pairs ? tiles : pairs)));
     cfg.blockDim = dim3(kPairThreads);
@@ -921,9 +924,10 @@ int launch_pair(cudaStream_t s, const LinearParams& p, int sms) {
     return VB200_OK;
 }
 
-// More than 64 rows.  Pairs of CTAs with tiles of 256 columns; of 128 columns while one round over the SM pairs takes them all (768 rows, 2048 x 2048:
-// 13.6 us, 2048 x 5632 25.3; 256 columns 21.3 and 37.5; with more rounds the wider tile is up to 1.6 times faster); single CTAs where the rows
-// of a pair's last tile would be mostly padding and cost rounds (300 rows, 11264 x 2048: 25.1 us against 29.2).
+// More than 64 rows.  Pairs of CTAs with tiles of 256 columns; of 128 columns while one round over the SM pairs takes them all (768 rows, weights from
+// HBM, 128 / 256 columns: 2048 x 2048 13.0 / 15.4 us, 2048 x 5632 23.5 / 31.8; with more rounds the wider tile is faster: 3003 rows, 11264 x 2048 118 / 92);
+// single CTAs where the rows of a pair's last tile would be mostly padding and cost rounds (single / pairs: 300 rows, 11264 x 2048 17.9 / 22.7 us, 384 rows
+// 18.1 / 22.8, though the pairs' last round is one of halves; 256 rows, which fill them, 18.2 / 17.0; 3003 rows 104.6 / 92.5).
 template <int EPI>
 int launch_many_rows(cudaStream_t s, const LinearParams& p) {
     int sms = 0;
