@@ -107,6 +107,7 @@ typedef struct vb200_prefill_args {
 } vb200_prefill_args;
 
 size_t vb200_prefill_workspace_bytes(const vb200_prefill_args* a);
+size_t vb200_prefill_workspace_bytes_min(const vb200_prefill_args* a);      /* without the optional part */
 int vb200_prefill_fwd(const vb200_prefill_args* a);
 
 /* ---- decode ---------------------------------------------------------------
@@ -282,6 +283,7 @@ typedef struct vb200_attention_bwd_args {
     size_t workspace_bytes;
 } vb200_attention_bwd_args;
 size_t vb200_attention_bwd_workspace_bytes(const vb200_attention_bwd_args* a);
+size_t vb200_attention_bwd_workspace_bytes_min(const vb200_attention_bwd_args* a);   /* B*H*N floats */
 int vb200_attention_bwd(const vb200_attention_bwd_args* a);
 
 /* ---- cache append without attention ---------------------------------------
@@ -321,7 +323,7 @@ int vb200_abi_version(void);
 uint64_t vb200_launch_count(void);
 void vb200_reset_launch_count(void);
 /* Name of the attention kernel the calling thread's last vb200_prefill_fwd launched ("prefill_sm100_kernel",
- * "prefill_pair_kernel", "prefill_f32_kernel"; "" before the first call): which of the kernels a shape, a dtype or the
+ * "prefill_pair_kernel", "prefill_f32_kernel", "attention_f32_forward_kernel"; "" before the first call): which of the kernels a shape, a dtype or the
  * VB200_PREFILL_KERNEL switch selected, for reports and tests. */
 const char* vb200_last_prefill_kernel(void);
 /* Optional timing of the dominant kernel of each call (the attention kernel of

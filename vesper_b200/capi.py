@@ -50,9 +50,9 @@ class DecodeArgs(C.Structure):
 
 
 EXPORTS = [
-    "vb200_prefill_workspace_bytes", "vb200_prefill_fwd", "vb200_decode_workspace_bytes", "vb200_decode_workspace_bytes_max", "vb200_decode_fwd",
+    "vb200_prefill_workspace_bytes", "vb200_prefill_workspace_bytes_min", "vb200_prefill_fwd", "vb200_decode_workspace_bytes", "vb200_decode_workspace_bytes_max", "vb200_decode_fwd",
     "vb200_decode_fwd_static", "vb200_exchange_buffer_bytes", "vb200_exchange_combine", "vb200_decode_exchange_fwd",
-    "vb200_attention_bwd_workspace_bytes", "vb200_attention_bwd",
+    "vb200_attention_bwd_workspace_bytes", "vb200_attention_bwd_workspace_bytes_min", "vb200_attention_bwd",
     "vb200_lse_combine", "vb200_kv_append", "vb200_apply_rope", "vb200_repeat_kv", "vb200_rope_inv_freq",
     "vb200_strerror", "vb200_last_error_detail", "vb200_abi_version", "vb200_launch_count",
     "vb200_reset_launch_count", "vb200_last_prefill_kernel", "vb200_check_kernel_status",
@@ -124,8 +124,8 @@ def load():
     if not os.path.exists(path):
         raise FileNotFoundError(f"{path} is missing: run `python -m vesper_b200.build` (needs nvcc)")
     L = C.CDLL(path)
-    L.vb200_prefill_workspace_bytes.argtypes = [C.POINTER(PrefillArgs)]
-    L.vb200_prefill_workspace_bytes.restype = C.c_size_t
+    for f in (L.vb200_prefill_workspace_bytes, L.vb200_prefill_workspace_bytes_min):
+        f.argtypes, f.restype = [C.POINTER(PrefillArgs)], C.c_size_t
     L.vb200_prefill_fwd.argtypes = [C.POINTER(PrefillArgs)]
     L.vb200_decode_workspace_bytes.argtypes = [C.POINTER(DecodeArgs)]
     L.vb200_decode_workspace_bytes.restype = C.c_size_t
@@ -150,8 +150,8 @@ def load():
     L.vb200_kernel_status_of.argtypes = [C.c_int32]
     L.vb200_profile_enable.argtypes = [C.c_int]
     L.vb200_profile_read.argtypes = [C.POINTER(C.c_double), C.POINTER(C.c_uint64)]
-    L.vb200_attention_bwd_workspace_bytes.argtypes = [C.POINTER(AttnBwdArgs)]
-    L.vb200_attention_bwd_workspace_bytes.restype = C.c_size_t
+    for f in (L.vb200_attention_bwd_workspace_bytes, L.vb200_attention_bwd_workspace_bytes_min):
+        f.argtypes, f.restype = [C.POINTER(AttnBwdArgs)], C.c_size_t
     L.vb200_attention_bwd.argtypes = [C.POINTER(AttnBwdArgs)]
     L.vb200_exchange_buffer_bytes.argtypes = [C.c_int32, C.c_int64, C.c_int32]
     L.vb200_exchange_buffer_bytes.restype = C.c_size_t
@@ -209,12 +209,18 @@ def _stream_ptr(stream):
     return C.c_void_p(s.cuda_stream)
 
 
-def _workspace(nbytes, device, stream):
-    """Bytes that belong to `stream` (None: the current one): torch gives their memory to later work of that stream only."""
+def _workspace(nbytes, device, stream, least=None):
+    """Bytes that belong to `stream` (None: the current one): torch gives their memory to later work of that stream only.  `least` bytes where the device
+    has no room for all."""
     import contextlib
     import torch
     with torch.cuda.stream(stream) if isinstance(stream, torch.cuda.Stream) else contextlib.nullcontext():
-        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        try:
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        except torch.cuda.OutOfMemoryError:
+            if least is None or least >= nbytes:
+                raise
+        return torch.empty(least, dtype=torch.uint8, device=device)
 
 
 def _ptr(t):
@@ -258,8 +264,8 @@ def prefill(q, k, v, o, lse=None, *, scale, causal=True, start_pos=0, theta=None
     need = L.vb200_prefill_workspace_bytes(C.byref(a))
     rc = ERR_WORKSPACE if need > a.workspace_bytes and workspace is None else L.vb200_prefill_fwd(C.byref(a))
     if rc == ERR_WORKSPACE:
-        workspace = _workspace(need, q.device, stream)
-        a.workspace, a.workspace_bytes = _ptr(workspace), need
+        workspace = _workspace(need, q.device, stream, L.vb200_prefill_workspace_bytes_min(C.byref(a)))
+        a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel()
         rc = L.vb200_prefill_fwd(C.byref(a))
     check(rc)
     return workspace
@@ -350,7 +356,8 @@ def attention_bwd(d_out, q, k, v, out, lse, *, scale, causal=True, stream=None, 
         assert t.is_contiguous()
         setattr(a, name, _ptr(t))
     if workspace is None:
-        workspace = _workspace(load().vb200_attention_bwd_workspace_bytes(C.byref(a)), q.device, stream)
+        need, least = load().vb200_attention_bwd_workspace_bytes(C.byref(a)), load().vb200_attention_bwd_workspace_bytes_min(C.byref(a))
+        workspace = _workspace(need, q.device, stream, least)
     a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel() * workspace.element_size()
     check(load().vb200_attention_bwd(C.byref(a)))
     return dq, dk, dv

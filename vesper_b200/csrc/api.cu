@@ -332,6 +332,11 @@ size_t vb200_prefill_workspace_bytes(const vb200_prefill_args* a) {
     return pl.total + pl.split_bytes;
 }
 
+size_t vb200_prefill_workspace_bytes_min(const vb200_prefill_args* a) {
+    if (!a || a->struct_size != sizeof(vb200_prefill_args)) return 0;
+    return plan_prefill(a).total;
+}
+
 int vb200_prefill_fwd(const vb200_prefill_args* a) {
     if (int rc = validate_prefill(a)) return rc;
     PrefillPlan pl = plan_prefill(a);
@@ -567,6 +572,11 @@ size_t vb200_attention_bwd_workspace_bytes(const vb200_attention_bwd_args* a) {
     return bwd_delta_bytes(a) + (terms ? attention_bwd_f32_split_bytes(a->D, a->B * a->H, a->N) : 0);
 }
 
+size_t vb200_attention_bwd_workspace_bytes_min(const vb200_attention_bwd_args* a) {
+    if (!a || a->struct_size != sizeof(vb200_attention_bwd_args) || a->B <= 0 || a->H <= 0 || a->N <= 0) return 0;
+    return sizeof(float) * static_cast<size_t>(a->B) * a->H * a->N;
+}
+
 int vb200_attention_bwd(const vb200_attention_bwd_args* a) {
     if (!a || a->struct_size != sizeof(vb200_attention_bwd_args)) return set_detail(VB200_ERR_INVALID_ARG, "vb200_attention_bwd_args: null or struct_size mismatch");
     if (a->dtype != VB200_F32) return set_detail(VB200_ERR_UNSUPPORTED, "vb200_attention_bwd: fp32 only (the reference's training dtype)");
@@ -575,7 +585,7 @@ int vb200_attention_bwd(const vb200_attention_bwd_args* a) {
     if (!a->d_out || !a->q || !a->k || !a->v || !a->out || !a->lse || !a->dq || !a->dk || !a->dv)
         return set_detail(VB200_ERR_INVALID_ARG, "vb200_attention_bwd: null tensor");
     // enough for the row sums: the CUDA cores; enough for the terms too, and aligned: the tensor cores
-    if (!a->workspace || a->workspace_bytes < sizeof(float) * static_cast<size_t>(a->B) * a->H * a->N)
+    if (!a->workspace || a->workspace_bytes < vb200_attention_bwd_workspace_bytes_min(a))
         return set_detail(VB200_ERR_WORKSPACE, "vb200_attention_bwd: workspace missing or too small");
     DeviceGuard g;
     if (int rc = g.init(a->device)) return rc;

@@ -45,6 +45,13 @@ void* current_stream() { return Stream::current(Device::CUDA).raw_handle(); }
 Tensor workspace(size_t bytes) {
     return empty({static_cast<int64_t>((bytes + 255) / 256 * 64)}, DType::Float32, Device::CUDA);
 }
+// the same, or what a call cannot do without where the device has no room for all of it
+Tensor workspace(size_t bytes, size_t least) {
+    if (bytes > least) {
+        try { return workspace(bytes); } catch (const std::runtime_error&) {}
+    }
+    return workspace(least);
+}
 
 }  // namespace
 
@@ -66,7 +73,7 @@ void flash_attention_cuda_dispatch(const Tensor& q, const Tensor& k, const Tenso
     a.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
     Tensor ws;
     if (const size_t need = vb200_prefill_workspace_bytes(&a)) {
-        ws = workspace(need);
+        ws = workspace(need, vb200_prefill_workspace_bytes_min(&a));
         a.workspace = ws.data_ptr<char>();
         a.workspace_bytes = ws.numel() * 4;
     }
@@ -122,7 +129,7 @@ void flash_attention_backward_cuda_dispatch(const Tensor& grad_output, const Ten
     a.d_out = dO.data_ptr<char>(); a.q = qc.data_ptr<char>(); a.k = kc.data_ptr<char>(); a.v = vc.data_ptr<char>(); a.out = oc.data_ptr<char>();
     a.lse = lc.data_ptr<float>();
     a.dq = grad_q.data_ptr<char>(); a.dk = grad_k.data_ptr<char>(); a.dv = grad_v.data_ptr<char>();
-    Tensor ws = workspace(vb200_attention_bwd_workspace_bytes(&a));
+    Tensor ws = workspace(vb200_attention_bwd_workspace_bytes(&a), vb200_attention_bwd_workspace_bytes_min(&a));
     a.workspace = ws.data_ptr<char>();
     a.workspace_bytes = ws.numel() * 4;
     check(vb200_attention_bwd(&a), "flash_attention_backward");
@@ -254,7 +261,7 @@ Tensor fused_attention(const Tensor& q, const Tensor& k, const Tensor& v, KVCach
         a.k_cache = view4(cache->k()); a.v_cache = view4(cache->v());
         a.cache_cap = cache->get_max_seq_len();
     }
-    Tensor ws = workspace(vb200_prefill_workspace_bytes(&a));
+    Tensor ws = workspace(vb200_prefill_workspace_bytes(&a), vb200_prefill_workspace_bytes_min(&a));
     a.workspace = ws.data_ptr<char>();
     a.workspace_bytes = ws.numel() * 4;
     check(vb200_prefill_fwd(&a), "attention");

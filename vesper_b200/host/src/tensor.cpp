@@ -75,6 +75,7 @@ public:
             std::lock_guard<std::mutex> lock(mu_);
             give_back(dev, 0);
             e = cudaMalloc(&p, rounded);
+            if (e != cudaSuccess) cudaGetLastError();        // said by the exception: not for the next launch to find
         }
         cuda_check(e, "cudaMalloc");
         return p;
