@@ -21,24 +21,24 @@ int main() {
     const size_t one = fake::given();
     buffer(kGiB + 8192);
     CHECK(fake::given() == one);
-    // the free blocks of many large buffers go back beyond 8 GiB
+    // the free blocks of many large buffers go back beyond 32 GiB
     {
         std::vector<Tensor> t;
-        for (int i = 0; i < 20; ++i) t.push_back(buffer(kGiB + kGiB / 2));
-        CHECK(fake::given() >= 30 * kGiB);
+        for (int i = 0; i < 40; ++i) t.push_back(buffer(kGiB + kGiB / 2));
+        CHECK(fake::given() >= 60 * kGiB);
     }
-    CHECK(fake::given() <= 8 * kGiB);
+    CHECK(fake::given() <= 32 * kGiB);
     // not those that a stream still works on, and none while the thread captures
     for (const auto state : {fake::kBusy, fake::kCapturing}) {
         {
             std::vector<Tensor> t;
-            for (int i = 0; i < 10; ++i) t.push_back(buffer(kGiB + kGiB / 2));
+            for (int i = 0; i < 30; ++i) t.push_back(buffer(kGiB + kGiB / 2));
             fake::streams[static_cast<cudaStream_t>(a.raw_handle())] = state;
         }
-        CHECK(fake::given() >= 15 * kGiB);
+        CHECK(fake::given() >= 45 * kGiB);
         fake::streams[static_cast<cudaStream_t>(a.raw_handle())] = fake::kIdle;
         buffer(1024);
-        CHECK(fake::given() <= 8 * kGiB);
+        CHECK(fake::given() <= 32 * kGiB);
     }
     // a full device: what is free goes back and the buffer is had after all
     fake::memory = 10 * kGiB;

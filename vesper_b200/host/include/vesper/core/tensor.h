@@ -12,6 +12,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <cstring>
 #include <memory>
 #include <optional>
 #include <stdexcept>
@@ -72,7 +73,7 @@ private:
 };
 
 // Reference-counted buffer; CUDA buffers come from a small caching allocator
-// (bins by size, as src/core/allocator.cpp:171-221 has), which gives back what is free beyond 8 GiB.  A buffer may be let go of while
+// (bins by size, as src/core/allocator.cpp:171-221 has), which gives back what is free beyond 32 GiB.  A buffer may be let go of while
 // the stream that was current when it was created, or the one current now, still has work on it: another stream
 // gets it only afterwards.  (Work on a third stream has to be waited for first.)
 class Storage {
@@ -154,8 +155,19 @@ Tensor zeros(const std::vector<int64_t>& shape, DType dtype, Device device, bool
 // Host-side 16-bit conversions.  BFloat16 rounds to nearest even like
 // include/vesper/core/half.h:162-173; Float16 rounds to nearest even too (the
 // reference truncates, half.h:56, which does not match what the GPU does).
-uint16_t float_to_bf16(float f);
-float bf16_to_float(uint16_t h);
+// (inline: called for every value of a model's weights)
+inline uint16_t float_to_bf16(float f) {
+    uint32_t bits;
+    std::memcpy(&bits, &f, 4);
+    bits += 0x7FFFu + ((bits >> 16) & 1u);
+    return static_cast<uint16_t>(bits >> 16);
+}
+inline float bf16_to_float(uint16_t h) {
+    const uint32_t bits = static_cast<uint32_t>(h) << 16;
+    float f;
+    std::memcpy(&f, &bits, 4);
+    return f;
+}
 uint16_t float_to_fp16(float f);
 float fp16_to_float(uint16_t h);
 

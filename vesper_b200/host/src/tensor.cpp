@@ -88,7 +88,7 @@ public:
     }
 
 private:
-    static constexpr size_t kLarge = size_t{64} << 20, kMostFree = size_t{8} << 30;
+    static constexpr size_t kLarge = size_t{512} << 20, kMostFree = size_t{32} << 30;
     struct Block { void* p; Streams streams; };
     // Idle blocks, the largest first, until at most `keep` bytes are free.  Not while this thread captures a graph (cudaFree would end that).
     void give_back(int dev, size_t keep) {
@@ -120,6 +120,25 @@ struct PageLockedWord {
     int32_t* p = nullptr;
     PageLockedWord() { cuda_check(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int32_t), cudaHostAllocPortable), "cudaHostAlloc"); *p = 0; }
     ~PageLockedWord() { cudaFreeHost(p); }
+};
+
+// Around a wait for a stream's work: queues a copy of the device status word behind that work, and throws after the wait if a kernel's own wait has
+// expired.  Queued ahead of a copy that the host waits for anyway it costs no round trip of its own.
+class KernelStatus {
+public:
+    explicit KernelStatus(void* stream) : stream_(stream) { queued_ = vb200_copy_kernel_status(-1, stream, word().p) == VB200_OK; }
+    void check() const {
+        // (a note about a full sequence or an id out of range stays for vb200_check_kernel_status)
+        if (!queued_ || vb200_kernel_status_of(*word().p) != VB200_ERR_KERNEL_TIMEOUT) return;
+        const std::string text = vb200_last_error_detail();
+        vb200_check_kernel_status(-1, stream_);                  // clears it
+        throw std::runtime_error("a kernel gave up waiting, its results are void: " + text);
+    }
+
+private:
+    static PageLockedWord& word() { static thread_local PageLockedWord w; return w; }
+    void* stream_;
+    bool queued_;
 };
 
 thread_local Stream* t_current = nullptr;
@@ -155,14 +174,9 @@ Stream::~Stream() {
 }
 void Stream::synchronize() const {
     if (device_ != Device::CUDA) return;
-    static thread_local PageLockedWord word;
-    const int queued = vb200_copy_kernel_status(-1, handle_, word.p);
+    const KernelStatus status(handle_);
     cuda_check(cudaStreamSynchronize(static_cast<cudaStream_t>(handle_)), "cudaStreamSynchronize");
-    // (a note about a full sequence or an id out of range stays for vb200_check_kernel_status)
-    if (queued != VB200_OK || vb200_kernel_status_of(*word.p) != VB200_ERR_KERNEL_TIMEOUT) return;
-    const std::string text = vb200_last_error_detail();
-    vb200_check_kernel_status(-1, handle_);                  // clears it
-    throw std::runtime_error("a kernel gave up waiting, its results are void: " + text);
+    status.check();
 }
 Stream& Stream::default_stream(Device device) {
     static Stream& cuda_default = *new Stream(Device::CUDA, nullptr);   // legacy stream 0 (src/core/stream.cpp:104-111)
@@ -222,8 +236,11 @@ void Tensor::copy_to_host(void* host_ptr) const {
     if (!is_contiguous()) { contiguous().copy_to_host(host_ptr); return; }
     size_t bytes = numel() * GetDTypeSize(dtype_);
     if (device() == Device::CUDA) {
-        Stream::current(Device::CUDA).synchronize();
-        cuda_check(cudaMemcpy(host_ptr, data_ptr<char>(), bytes, cudaMemcpyDeviceToHost), "cudaMemcpy D2H");
+        const cudaStream_t stream = static_cast<cudaStream_t>(Stream::current(Device::CUDA).raw_handle());
+        const KernelStatus status(stream);
+        cuda_check(cudaMemcpyAsync(host_ptr, data_ptr<char>(), bytes, cudaMemcpyDeviceToHost, stream), "cudaMemcpy D2H");
+        cuda_check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+        status.check();
     } else {
         std::memcpy(host_ptr, data_ptr<char>(), bytes);
     }
@@ -393,18 +410,6 @@ Tensor zeros(const std::vector<int64_t>& shape, DType dtype, Device device, bool
 }
 
 // ---- 16-bit conversions ----
-uint16_t float_to_bf16(float f) {
-    uint32_t bits;
-    std::memcpy(&bits, &f, 4);
-    bits += 0x7FFFu + ((bits >> 16) & 1u);
-    return static_cast<uint16_t>(bits >> 16);
-}
-float bf16_to_float(uint16_t h) {
-    uint32_t bits = static_cast<uint32_t>(h) << 16;
-    float f;
-    std::memcpy(&f, &bits, 4);
-    return f;
-}
 uint16_t float_to_fp16(float f) {
     uint32_t x;
     std::memcpy(&x, &f, 4);
