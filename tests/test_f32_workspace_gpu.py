@@ -62,7 +62,7 @@ def test_a_caller_may_decline_the_terms(cuda, lib):
     assert lib.vb200_last_prefill_kernel() == b"prefill_f32_kernel"
     got = capi.attention_bwd(do, q, k, v, o, lse, scale=D ** -0.5, workspace=rows)
     torch.cuda.synchronize()
-    assert torch.cuda.max_memory_allocated() - before <= 3 * q.numel() * 4 + (1 << 20)
+    assert torch.cuda.max_memory_allocated() - before <= 3 * q.numel() * 4 + (8 << 20)          # (the gradients, in torch's rounded blocks)
     whole = capi.prefill(q, k, v, o.clone(), lse.clone(), scale=D ** -0.5)
     assert lib.vb200_last_prefill_kernel() == b"attention_f32_forward_kernel" and whole.numel() > 4 * q.numel()
     for x, w in zip((o, lse, *got), _reference(q, k, v, do, 0, True)):

@@ -210,17 +210,18 @@ def _stream_ptr(stream):
 
 
 def _workspace(nbytes, device, stream, least=None):
-    """Bytes that belong to `stream` (None: the current one): torch gives their memory to later work of that stream only.  `least` bytes where the device
+    """Bytes that belong to `stream` (None: the current one): torch gives their memory to later work of that stream only.  least() bytes where the device
     has no room for all."""
-    import contextlib
     import torch
-    with torch.cuda.stream(stream) if isinstance(stream, torch.cuda.Stream) else contextlib.nullcontext():
-        try:
-            return torch.empty(nbytes, dtype=torch.uint8, device=device)
-        except torch.cuda.OutOfMemoryError:
-            if least is None or least >= nbytes:
-                raise
-        return torch.empty(least, dtype=torch.uint8, device=device)
+    if isinstance(stream, torch.cuda.Stream):
+        with torch.cuda.stream(stream):
+            return _workspace(nbytes, device, None, least)
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        if least is None or least() >= nbytes:
+            raise
+    return torch.empty(least(), dtype=torch.uint8, device=device)
 
 
 def _ptr(t):
@@ -264,7 +265,7 @@ def prefill(q, k, v, o, lse=None, *, scale, causal=True, start_pos=0, theta=None
     need = L.vb200_prefill_workspace_bytes(C.byref(a))
     rc = ERR_WORKSPACE if need > a.workspace_bytes and workspace is None else L.vb200_prefill_fwd(C.byref(a))
     if rc == ERR_WORKSPACE:
-        workspace = _workspace(need, q.device, stream, L.vb200_prefill_workspace_bytes_min(C.byref(a)))
+        workspace = _workspace(need, q.device, stream, lambda: L.vb200_prefill_workspace_bytes_min(C.byref(a)))
         a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel()
         rc = L.vb200_prefill_fwd(C.byref(a))
     check(rc)
@@ -356,8 +357,7 @@ def attention_bwd(d_out, q, k, v, out, lse, *, scale, causal=True, stream=None, 
         assert t.is_contiguous()
         setattr(a, name, _ptr(t))
     if workspace is None:
-        need, least = load().vb200_attention_bwd_workspace_bytes(C.byref(a)), load().vb200_attention_bwd_workspace_bytes_min(C.byref(a))
-        workspace = _workspace(need, q.device, stream, least)
+        workspace = _workspace(load().vb200_attention_bwd_workspace_bytes(C.byref(a)), q.device, stream, lambda: load().vb200_attention_bwd_workspace_bytes_min(C.byref(a)))
     a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel() * workspace.element_size()
     check(load().vb200_attention_bwd(C.byref(a)))
     return dq, dk, dv
