@@ -17,11 +17,11 @@
 //
 // The terms of the streamed operands are written to the workspace beforehand (split_blocks_kernel), each block as it will stand in
 // shared memory: splitting them where they are used repeats the work for every tile of rows that reads them, and eight warps that did
-// so were what the kernel waited for (2 x 16 x 1999 x 128: forward 278 us, backward 1086; now 168 and 780, with 79 for the splits).
+// so were what the kernel waited for (2 x 16 x 1999 x 128: forward 278 us, backward 1086; calls now 197 and 860-950, splits included).
 //
-// What bounds it: with head_dim 128 the products, 48 of 64 columns (39 cycles each, 32 at the nominal rate) and 24 of 128 per block in
-// the forward, beside the weights of one warpgroup; in dQ and dK also the wait for W, whose slot TMEM holds only once.  The same calls on
-// the CUDA cores (prefill_f32.cu, flash_bwd_f32.cu): 1109 and 3086 us; 16 x 512 x 64 49 and 126 us against 21 and 31.
+// What bounds it: with head_dim 128 the products, 48 of 64 columns and 24 of 128 per block in the forward, beside the weights of one warpgroup (tensor
+// pipe busy 64 % of the forward's time, 57 % of the backward's, 16 x 2048 x 128); in dQ and dK also the wait for W, whose slot TMEM holds only once.
+// The same calls on the CUDA cores (prefill_f32.cu, flash_bwd_f32.cu): 1105 and 3087 us; 16 x 512 x 64 50 and 128 us against 21 and 36-40.
 //
 // The tensor cores add with truncation, so no sum stays with them for long: a block's six products are added smallest first, and
 // each block's result is added to the sum in registers, rounded to nearest.  What the last eight (or four) additions of a score lose
