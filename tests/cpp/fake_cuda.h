@@ -48,7 +48,11 @@ cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* c) {
     return cudaSuccess;
 }
 cudaError_t cudaStreamQuery(cudaStream_t s) {
-    if (fake::streams.at(s) == fake::kCapturing) { std::puts("FAIL: a capturing stream was queried"); std::exit(1); }
+    const auto current = static_cast<cudaStream_t>(vesper::Stream::current(vesper::Device::CUDA).raw_handle());
+    if (fake::streams.at(s) == fake::kCapturing || (current && fake::streams.at(current) == fake::kCapturing)) {
+        std::puts("FAIL: a stream was queried that captures, or by a thread that does");
+        std::exit(1);
+    }
     return fake::last = fake::streams.at(s) == fake::kBusy ? cudaErrorNotReady : cudaSuccess;
 }
 cudaError_t cudaMemcpy(void*, const void*, size_t, cudaMemcpyKind) { return cudaSuccess; }

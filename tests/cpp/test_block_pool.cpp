@@ -35,6 +35,7 @@ int main() {
     fake::streams[raw(a)] = fake::kCapturing;
     void* c = use(a, 5000);
     CHECK(use(b, 5000) != c);
+    use(a, 5000);                                             // its own or a new one, without a question to b
     // idle: anyone's
     fake::streams[raw(a)] = fake::kIdle;
     CHECK(use(b, 1000) == p || use(b, 1000) == q);

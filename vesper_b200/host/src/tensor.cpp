@@ -28,11 +28,14 @@ void add_stream(Streams& list, const std::shared_ptr<void>& s) {
     if (s) list.push_back(s);
 }
 
+bool capturing(const std::shared_ptr<void>& s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return s && (cudaStreamIsCapturing(static_cast<cudaStream_t>(s.get()), &status) != cudaSuccess || status != cudaStreamCaptureStatusNone);
+}
+
 bool idle(const std::shared_ptr<void>& s) {
-    cudaStream_t stream = static_cast<cudaStream_t>(s.get());
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
-    const cudaError_t e = cudaStreamQuery(stream);
+    if (capturing(s)) return false;
+    const cudaError_t e = cudaStreamQuery(static_cast<cudaStream_t>(s.get()));
     if (e == cudaErrorNotReady) cudaGetLastError();          // an answer, not an error for the next check to find
     return e == cudaSuccess;
 }
@@ -56,11 +59,12 @@ public:
         {
             std::lock_guard<std::mutex> lock(mu_);
             auto& bin = free_[{dev, rounded}];
+            const bool ask = !bin.empty() && !capturing(current);        // (a thread that captures asks nothing of other streams)
             for (size_t i = bin.size(); i-- > 0;) {
                 Block& b = bin[i];
-                const bool only_own = b.streams.empty() || (b.streams.size() == 1 && b.streams[0] == current);
-                if (current ? !only_own : b.streams.size() > 4) drop_idle(b.streams, current);
-                if (current && !(b.streams.empty() || (b.streams.size() == 1 && b.streams[0] == current))) continue;
+                auto in_order = [&] { return !current || b.streams.empty() || (b.streams.size() == 1 && b.streams[0] == current); };
+                if (ask && (!in_order() || b.streams.size() > 4)) drop_idle(b.streams, current);
+                if (!in_order()) continue;
                 void* p = b.p;
                 streams = std::move(b.streams);
                 bin.erase(bin.begin() + static_cast<std::ptrdiff_t>(i));
@@ -92,9 +96,7 @@ private:
     struct Block { void* p; Streams streams; };
     // Idle blocks, the largest first, until at most `keep` bytes are free.  Not while this thread captures a graph (cudaFree would end that).
     void give_back(int dev, size_t keep) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        const auto current = Stream::current(Device::CUDA).owner();
-        if (current && (cudaStreamIsCapturing(static_cast<cudaStream_t>(current.get()), &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)) return;
+        if (capturing(Stream::current(Device::CUDA).owner())) return;
         for (auto it = free_.rbegin(); it != free_.rend() && free_bytes_[dev] > keep; ++it) {
             if (it->first.first != dev) continue;
             auto& bin = it->second;
