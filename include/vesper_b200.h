@@ -340,10 +340,9 @@ int vb200_profile_read(double* total_ms, uint64_t* launches);
  * kernels' capacity check set (synchronises the given stream).  Returns VB200_OK,
  * VB200_ERR_KERNEL_TIMEOUT or VB200_ERR_CACHE_OVERFLOW. */
 int vb200_check_kernel_status(int device, void* stream);
-/* The same word without a synchronisation of its own: queues a copy of it to page-locked host memory behind the
- * stream's work, to be looked at (vb200_kernel_status_of: the same results) after the caller's next synchronisation.
- * Does not clear it. */
-int vb200_copy_kernel_status(int device, void* stream, int32_t* host_word);
+/* Where that word is: page-locked memory of the host, one word per device, 0 until a kernel sets it.  To be looked at
+ * after the caller has waited for the work, and read with vb200_kernel_status_of (the same results, without clearing). */
+int vb200_kernel_status_on_host(int device, const volatile int32_t** word);
 int vb200_kernel_status_of(int32_t word);
 
 #ifdef __cplusplus

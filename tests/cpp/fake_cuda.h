@@ -19,7 +19,7 @@ std::map<void*, size_t> blocks;         // what the driver has given out, at mos
 size_t memory = size_t{180} << 30;
 size_t given() { size_t n = 0; for (auto& b : blocks) n += b.second; return n; }
 cudaError_t last = cudaSuccess;
-int32_t status = 0;             // the device status word
+int32_t status = 0;             // the device's status word
 char detail[64];
 }  // namespace fake
 
@@ -58,11 +58,9 @@ cudaError_t cudaStreamQuery(cudaStream_t s) {
 cudaError_t cudaMemcpy(void*, const void*, size_t, cudaMemcpyKind) { return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n); return cudaSuccess; }
-cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
 const char* vb200_strerror(int) { return ""; }
 const char* vb200_last_error_detail(void) { return fake::detail; }
-int vb200_copy_kernel_status(int, void*, int32_t* word) { *word = fake::status; return VB200_OK; }
+int vb200_kernel_status_on_host(int, const volatile int32_t** word) { *word = &fake::status; return VB200_OK; }
 int vb200_kernel_status_of(int32_t word) {
     std::snprintf(fake::detail, sizeof(fake::detail), "code %d, site 0x%x", word >> 24, word & 0xFFFFFF);
     return word == 0 ? VB200_OK : word >> 24 == 2 ? VB200_ERR_CACHE_OVERFLOW : VB200_ERR_KERNEL_TIMEOUT;

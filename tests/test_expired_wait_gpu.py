@@ -1,4 +1,6 @@
 """A wait inside a kernel that ran out is an error of the next call that waits for the device, not a silently wrong result."""
+import os
+
 import numpy as np
 import pytest
 
@@ -45,3 +47,38 @@ def test_an_expired_wait_replaces_a_note_about_an_id(cuda):
     with pytest.raises(capi.Vb200Error, match="bounded in-kernel wait"):
         capi.check_kernel_status(0)
     capi.check_kernel_status(0)
+
+
+def test_the_word_in_host_memory(cuda, lib):
+    """Set by the kernels themselves, seen without a copy and cleared by a check; the same on a first use while a graph is captured (a process of its own)."""
+    import ctypes as C
+    import subprocess
+    import sys
+    import torch
+    from vesper_b200 import capi
+    word = C.POINTER(C.c_int32)()
+    capi.check(lib.vb200_kernel_status_on_host(0, C.byref(word)))
+    assert word[0] == 0
+    _expire(cuda)
+    assert word[0] >> 24 == 3 and lib.vb200_kernel_status_of(word[0]) == -7
+    with pytest.raises(capi.Vb200Error):
+        capi.check_kernel_status(0)
+    assert word[0] == 0
+    r = subprocess.run([sys.executable, "-c", CAPTURED], capture_output=True, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and r.stdout.strip() == "-8 0", r.stdout + r.stderr
+
+
+# the library's first launch is a captured one: ids outside the vocabulary, replayed
+CAPTURED = """
+import torch
+from vesper_b200 import capi
+lib = capi.load()
+ids, table, out = torch.tensor([9], dtype=torch.int32, device="cuda"), torch.ones(4, 128, dtype=torch.bfloat16, device="cuda"), torch.ones(1, 128, device="cuda")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    capi.embedding(ids, table, out)
+graph.replay()
+torch.cuda.synchronize()
+assert (out == 0).all()
+print(lib.vb200_check_kernel_status(0, None), lib.vb200_check_kernel_status(0, None))
+"""

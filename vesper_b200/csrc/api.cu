@@ -4,25 +4,34 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 
 #include "kernels.h"
 
 namespace vb200 {
 
-__device__ int g_kernel_status = 0;
-
+// The status word of a device: page-locked host memory that its kernels write (only when a wait expires, a sequence is full or an id is out of
+// range), so that the host can look at it without a copy.  Allocated on first use, also while a graph is captured; kept until the process ends.
 int* kernel_status_word() {
-    // one symbol instance per device; cache the address per ordinal
-    static thread_local int* cache[64] = {nullptr};
+    static int* volatile words[64] = {nullptr};
+    static std::mutex mu;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    if (!cache[dev]) {
-        void* p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_kernel_status) != cudaSuccess) return nullptr;
-        cache[dev] = static_cast<int*>(p);
+    if (!words[dev]) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!words[dev]) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // (this thread's; the allocation is no part of what is captured)
+            if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+            int* p = nullptr;
+            const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&p), 64, cudaHostAllocPortable | cudaHostAllocMapped);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) return nullptr;
+            *p = 0;
+            words[dev] = p;
+        }
     }
-    return cache[dev];
+    return words[dev];
 }
 
 namespace {
@@ -262,27 +271,22 @@ void vb200_rope_inv_freq(float theta, int32_t D, float* inv_freq_host) {
     for (int i = 0; i < D / 2; ++i) inv_freq_host[i] = std::pow(theta, -2.0f * i / D);
 }
 
-int vb200_copy_kernel_status(int device, void* stream, int32_t* host_word) {
-    if (!host_word) return set_detail(VB200_ERR_INVALID_ARG, "vb200_copy_kernel_status: null word");
+int vb200_kernel_status_on_host(int device, const volatile int32_t** word) {
+    if (!word) return set_detail(VB200_ERR_INVALID_ARG, "vb200_kernel_status_on_host: null word");
     DeviceGuard g;
     if (int rc = g.init(device)) return rc;
-    const int* word = kernel_status_word();
-    if (!word) return set_detail(VB200_ERR_CUDA, "cannot resolve the device status word");
-    VB200_CUDA_TRY(cudaMemcpyAsync(host_word, word, sizeof(int), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
-    return VB200_OK;
+    *word = kernel_status_word();
+    return *word ? VB200_OK : set_detail(VB200_ERR_CUDA, "cannot allocate the status word");
 }
 
 int vb200_check_kernel_status(int device, void* stream) {
     DeviceGuard g;
     if (int rc = g.init(device)) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int host = 0;
-    VB200_CUDA_TRY(cudaMemcpyFromSymbolAsync(&host, g_kernel_status, sizeof(int), 0, cudaMemcpyDeviceToHost, s));
-    VB200_CUDA_TRY(cudaStreamSynchronize(s));
-    if (host == 0) return VB200_OK;
-    int zero = 0;
-    VB200_CUDA_TRY(cudaMemcpyToSymbolAsync(g_kernel_status, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, s));
-    VB200_CUDA_TRY(cudaStreamSynchronize(s));
+    volatile int* word = kernel_status_word();
+    if (!word) return set_detail(VB200_ERR_CUDA, "cannot allocate the status word");
+    VB200_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+    const int host = *word;
+    if (host != 0) *word = 0;
     return vb200_kernel_status_of(host);
 }
 
@@ -372,7 +376,7 @@ int vb200_prefill_fwd(const vb200_prefill_args* a) {
     p.q_rope_table = table;
     p.inv_freq = f;
     p.status = kernel_status_word();
-    if (!p.status) return set_detail(VB200_ERR_CUDA, "cannot resolve the device status word");
+    if (!p.status) return set_detail(VB200_ERR_CUDA, "cannot allocate the status word");
     // fp32 with a smaller workspace, or none, runs on the CUDA cores
     if (pl.split_bytes > 0 && a->workspace && a->workspace_bytes >= pl.total + pl.split_bytes && reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0) p.split = ws + pl.total;
 
@@ -485,7 +489,7 @@ int decode_impl(const vb200_decode_args* a, const vb200_exchange_args* x) {
     p.workspace = static_cast<float*>(a->workspace);
     p.ws_header = pl.ws_header;
     p.status = kernel_status_word();
-    if (!p.status) return set_detail(VB200_ERR_CUDA, "cannot resolve the device status word");
+    if (!p.status) return set_detail(VB200_ERR_CUDA, "cannot allocate the status word");
     if (x) {
         if (int rc = fill_exchange(p.xchg, x, "vb200_decode_exchange_fwd")) return rc;
         if (x->rows != static_cast<int64_t>(a->B) * a->Hq || x->D != a->D || x->dtype != a->dtype)
@@ -596,7 +600,7 @@ int vb200_attention_bwd(const vb200_attention_bwd_args* a) {
     p.dq = static_cast<float*>(a->dq); p.dk = static_cast<float*>(a->dk); p.dv = static_cast<float*>(a->dv);
     p.delta = static_cast<float*>(a->workspace);
     p.status = kernel_status_word();
-    if (!p.status) return set_detail(VB200_ERR_CUDA, "cannot resolve the device status word");
+    if (!p.status) return set_detail(VB200_ERR_CUDA, "cannot allocate the status word");
     if (attention_bwd_f32_on_tensor_cores(a->D, a->N) && a->workspace_bytes >= vb200_attention_bwd_workspace_bytes(a) && reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0)
         p.split = static_cast<unsigned char*>(a->workspace) + bwd_delta_bytes(a);
     return launch_attention_bwd_f32(static_cast<cudaStream_t>(a->stream), p);

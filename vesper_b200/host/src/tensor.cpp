@@ -117,31 +117,15 @@ private:
     std::map<int, size_t> free_bytes_;          // per device
 };
 
-// A word of page-locked memory per thread, into which the device status word is copied along with a synchronisation.
-struct PageLockedWord {
-    int32_t* p = nullptr;
-    PageLockedWord() { cuda_check(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int32_t), cudaHostAllocPortable), "cudaHostAlloc"); *p = 0; }
-    ~PageLockedWord() { cudaFreeHost(p); }
-};
-
-// Around a wait for a stream's work: queues a copy of the device status word behind that work, and throws after the wait if a kernel's own wait has
-// expired.  Queued ahead of a copy that the host waits for anyway it costs no round trip of its own.
-class KernelStatus {
-public:
-    explicit KernelStatus(void* stream) : stream_(stream) { queued_ = vb200_copy_kernel_status(-1, stream, word().p) == VB200_OK; }
-    void check() const {
-        // (a note about a full sequence or an id out of range stays for vb200_check_kernel_status)
-        if (!queued_ || vb200_kernel_status_of(*word().p) != VB200_ERR_KERNEL_TIMEOUT) return;
-        const std::string text = vb200_last_error_detail();
-        vb200_check_kernel_status(-1, stream_);                  // clears it
-        throw std::runtime_error("a kernel gave up waiting, its results are void: " + text);
-    }
-
-private:
-    static PageLockedWord& word() { static thread_local PageLockedWord w; return w; }
-    void* stream_;
-    bool queued_;
-};
+// After a wait for a stream's work: throws if a wait inside a kernel has expired on the current device.  (A note about a full sequence or an id out
+// of range stays for vb200_check_kernel_status.)
+void check_kernel_waits(void* stream) {
+    const volatile int32_t* word = nullptr;
+    if (vb200_kernel_status_on_host(-1, &word) != VB200_OK || vb200_kernel_status_of(*word) != VB200_ERR_KERNEL_TIMEOUT) return;
+    const std::string text = vb200_last_error_detail();
+    vb200_check_kernel_status(-1, stream);                       // clears it
+    throw std::runtime_error("a kernel gave up waiting, its results are void: " + text);
+}
 
 thread_local Stream* t_current = nullptr;
 
@@ -176,9 +160,8 @@ Stream::~Stream() {
 }
 void Stream::synchronize() const {
     if (device_ != Device::CUDA) return;
-    const KernelStatus status(handle_);
     cuda_check(cudaStreamSynchronize(static_cast<cudaStream_t>(handle_)), "cudaStreamSynchronize");
-    status.check();
+    check_kernel_waits(handle_);
 }
 Stream& Stream::default_stream(Device device) {
     static Stream& cuda_default = *new Stream(Device::CUDA, nullptr);   // legacy stream 0 (src/core/stream.cpp:104-111)
@@ -239,10 +222,9 @@ void Tensor::copy_to_host(void* host_ptr) const {
     size_t bytes = numel() * GetDTypeSize(dtype_);
     if (device() == Device::CUDA) {
         const cudaStream_t stream = static_cast<cudaStream_t>(Stream::current(Device::CUDA).raw_handle());
-        const KernelStatus status(stream);
         cuda_check(cudaMemcpyAsync(host_ptr, data_ptr<char>(), bytes, cudaMemcpyDeviceToHost, stream), "cudaMemcpy D2H");
         cuda_check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-        status.check();
+        check_kernel_waits(stream);
     } else {
         std::memcpy(host_ptr, data_ptr<char>(), bytes);
     }
