@@ -213,7 +213,7 @@ def _workspace(nbytes, device, stream, least=None):
     """Bytes that belong to `stream` (None: the current one): torch gives their memory to later work of that stream only.  least() bytes where the device
     has no room for all."""
     import torch
-    if isinstance(stream, torch.cuda.Stream):
+    if stream is not None and isinstance(stream, torch.cuda.Stream):
         with torch.cuda.stream(stream):
             return _workspace(nbytes, device, None, least)
     try:
@@ -350,16 +350,17 @@ def attention_bwd(d_out, q, k, v, out, lse, *, scale, causal=True, stream=None, 
     a.dtype = dtype_code(q)
     a.B, a.H, a.N, a.D, a.causal, a.scale = B, H, N, D, int(causal), scale
     dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.empty_like(q)
-    if isinstance(stream, torch.cuda.Stream):
+    if stream is not None and isinstance(stream, torch.cuda.Stream):
         for t in (dq, dk, dv):
             t.record_stream(stream)                        # let go of early, they are not the current stream's again before this call is done
     for name, t in (("d_out", d_out), ("q", q), ("k", k), ("v", v), ("out", out), ("lse", lse), ("dq", dq), ("dk", dk), ("dv", dv)):
         assert t.is_contiguous()
         setattr(a, name, _ptr(t))
+    L = load()
     if workspace is None:
-        workspace = _workspace(load().vb200_attention_bwd_workspace_bytes(C.byref(a)), q.device, stream, lambda: load().vb200_attention_bwd_workspace_bytes_min(C.byref(a)))
-    a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel() * workspace.element_size()
-    check(load().vb200_attention_bwd(C.byref(a)))
+        workspace = _workspace(L.vb200_attention_bwd_workspace_bytes(C.byref(a)), q.device, stream, lambda: L.vb200_attention_bwd_workspace_bytes_min(C.byref(a)))
+    a.workspace, a.workspace_bytes = _ptr(workspace), workspace.nbytes
+    check(L.vb200_attention_bwd(C.byref(a)))
     return dq, dk, dv
 
 
