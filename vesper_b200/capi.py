@@ -209,19 +209,19 @@ def _stream_ptr(stream):
     return C.c_void_p(s.cuda_stream)
 
 
-def _workspace(nbytes, device, stream, least=None):
-    """Bytes that belong to `stream` (None: the current one): torch gives their memory to later work of that stream only.  least() bytes where the device
-    has no room for all."""
+def _workspace(nbytes, device, stream, least=None, args=None):
+    """Bytes that belong to `stream` (None: the current one): torch gives their memory to later work of that stream only.  least(args) bytes where the
+    device has no room for all."""
     import torch
     if stream is not None and isinstance(stream, torch.cuda.Stream):
         with torch.cuda.stream(stream):
-            return _workspace(nbytes, device, None, least)
+            return _workspace(nbytes, device, None, least, args)
     try:
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
     except torch.cuda.OutOfMemoryError:
-        if least is None or least() >= nbytes:
+        if least is None or least(args) >= nbytes:
             raise
-    return torch.empty(least(), dtype=torch.uint8, device=device)
+    return torch.empty(least(args), dtype=torch.uint8, device=device)
 
 
 def _ptr(t):
@@ -262,13 +262,16 @@ def prefill(q, k, v, o, lse=None, *, scale, causal=True, start_pos=0, theta=None
     L = load()
     a = prefill_args(q, k, v, o, lse, scale=scale, causal=causal, start_pos=start_pos, theta=theta,
                      k_cache=k_cache, v_cache=v_cache, workspace=workspace, stream=stream, cache_read_only=cache_read_only)
-    need = L.vb200_prefill_workspace_bytes(C.byref(a))
-    rc = ERR_WORKSPACE if need > a.workspace_bytes and workspace is None else L.vb200_prefill_fwd(C.byref(a))
-    if rc == ERR_WORKSPACE:
-        workspace = _workspace(need, q.device, stream, lambda: L.vb200_prefill_workspace_bytes_min(C.byref(a)))
+    ref = C.byref(a)
+    need = L.vb200_prefill_workspace_bytes(ref)
+    if need > a.workspace_bytes:
+        rc = ERR_WORKSPACE if workspace is None else L.vb200_prefill_fwd(ref)
+        if rc != ERR_WORKSPACE:
+            check(rc)
+            return workspace
+        workspace = _workspace(need, q.device, stream, L.vb200_prefill_workspace_bytes_min, ref)
         a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel()
-        rc = L.vb200_prefill_fwd(C.byref(a))
-    check(rc)
+    check(L.vb200_prefill_fwd(ref))
     return workspace
 
 
@@ -356,11 +359,11 @@ def attention_bwd(d_out, q, k, v, out, lse, *, scale, causal=True, stream=None, 
     for name, t in (("d_out", d_out), ("q", q), ("k", k), ("v", v), ("out", out), ("lse", lse), ("dq", dq), ("dk", dk), ("dv", dv)):
         assert t.is_contiguous()
         setattr(a, name, _ptr(t))
-    L = load()
+    L, ref = load(), C.byref(a)
     if workspace is None:
-        workspace = _workspace(L.vb200_attention_bwd_workspace_bytes(C.byref(a)), q.device, stream, lambda: L.vb200_attention_bwd_workspace_bytes_min(C.byref(a)))
+        workspace = _workspace(L.vb200_attention_bwd_workspace_bytes(ref), q.device, stream, L.vb200_attention_bwd_workspace_bytes_min, ref)
     a.workspace, a.workspace_bytes = _ptr(workspace), workspace.nbytes
-    check(L.vb200_attention_bwd(C.byref(a)))
+    check(L.vb200_attention_bwd(ref))
     return dq, dk, dv
 
 
